@@ -25,6 +25,7 @@
 //   target's own vesicle is skipped.
 // * Each CTA writes an FP64 partial for its source range; a fixed-order
 //   reduction over the ranges produces the result (deterministic).
+// * The FP64 rule (parity) has its own kernel, ff64_kernel below.
 #include "ves_internal.h"
 
 namespace {
@@ -60,8 +61,6 @@ template <>
 struct FFT<double> {
   typedef Rec64 Rec;
   typedef double2 Pair;
-  static __device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
-  static __device__ __forceinline__ double lg2(double x) { return log2(x); }
   static __device__ __forceinline__ Rec rec(double x, double y, double a, double b) { return Rec64{x, y, a, b}; }
   static __device__ __forceinline__ Pair pair(double a, double b) { return make_double2(a, b); }
 };
@@ -373,6 +372,135 @@ __global__ void ff_reduce_kernel(long long total_pts, int ntp, int nsplit, const
   out[col * 2 * ntp + ntp + j] = sy * scale;
 }
 
+// --------------------------------------------------------------------------
+// FP64 direct rule.  Bound by the FP64 pipe (2 fma/clk/SM: a pair costs ~70
+// FP64 instructions in log2 and the divide, 16 cycles each per warp), so the
+// operands need no staging: what matters is that every SM has several warps.
+// One thread per target point, and the sources are cut into pieces of a
+// vesicle (``chunk`` points), ``per_split`` pieces per CTA row; a small
+// suspension then spreads over the chip where whole source vesicles staged
+// two at a time left it to a single CTA (16 vesicles of N = 32: 43 ms per sum
+// on one SM, 0.17 ms like this).  Each piece is summed relative to
+// its vesicle's centre as in the FP32 kernel, the centre's log times the
+// vesicle's density sum being added with the first piece.
+struct FF64Args {
+  int nsrc, ns, ntp;
+  long long total_pts;
+  const Rec64* src;
+  const double2* src_hi;
+  const double2* src_dsum;
+  const double2* tgt_local;
+  const double2* tgt_hi;
+  const int* self_idx;
+  const int* cand_count;
+  const int* cand_src;
+  const uint32_t* excl_mask;
+  int maxc, nwords;
+  int nchunk, chunk;       // pieces per source vesicle, points per piece
+  int per_split, nsplit;   // pieces per split
+  double* partial;         // [nsplit][total_pts][2]
+};
+
+constexpr int FF64_THREADS = 128;
+
+__global__ void __launch_bounds__(FF64_THREADS) ff64_kernel(FF64Args p) {
+  const long long pt = (long long)blockIdx.x * FF64_THREADS + threadIdx.x;
+  const bool valid = pt < p.total_pts;
+  const long long pq = valid ? pt : 0;
+  const int col = (int)(pq / p.ntp), pidx = (int)(pq % p.ntp);
+  const int self = p.self_idx ? p.self_idx[col] : -1;
+  const double2 tl = p.tgt_local[pq], th = p.tgt_hi[col];
+  const int cend = p.cand_count ? min(p.cand_count[col], p.maxc) : 0;
+  const int* cands = p.cand_src + (long long)col * p.maxc;
+  const int units = p.nsrc * p.nchunk;
+  const int u0 = blockIdx.y * p.per_split, u1 = min(units, u0 + p.per_split);
+  double tot_x = 0, tot_y = 0, cmp_x = 0, cmp_y = 0;
+  int cur = 0;
+  for (int u = u0; u < u1; ++u) {
+    const int s = u / p.nchunk, c = u - s * p.nchunk;
+    bool excl = false;  // near-pair list: ascending source vesicles per target column
+    if (cend > 0) {
+      while (cur < cend && cands[cur] < s) ++cur;
+      if (cur < cend && cands[cur] == s) {
+        const uint32_t w = p.excl_mask[((long long)col * p.maxc + cur) * p.nwords + (pidx >> 5)];
+        excl = (w >> (pidx & 31)) & 1u;
+      }
+    }
+    const bool use = valid && s != self && !excl;
+    if (!__any_sync(0xffffffffu, use)) continue;  // e.g. the warp's own vesicle
+    const double2 shi = p.src_hi[s];
+    const double tx = tl.x + (th.x - shi.x), ty = tl.y + (th.y - shi.y);
+    const double rc2 = tx * tx + ty * ty;
+    const double irc2 = 1.0 / rc2;
+    const int j0 = c * p.chunk, j1 = min(p.ns, j0 + p.chunk);
+    const Rec64* S = p.src + (long long)s * p.ns;
+    double acx = 0, acy = 0, alx = 0, aly = 0;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+      const double2 a = __ldg(reinterpret_cast<const double2*>(S + j));
+      const double2 b = __ldg(reinterpret_cast<const double2*>(S + j) + 1);
+      const double dx = tx - a.x, dy = ty - a.y;
+      const double r2 = fma(dx, dx, dy * dy);
+      const double inv = 1.0 / r2;
+      const double lg = log2(r2 * irc2);
+      const double cc = fma(dx, b.x, dy * b.y) * inv;
+      acx = fma(cc, dx, acx);
+      acy = fma(cc, dy, acy);
+      alx = fma(lg, b.x, alx);
+      aly = fma(lg, b.y, aly);
+    }
+    if (use) {
+      double px = acx - FF_HALF_LN2 * alx, py = acy - FF_HALF_LN2 * aly;
+      if (c == 0) {
+        const double2 ds = p.src_dsum[s];
+        const double lgc = FF_HALF_LN2 * log2(rc2);
+        px = fma(-lgc, ds.x, px);
+        py = fma(-lgc, ds.y, py);
+      }
+      double t = tot_x + px;  // Neumaier compensated accumulation
+      cmp_x += (fabs(tot_x) >= fabs(px)) ? (tot_x - t) + px : (px - t) + tot_x;
+      tot_x = t;
+      t = tot_y + py;
+      cmp_y += (fabs(tot_y) >= fabs(py)) ? (tot_y - t) + py : (py - t) + tot_y;
+      tot_y = t;
+    }
+  }
+  if (valid) {
+    double* o = p.partial + ((long long)blockIdx.y * p.total_pts + pt) * 2;
+    o[0] = tot_x + cmp_x;
+    o[1] = tot_y + cmp_y;
+  }
+}
+
+// out[col][c][pidx] = sum over splits (fixed order: eight strided partial
+// sums per point, then a fixed tree) / (4 pi); 32 points per CTA
+__global__ void __launch_bounds__(256) ff64_reduce_kernel(long long total_pts, int ntp, int nsplit,
+                                                          const double* __restrict__ partial,
+                                                          double* __restrict__ out) {
+  __shared__ double2 red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long pt = (long long)blockIdx.x * 32 + lane;
+  double2 a = make_double2(0.0, 0.0);
+  if (pt < total_pts)
+    for (int s = w; s < nsplit; s += 8) {
+      const double2 v = *reinterpret_cast<const double2*>(partial + ((long long)s * total_pts + pt) * 2);
+      a.x += v.x;
+      a.y += v.y;
+    }
+  red[w][lane] = a;
+  __syncthreads();
+  if (w != 0 || pt >= total_pts) return;
+  for (int h = 4; h > 0; h >>= 1)
+    for (int q = 0; q < h; ++q) {
+      red[q][lane].x += red[q + h][lane].x;
+      red[q][lane].y += red[q + h][lane].y;
+    }
+  const long long col = pt / ntp, j = pt % ntp;
+  const double scale = 1.0 / (4.0 * VES_PI);
+  out[col * 2 * ntp + j] = red[0][lane].x * scale;
+  out[col * 2 * ntp + ntp + j] = red[0][lane].y * scale;
+}
+
 struct FFPlan {
   int sv_per_stage, nsplit, src_per_split, tgt_blocks;
   size_t smem;
@@ -472,13 +600,98 @@ int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double*
   return ves_launch_check("farfield");
 }
 
+struct FF64Plan {
+  int tgt_blocks, nchunk, chunk, per_split, nsplit;
+};
+
+// Pieces of at least 16 points (below that the per-piece centre terms, one
+// log and one divide, are over a tenth of the work), as many splits as give
+// 16 CTAs of 4 warps per SM (two rounds of resident CTAs).  The partial sums
+// fit in what the staged plan of whole vesicles took, or in 32 MiB with the
+// records: a caller's fixed scratch holds every size that it held.
+FF64Plan ff64_plan(int nsrc, int ns, long long total_pts) {
+  FF64Plan pl;
+  const long long tb = (total_pts + FF64_THREADS - 1) / FF64_THREADS;
+  pl.tgt_blocks = (int)tb;
+  long long want = tb > 0 ? (152LL * 16 + tb - 1) / tb : 1;
+  const long long held = ff_plan<double>(nsrc, ns, total_pts).nsplit;
+  const long long base = (long long)nsrc * ns * (long long)sizeof(Rec64), room = (32LL << 20) - base;
+  const long long fit = total_pts > 0 && room > 0 ? room / (total_pts * 16) : 0;
+  want = std::max(1LL, std::min(want, std::max(held, fit)));
+  const long long most = std::max(1, ns / 16);
+  pl.nchunk = (int)std::max(1LL, std::min(most, nsrc > 0 ? (want + nsrc - 1) / nsrc : 1));
+  pl.chunk = (ns + pl.nchunk - 1) / pl.nchunk;
+  pl.nchunk = (ns + pl.chunk - 1) / pl.chunk;
+  const long long units = (long long)nsrc * pl.nchunk;
+  pl.per_split = (int)std::max(1LL, (units + want - 1) / want);
+  pl.nsplit = (int)std::max(1LL, (units + pl.per_split - 1) / pl.per_split);
+  return pl;
+}
+
+int ff64_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double* den, int nt, int ntp,
+             const double* Xtar, const int* self_idx, const ves_near_lists* nl, double* out, WsCarver& ws,
+             cudaStream_t s) {
+  const long long total_pts = (long long)nt * ntp;
+  const FF64Plan pl = ff64_plan(nsrc, ns, total_pts);
+  Rec64* rec = ws.take<Rec64>((size_t)nsrc * ns);
+  double2* shi = ws.take<double2>(nsrc);
+  double2* slo = ws.take<double2>(nsrc);
+  double2* dsum = ws.take<double2>(nsrc);
+  double2* tloc = ws.take<double2>((size_t)total_pts);
+  double2* thi = ws.take<double2>(nt);
+  double2* tlo = ws.take<double2>(nt);
+  double* partial = ws.take<double>((size_t)pl.nsplit * total_pts * 2);
+  if (ws.sizing) return VES_OK;
+  if (!ws.ok()) {
+    ves_record_error(VES_ERR_WORKSPACE, "farfield: workspace too small");
+    return VES_ERR_WORKSPACE;
+  }
+  if (total_pts == 0) return VES_OK;
+  if (nsrc == 0) return ves_cuda_status(cudaMemsetAsync(out, 0, (size_t)total_pts * 2 * sizeof(double), s), "ff zero");
+  if (nl && ntp != env.N) {
+    ves_record_error(VES_ERR_SHAPE, "farfield: near lists need N target points per column");
+    return VES_ERR_SHAPE;
+  }
+  ves_count_launch(2);
+  ff_prep_kernel<double><<<nsrc, 256, 0, s>>>(ns, Xsrc, den, rec, nullptr, shi, slo, dsum);
+  ff_prep_kernel<double><<<nt, 256, 0, s>>>(ntp, Xtar, nullptr, nullptr, tloc, thi, tlo, nullptr);
+  FF64Args a;
+  a.nsrc = nsrc;
+  a.ns = ns;
+  a.ntp = ntp;
+  a.total_pts = total_pts;
+  a.src = rec;
+  a.src_hi = shi;
+  a.src_dsum = dsum;
+  a.tgt_local = tloc;
+  a.tgt_hi = thi;
+  a.self_idx = self_idx;
+  a.cand_count = nl ? nl->cand_count : nullptr;
+  a.cand_src = nl ? nl->cand_src : nullptr;
+  a.excl_mask = nl ? nl->excl_mask : nullptr;
+  a.maxc = nl ? nl->maxc : 0;
+  a.nwords = (env.N + 31) / 32;
+  a.nchunk = pl.nchunk;
+  a.chunk = pl.chunk;
+  a.per_split = pl.per_split;
+  a.nsplit = pl.nsplit;
+  a.partial = partial;
+  ves_count_launch();
+  if (env.timing) ves_ff_timing_begin(env.timing, s);
+  ff64_kernel<<<dim3(pl.tgt_blocks, pl.nsplit), FF64_THREADS, 0, s>>>(a);
+  if (env.timing) ves_ff_timing_end(env.timing, s, (double)total_pts * ns * (double)nsrc);
+  ves_count_launch();
+  ff64_reduce_kernel<<<ceil_div(total_pts, 32), 256, 0, s>>>(total_pts, ntp, pl.nsplit, partial, out);
+  return ves_launch_check("farfield");
+}
+
 }  // namespace
 
 int farfield_run_env(const FFEnv& env, int precision, int nsrc, int ns, const double* Xsrc, const double* den,
                      int nt, int ntp, const double* Xtar, const int* self_idx, const ves_near_lists* nl,
                      double* out, WsCarver& ws, cudaStream_t s) {
   if (precision == VES_PREC_FP64)
-    return ff_run<double>(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
+    return ff64_run(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
   if (precision == VES_PREC_FP32C)
     return ff_run<float>(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
   if (precision == VES_PREC_FP32M)
