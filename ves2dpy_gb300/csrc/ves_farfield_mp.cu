@@ -34,14 +34,15 @@
 // the series are evaluated in FP32 (Horner) and the per-source contributions
 // are added with Neumaier compensation.
 #include "ves_internal.h"
+#include "ves_tc.cuh"
 
 namespace {
 
 constexpr int kPMax = 24;                 // highest expansion order
 constexpr float kRhoMax = 0.35f;          // 0.35^25 / 0.65 < 1e-11
 constexpr float kEps = 1e-10f;            // truncation bound relative to sum |f_j|
-constexpr int kStage = 16;                // source vesicles per shared-memory stage
-constexpr int kDrecChunk = 512;           // direct-rule points per shared-memory stage (8 KB)
+constexpr int kStage = 32;                // source vesicles per shared-memory stage
+constexpr int kLow = 13;                  // orders 0 .. kLow - 1 of a source are staged, the others read from L2
 constexpr double kHalfLn2 = 0.34657359027997264;
 
 struct __align__(16) MPSrc {
@@ -51,10 +52,17 @@ struct __align__(16) MPSrc {
   float pad;
 };
 
-// one order k of one source: Al = A_k/(2k) (0 at k=0), Bc = conj(B_k/(2k)) (0 at k=0), A_k, E_k
+// one order k of one source: Al = A_k/(2k) (0 at k=0), Bc = conj(B_k/(2k))
+// (0 at k=0), A_k, E_k, the real and the imaginary parts of (Al, Bc) and of
+// (A, E) side by side, as the packed FP32x2 Horner steps take them
 struct __align__(16) MPMom {
-  float2 al, bc, ac, ec;
+  float2 abr, abi, aer, aei;
 };
+// order k of source s: the low orders of every source come first, so that a
+// stage of sources is one contiguous copy
+__host__ __device__ inline long long mom_at(int nsrc, int s, int k) {
+  return k < kLow ? (long long)s * kLow + k : (long long)nsrc * kLow + (long long)s * (kPMax + 1 - kLow) + (k - kLow);
+}
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
@@ -67,6 +75,7 @@ __global__ void __launch_bounds__(256) mp_prep_kernel(int ns, const double* __re
                                                       const double* __restrict__ den, float4* __restrict__ rec,
                                                       MPSrc* __restrict__ src, MPMom* __restrict__ mom) {
   __shared__ double red[3][256];
+  __shared__ float4 pts[256];  // (v, f) of 256 points
   const int s = blockIdx.x, t = threadIdx.x;
   const double* x = X + (long long)s * 2 * ns;
   const double* f = den + (long long)s * 2 * ns;
@@ -129,27 +138,39 @@ __global__ void __launch_bounds__(256) mp_prep_kernel(int ns, const double* __re
 #pragma unroll
   for (int q = 0; q < kPer; ++q) A[q] = B[q] = E[q] = make_float2(0.f, 0.f);
   const double iR = 1.0 / R;
-  for (int j = lane; j < ns; j += 32) {
-    const float2 v = make_float2((float)((x[j] - cx) * iR), (float)((x[ns + j] - cy) * iR));
-    const float2 fj = make_float2((float)f[j], (float)f[ns + j]);
-    float2 pw = make_float2(1.f, 0.f), v8 = v;  // pw = v^warp, v8 = v^8
-    for (int e = 0; e < warp; ++e) pw = cmulf(pw, v);
-    v8 = cmulf(v8, v8);
-    v8 = cmulf(v8, v8);
-    v8 = cmulf(v8, v8);
-    const float2 fvb = cmulf(fj, make_float2(v.x, -v.y));  // f conj(v)
+  for (int c0 = 0; c0 < ns; c0 += 256) {
+    // each point scaled once (FP64 is the slow pipe: 80 of 262 us at 1024 x
+    // N=128 went on every warp scaling every point) and read by every warp
+    __syncthreads();
+    if (c0 + t < ns) {
+      const int j = c0 + t;
+      pts[t] = make_float4((float)((x[j] - cx) * iR), (float)((x[ns + j] - cy) * iR), (float)f[j], (float)f[ns + j]);
+    }
+    __syncthreads();
+    for (int j = lane; j < min(256, ns - c0); j += 32) {
+      const float4 pt = pts[j];
+      const float2 v = make_float2(pt.x, pt.y);
+      const float2 fj = make_float2(pt.z, pt.w);
+      float2 pw = make_float2(1.f, 0.f), v8 = v;  // pw = v^warp, v8 = v^8
+      for (int e = 0; e < warp; ++e) pw = cmulf(pw, v);
+      v8 = cmulf(v8, v8);
+      v8 = cmulf(v8, v8);
+      v8 = cmulf(v8, v8);
+      const float2 fvb = cmulf(fj, make_float2(v.x, -v.y));  // f conj(v)
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const float2 a = cmulf(fj, pw);
-      const float2 b = cmulf(fj, make_float2(pw.x, -pw.y));
-      const float2 e = cmulf(fvb, pw);
-      A[q].x += a.x;
-      A[q].y += a.y;
-      B[q].x += b.x;
-      B[q].y += b.y;
-      E[q].x += e.x;
-      E[q].y += e.y;
-      pw = cmulf(pw, v8);
+      for (int q = 0; q < kPer; ++q) {
+        if (warp + 8 * q > kPMax) break;
+        const float2 a = cmulf(fj, pw);
+        const float2 b = cmulf(fj, make_float2(pw.x, -pw.y));
+        const float2 e = cmulf(fvb, pw);
+        A[q].x += a.x;
+        A[q].y += a.y;
+        B[q].x += b.x;
+        B[q].y += b.y;
+        E[q].x += e.x;
+        E[q].y += e.y;
+        pw = cmulf(pw, v8);
+      }
     }
   }
 #pragma unroll
@@ -166,11 +187,12 @@ __global__ void __launch_bounds__(256) mp_prep_kernel(int ns, const double* __re
     if (lane == 0 && k <= kPMax) {
       MPMom m;
       const float h = k > 0 ? 0.5f / k : 0.f;
-      m.al = make_float2(A[q].x * h, A[q].y * h);
-      m.bc = make_float2(B[q].x * h, -B[q].y * h);
-      m.ac = k > 0 ? A[q] : make_float2((float)red[1][0], (float)red[2][0]);  // A_0 = F0 (FP64 sum)
-      m.ec = E[q];
-      mom[(long long)s * (kPMax + 1) + k] = m;
+      const float2 ac = k > 0 ? A[q] : make_float2((float)red[1][0], (float)red[2][0]);  // A_0 = F0 (FP64 sum)
+      m.abr = make_float2(A[q].x * h, B[q].x * h);
+      m.abi = make_float2(A[q].y * h, -B[q].y * h);
+      m.aer = make_float2(ac.x, E[q].x);
+      m.aei = make_float2(ac.y, E[q].y);
+      mom[mom_at(gridDim.x, s, k)] = m;
     }
   }
 }
@@ -206,270 +228,334 @@ __global__ void __launch_bounds__(256) mp_prep_targets_kernel(int ntp, const dou
   }
 }
 
-__device__ __forceinline__ void neumaier(float& tot, float& cmp, float v) {
-  const float t = tot + v;
-  cmp += (fabsf(tot) >= fabsf(v)) ? (tot - t) + v : (v - t) + tot;
-  tot = t;
-}
-
 // One source set (the upsampled points of one group of vesicles).
 struct MPSet {
   int nsrc, ns;
   const float4* rec;  // [nsrc][ns] direct-rule records
   const MPSrc* src;   // [nsrc]
-  const MPMom* mom;   // [nsrc][kPMax + 1]
+  const MPMom* mom;   // moments, see mom_at
 };
 
-// The near-candidate list of one target column against one source set.
-struct MPNearCol {
-  int self;              // source index of the target's own vesicle, or -1
-  int cend;              // candidates on the list
-  const int* cands;      // ascending source indices
-  const uint32_t* excl;  // [maxc][nwords] excluded target points per candidate
-  int nwords;
-};
-
-// Per-CTA staging of the source records and moments.
-struct MPStage {
-  MPSrc* src;                 // [kStage]
-  MPMom (*mom)[kPMax + 1];    // [kStage][kPMax + 1]
-  float4* drec;               // [ns] direct-rule records of one source
-};
-
-// Sum over every source of one set onto this thread's target point (tl
-// relative to the target centre thi + tlo, RT the target radius): the
-// expansion for well-separated pairs, the direct rule for the others and for
-// every pair on the near list (excluded points dropped); the target's own
-// vesicle is skipped.  Uniform control flow across the CTA.
-__device__ __forceinline__ void mp_sum_set(const MPSet& S, const MPNearCol& nr, const MPStage& st, int i, bool valid,
-                                           float2 tl, float2 thi, float2 tlo, float RT, float& tot_x, float& tot_y,
-                                           float& cmp_x, float& cmp_y, unsigned long long& terms,
-                                           unsigned long long& ndirect) {
-  int cur = 0;
-  for (int s0 = 0; s0 < S.nsrc; s0 += kStage) {
-    const int nst = min(kStage, S.nsrc - s0);
-    __syncthreads();
-    for (int q = i; q < nst; q += blockDim.x) st.src[q] = S.src[s0 + q];
-    for (int q = i; q < nst * (kPMax + 1); q += blockDim.x)
-      (&st.mom[0][0])[q] = S.mom[(long long)s0 * (kPMax + 1) + q];
-    __syncthreads();
-    for (int q = 0; q < nst; ++q) {
-      const int s = s0 + q;
-      if (s == nr.self) continue;
-      const MPSrc Sq = st.src[q];
-      // target relative to the source centre (hi/lo: no cancellation from absolute positions)
-      const float ox = (thi.x - Sq.chi.x) + (tlo.x - Sq.clo.x);
-      const float oy = (thi.y - Sq.chi.y) + (tlo.y - Sq.clo.y);
-      // near-candidate list of this column: ascending source indices
-      bool cand = false;
-      int cidx = 0;
-      if (nr.cend > 0) {
-        while (cur < nr.cend && nr.cands[cur] < s) ++cur;
-        cand = cur < nr.cend && nr.cands[cur] == s;
-        cidx = cur;
-      }
-      const float dc = sqrtf(ox * ox + oy * oy) - RT;
-      const float rp = dc > 0.f ? Sq.R / dc : 2.f;
-      if (!cand && rp <= kRhoMax) {
-        // expansion of order P: rp^(P+1) / (1 - rp) <= kEps
-        int P = rp > 0.f ? (int)ceilf(__logf(kEps * (1.f - rp)) / __logf(rp)) - 1 : 1;
-        P = max(1, min(P, kPMax));
-        terms += (unsigned long long)(P + 1);
-        const float tx = tl.x + ox, ty = tl.y + oy;  // omega
-        const float om2 = fmaf(tx, tx, ty * ty);
-        const float iom2 = mufu_rcp(om2);
-        const float ur = Sq.R * tx * iom2, ui = -Sq.R * ty * iom2;  // tau = R / omega
-        float2 hA = st.mom[q][P].al, hB = st.mom[q][P].bc, hC = st.mom[q][P].ac, hE = st.mom[q][P].ec;
-        for (int k = P - 1; k >= 0; --k) {
-          const MPMom m = st.mom[q][k];
-          float2 n;
-          n.x = fmaf(hA.x, ur, fmaf(-hA.y, ui, m.al.x));
-          n.y = fmaf(hA.x, ui, fmaf(hA.y, ur, m.al.y));
-          hA = n;
-          n.x = fmaf(hB.x, ur, fmaf(-hB.y, ui, m.bc.x));
-          n.y = fmaf(hB.x, ui, fmaf(hB.y, ur, m.bc.y));
-          hB = n;
-          n.x = fmaf(hC.x, ur, fmaf(-hC.y, ui, m.ac.x));
-          n.y = fmaf(hC.x, ui, fmaf(hC.y, ur, m.ac.y));
-          hC = n;
-          n.x = fmaf(hE.x, ur, fmaf(-hE.y, ui, m.ec.x));
-          n.y = fmaf(hE.x, ui, fmaf(hE.y, ur, m.ec.y));
-          hE = n;
-        }
-        const float lnom = (float)kHalfLn2 * mufu_lg2(om2);  // log|omega|
-        // (omega / conj(omega)) conj(hC) and conj(tau hE)
-        const float qr = (tx * tx - ty * ty) * iom2, qi = 2.f * tx * ty * iom2;
-        const float wcr = qr * hC.x + qi * hC.y, wci = qi * hC.x - qr * hC.y;
-        const float ter = ur * hE.x - ui * hE.y, tei = -(ur * hE.y + ui * hE.x);
-        const float px = fmaf(-lnom, Sq.f0.x, 0.5f * Sq.f0.x) + hA.x + hB.x + 0.5f * (wcr - ter);
-        const float py = fmaf(-lnom, Sq.f0.y, 0.5f * Sq.f0.y) + hA.y - hB.y + 0.5f * (wci - tei);
-        if (valid) {
-          neumaier(tot_x, cmp_x, px);
-          neumaier(tot_y, cmp_y, py);
-        }
-      } else {
-        // direct rule over the upsampled points (FP32, log relative to the
-        // source centre), staged kDrecChunk points at a time (the same order
-        // of summation as one stage)
-        ++ndirect;
-        const float4* R4 = S.rec + (long long)s * S.ns;
-        bool excl = false;
-        if (cand && valid) {
-          const uint32_t w = nr.excl[(long long)cidx * nr.nwords + (i >> 5)];
-          excl = (w >> (i & 31)) & 1u;
-        }
-        const float tx = tl.x + ox, ty = tl.y + oy;
-        const float rc2 = fmaf(tx, tx, ty * ty);
-        const float irc2 = mufu_rcp(rc2);
-        float acx = 0.f, acy = 0.f, alx = 0.f, aly = 0.f;
-        for (int j0 = 0; j0 < S.ns; j0 += kDrecChunk) {
-          const int nj = min(kDrecChunk, S.ns - j0);
-          __syncthreads();
-          for (int j = i; j < nj; j += blockDim.x) st.drec[j] = R4[j0 + j];
-          __syncthreads();
-#pragma unroll 4
-          for (int j = 0; j < nj; ++j) {
-            const float4 r = st.drec[j];
-            const float dx = tx - r.x, dy = ty - r.y;
-            const float r2 = fmaf(dx, dx, dy * dy);
-            const float inv = mufu_rcp(r2);
-            const float lg = mufu_lg2(r2 * irc2);
-            const float cc = fmaf(dx, r.z, dy * r.w) * inv;
-            acx = fmaf(cc, dx, acx);
-            acy = fmaf(cc, dy, acy);
-            alx = fmaf(lg, r.z, alx);
-            aly = fmaf(lg, r.w, aly);
-          }
-        }
-        if (valid && !excl) {
-          const float lgc = mufu_lg2(rc2);
-          const float px = acx - (float)kHalfLn2 * fmaf(lgc, Sq.f0.x, alx);
-          const float py = acy - (float)kHalfLn2 * fmaf(lgc, Sq.f0.y, aly);
-          neumaier(tot_x, cmp_x, px);
-          neumaier(tot_y, cmp_y, py);
-        }
-      }
-    }
-  }
-}
-
-// radius of the target vesicle about its centre (max over the CTA's valid points)
-__device__ __forceinline__ float mp_target_radius(float2 tl, int i, float* rmax_w) {
-  float rt = sqrtf(tl.x * tl.x + tl.y * tl.y);
-  for (int o = 16; o > 0; o >>= 1) rt = fmaxf(rt, __shfl_xor_sync(0xffffffffu, rt, o));
-  if ((i & 31) == 0) rmax_w[i >> 5] = rt;
-  __syncthreads();
-  float RT = 0.f;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) RT = fmaxf(RT, rmax_w[w]);
-  return RT * (1.0f + 1e-6f);
-}
-
-struct MPArgs {
-  int nsrc, ns, ntp;
-  const float4* rec;
-  const MPSrc* src;
-  const MPMom* mom;
-  const float2* tloc;
-  const float2* thi;
-  const float2* tlo;
-  const int* self_idx;
-  const int* cand_count;
-  const int* cand_src;
-  const uint32_t* excl_mask;
-  int maxc, nwords;
-  double* out;               // [nt][2][ntp], scaled by 1/(4 pi)
-  unsigned long long* work;  // optional: series terms, direct pairs (per target point)
-};
-
-// One CTA per target column (blockDim = ntp rounded up to a warp multiple).
-// Dynamic shared memory: direct-rule records of one source, min(ns,
-// kDrecChunk) float4.
-__global__ void __launch_bounds__(128) mp_eval_kernel(MPArgs p) {
-  extern __shared__ __align__(16) float4 drec[];
-  __shared__ MPSrc ssrc[kStage];
-  __shared__ MPMom smom[kStage][kPMax + 1];
-  __shared__ float rmax_w[32];
-  const int col = blockIdx.x, i = threadIdx.x;
-  const bool valid = i < p.ntp;
-  const float2 tl = valid ? p.tloc[(long long)col * p.ntp + i] : make_float2(0.f, 0.f);
-  const float2 thi = p.thi[col], tlo = p.tlo[col];
-  const float RT = mp_target_radius(tl, i, rmax_w);
-  MPSet S{p.nsrc, p.ns, p.rec, p.src, p.mom};
-  MPNearCol nr;
-  nr.self = p.self_idx ? p.self_idx[col] : -1;
-  nr.cend = p.cand_count ? min(p.cand_count[col], p.maxc) : 0;
-  nr.cands = p.cand_src ? p.cand_src + (long long)col * p.maxc : nullptr;
-  nr.excl = p.excl_mask ? p.excl_mask + (long long)col * p.maxc * p.nwords : nullptr;
-  nr.nwords = p.nwords;
-  MPStage st{ssrc, smom, drec};
-  float tot_x = 0.f, tot_y = 0.f, cmp_x = 0.f, cmp_y = 0.f;
-  unsigned long long terms = 0, ndirect = 0;  // work of this column (uniform across the CTA)
-  mp_sum_set(S, nr, st, i, valid, tl, thi, tlo, RT, tot_x, tot_y, cmp_x, cmp_y, terms, ndirect);
-  if (p.work && i == 0) {
-    atomicAdd(&p.work[0], terms * (unsigned long long)p.ntp);
-    atomicAdd(&p.work[1], ndirect * (unsigned long long)p.ntp * (unsigned long long)p.ns);
-  }
-  if (valid) {
-    const double scale = 1.0 / (4.0 * VES_PI);
-    p.out[(long long)col * 2 * p.ntp + i] = ((double)tot_x + (double)cmp_x) * scale;
-    p.out[(long long)col * 2 * p.ntp + p.ntp + i] = ((double)tot_y + (double)cmp_y) * scale;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Several point sets (a suspension of vesicles with different point counts)
-// in one launch: every target column of every set against every source set.
 constexpr int kMPSets = 4;
 
 struct MPGroupArgs {
   int ng;
   MPSet set[kMPSets];            // source sets
-  int col0[kMPSets + 1];         // first target column of each target set
-  int ntp[kMPSets];
+  int cta0[kMPSets + 1];         // first CTA of each target set
+  int upc[kMPSets];              // warps' worth of points (units) per target column
+  int nt[kMPSets], ntp[kMPSets];
   const float2* tloc[kMPSets];   // [nt][ntp] per target set
-  const float2* thi;             // [total columns]
-  const float2* tlo;
-  double* out[kMPSets];          // [nt][2][ntp] per target set
-  // near lists of target set g against source set q, [g][q]
+  const float2* thi[kMPSets];
+  const float2* tlo[kMPSets];
+  double* out[kMPSets];          // [nt][2][ntp] per target set, scaled by 1/(4 pi)
+  const int* self_idx[kMPSets];  // source index (in the same set) of each column's own vesicle; null: see own
+  int own[kMPSets];              // without self_idx: 1: column = source index, 0: no own vesicle
+  // near lists of target set g against source set q, [g][q]: ascending source indices
   const int* cand_count[kMPSets][kMPSets];
   const int* cand_src[kMPSets][kMPSets];
   const uint32_t* excl_mask[kMPSets][kMPSets];
   int maxc[kMPSets][kMPSets];
   int nwords[kMPSets];
+  unsigned long long* work;      // optional: series terms, direct pairs (per target point)
+  VesDeviceStatus* st;
 };
 
-__global__ void __launch_bounds__(128) mp_eval_groups_kernel(MPGroupArgs p) {
-  extern __shared__ __align__(16) float4 drec[];
-  __shared__ MPSrc ssrc[kStage];
-  __shared__ MPMom smom[kStage][kPMax + 1];
-  __shared__ float rmax_w[32];
-  const int col = blockIdx.x, i = threadIdx.x;
+// Every pair of a stage as one lane of the warp sees it: target centre
+// relative to the source's (hi/lo: no cancellation from absolute positions)
+// and what to do: order P >= 1 of the expansion, 0: the target's own vesicle,
+// < 0: direct rule (-1, or -2 - place on the near list).
+struct __align__(16) MPPair {
+  float ox, oy, R;
+  int code;
+};
+
+// Compensated addition of one source's contribution to (x, y) totals; the
+// error term of the rounded sum is exact (Knuth's TwoSum).
+__device__ __forceinline__ void two_sum(float2& tot, float2& cmp, float2 v) {
+  const float2 m1 = make_float2(-1.f, -1.f);  // a - b as fma(b, -1, a): the same rounding
+  const float2 t = __fadd2_rn(tot, v);
+  const float2 z = __ffma2_rn(tot, m1, t);
+  const float2 a = __ffma2_rn(__ffma2_rn(z, m1, t), m1, tot), b = __ffma2_rn(z, m1, v);
+  cmp = __fadd2_rn(cmp, __fadd2_rn(a, b));
+  tot = t;
+}
+
+// One Horner step of the four series, two to a packed FP32x2 register pair
+// (A/2k with conj B/2k, A with E): h = h tau + m.  u = (ur, ur), w = (ui, ui),
+// mw = (-ui, -ui).
+__device__ __forceinline__ void horner(float2& xr, float2& xi, float2& yr, float2& yi, const MPMom& m, float2 u,
+                                       float2 w, float2 mw) {
+  const float2 a = __ffma2_rn(xr, u, __ffma2_rn(xi, mw, m.abr));
+  xi = __ffma2_rn(xr, w, __ffma2_rn(xi, u, m.abi));
+  xr = a;
+  const float2 b = __ffma2_rn(yr, u, __ffma2_rn(yi, mw, m.aer));
+  yi = __ffma2_rn(yr, w, __ffma2_rn(yi, u, m.aei));
+  yr = b;
+}
+
+// Sum over the sources of every set onto the target points of every set.
+//
+// Bound by instruction issue: 16 fma per series term (about 6 terms per
+// separated pair) and ~60 operations more per pair.  A warp owns 32 points of
+// one target column (one unit); the warps of a CTA share the staged sources
+// (kLow orders of 32 bytes and one record each, by bulk copy, two stages in
+// flight).  What depends on the pair of vesicles alone (offset, order of the
+// expansion, place on the near list) is worked out once per warp, one source
+// per lane, and read back as a broadcast; the four complex Horner recurrences
+// run as packed FP32x2 fmas, two series to a register pair, which halves the
+// instructions per term.  Close pairs run the direct rule on records staged
+// 32 at a time by the warp itself, so no warp waits for another's close pairs
+// inside a stage.  Five CTAs of four warps per SM (102 registers): with 80
+// registers the direct rule's loads and MUFU results are not overlapped, with
+// 128 the series wait.  One sum, before (one column per CTA, every thread
+// working out every pair, all 25 orders staged) and now: 8192 x N=32 32.6 ->
+// 13.3 ms, 4096 x N=128 20.7 -> 15.0, 1024 x N=128 2.44 -> 2.05, 333 x N=64
+// 0.49 -> 0.23.  Two points per lane, which halves the operand loads, was
+// slower (20.4 and 19.6 ms on the first two): 96 registers are too few for it.
+//
+// S warps share one unit when there are too few units to fill the chip: they
+// take the sources of a stage in turn and leave the contributions in shared
+// memory, where the unit's first warp adds them in source order.  A point's
+// contributions are always added in source order, so the result does not
+// depend on S.
+template <int WARPS, int S>
+__global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_kernel(MPGroupArgs p) {
+  constexpr int kUnits = WARPS / S;
+  __shared__ __align__(128) MPMom smom[2][kStage * kLow];
+  __shared__ __align__(16) MPSrc ssrc[2][kStage];
+  __shared__ MPPair pairs[WARPS][kStage];
+  __shared__ float4 drec[WARPS][32];
+  __shared__ float2 part[S > 1 ? 2 : 1][S > 1 ? kUnits : 1][S > 1 ? kStage : 1][32];
+  __shared__ int turn[2][kUnits];
+  __shared__ uint64_t bar[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int unit = warp / S, sub = warp % S;
   int g = 0;
-  while (g + 1 < p.ng && col >= p.col0[g + 1]) ++g;
-  const int lc = col - p.col0[g], ntp = p.ntp[g];
-  const bool valid = i < ntp;
-  const float2 tl = valid ? p.tloc[g][(long long)lc * ntp + i] : make_float2(0.f, 0.f);
-  const float2 thi = p.thi[col], tlo = p.tlo[col];
-  const float RT = mp_target_radius(tl, i, rmax_w);
-  MPStage st{ssrc, smom, drec};
-  float tot_x = 0.f, tot_y = 0.f, cmp_x = 0.f, cmp_y = 0.f;
-  unsigned long long terms = 0, ndirect = 0;
-  for (int q = 0; q < p.ng; ++q) {
-    MPNearCol nr;
-    nr.self = q == g ? lc : -1;
+  while (g + 1 < p.ng && (int)blockIdx.x >= p.cta0[g + 1]) ++g;
+  const int ntp = p.ntp[g], upc = p.upc[g];
+  const long long u = (long long)(blockIdx.x - p.cta0[g]) * kUnits + unit;
+  const bool live = u < (long long)p.nt[g] * upc;
+  const int col = live ? (int)(u / upc) : 0;
+  const int i = (live ? (int)(u % upc) : 0) * 32 + lane;
+  const bool valid = live && i < ntp;
+  const float2* tl_col = p.tloc[g] + (long long)col * ntp;
+  const float2 tl = valid ? tl_col[i] : make_float2(0.f, 0.f);
+  const float2 thi = p.thi[g][col], tlo = p.tlo[g][col];
+  // radius of the target vesicle about its centre
+  float RT = 0.f;
+  for (int k = lane; k < ntp; k += 32) {
+    const float2 t = tl_col[k];
+    RT = fmaxf(RT, sqrtf(t.x * t.x + t.y * t.y));
+  }
+  for (int o = 16; o > 0; o >>= 1) RT = fmaxf(RT, __shfl_xor_sync(0xffffffffu, RT, o));
+  RT = RT * (1.0f + 1e-6f);
+  if (threadIdx.x == 0) {
+    tc_mbar_init(&bar[0], 1);
+    tc_mbar_init(&bar[1], 1);
+    tc_mbar_fence_init();
+    tc_fence_async_smem();
+  }
+  if (threadIdx.x < 2 * kUnits) turn[threadIdx.x / kUnits][threadIdx.x % kUnits] = 0;
+  __syncthreads();
+  float2 tot = make_float2(0.f, 0.f), cmp = make_float2(0.f, 0.f);
+  unsigned terms = 0, ndirect = 0;
+  int kst = 0;  // stages so far: stage buffers and barrier phases alternate
+  bool failed = false;
+  for (int q = 0; q < p.ng && !failed; ++q) {
+    const MPSet& set = p.set[q];
+    const int nstages = (set.nsrc + kStage - 1) / kStage;
+    auto fetch = [&](int st, int buf) {  // thread 0
+      const int s0 = st * kStage, n = min(kStage, set.nsrc - s0);
+      tc_expect_tx(&bar[buf], (uint32_t)(n * (kLow * sizeof(MPMom) + sizeof(MPSrc))));
+      tc_bulk_g2s(smom[buf], set.mom + (long long)s0 * kLow, (uint32_t)(n * kLow * sizeof(MPMom)), &bar[buf]);
+      tc_bulk_g2s(ssrc[buf], set.src + s0, (uint32_t)(n * sizeof(MPSrc)), &bar[buf]);
+    };
+    if (threadIdx.x == 0)
+      for (int st = 0; st < 2 && st < nstages; ++st) fetch(st, (kst + st) & 1);
+    const int self = q != g ? -1 : (p.self_idx[g] ? p.self_idx[g][col] : (p.own[g] ? col : -1));
     const int mc = p.maxc[g][q];
-    nr.cend = p.cand_count[g][q] ? min(p.cand_count[g][q][lc], mc) : 0;
-    nr.cands = p.cand_src[g][q] ? p.cand_src[g][q] + (long long)lc * mc : nullptr;
-    nr.excl = p.excl_mask[g][q] ? p.excl_mask[g][q] + (long long)lc * mc * p.nwords[g] : nullptr;
-    nr.nwords = p.nwords[g];
-    mp_sum_set(p.set[q], nr, st, i, valid, tl, thi, tlo, RT, tot_x, tot_y, cmp_x, cmp_y, terms, ndirect);
+    const int cend = p.cand_count[g][q] ? min(p.cand_count[g][q][col], mc) : 0;
+    const int* cands = p.cand_src[g][q] ? p.cand_src[g][q] + (long long)col * mc : nullptr;
+    const uint32_t* excl = p.excl_mask[g][q] ? p.excl_mask[g][q] + (long long)col * mc * p.nwords[g] : nullptr;
+    for (int st = 0; st < nstages; ++st, ++kst) {
+      const int buf = kst & 1, s0 = st * kStage, n = min(kStage, set.nsrc - s0);
+      if (!tc_mbar_wait(&bar[buf], (kst >> 1) & 1, p.st, 30)) failed = true;
+      if (lane < n) {
+        const MPSrc Sq = ssrc[buf][lane];
+        const int s = s0 + lane;
+        const float ox = (thi.x - Sq.chi.x) + (tlo.x - Sq.clo.x);
+        const float oy = (thi.y - Sq.chi.y) + (tlo.y - Sq.clo.y);
+        int lo = 0, hi = cend;  // first candidate >= s
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (cands[mid] < s) lo = mid + 1; else hi = mid;
+        }
+        const bool cand = lo < cend && cands[lo] == s;
+        const float dc = sqrtf(ox * ox + oy * oy) - RT;
+        const float rp = dc > 0.f ? Sq.R / dc : 2.f;
+        int code;
+        if (s == self) {
+          code = 0;
+        } else if (!cand && rp <= kRhoMax) {
+          // expansion of order P: rp^(P+1) / (1 - rp) <= kEps
+          const int P = rp > 0.f ? (int)ceilf(__logf(kEps * (1.f - rp)) / __logf(rp)) - 1 : 1;
+          code = max(1, min(P, kPMax));
+        } else {
+          code = cand ? -2 - lo : -1;
+        }
+        if (p.work && live && sub == 0) {
+          terms += code > 0 ? code + 1 : 0;
+          ndirect += code < 0 ? set.ns : 0;
+        }
+        pairs[warp][lane] = MPPair{ox, oy, Sq.R, code};
+      }
+      __syncwarp();
+      for (int qs = 0;; ++qs) {
+        if (S > 1) {  // the unit's warps take the stage's sources in turn
+          if (lane == 0) qs = atomicAdd(&turn[buf][unit], 1);
+          qs = __shfl_sync(0xffffffffu, qs, 0);
+        }
+        if (qs >= n || !live) break;
+        const MPPair pr = pairs[warp][qs];
+        float2 v = make_float2(0.f, 0.f);
+        if (pr.code > 0) {
+          const float tx = tl.x + pr.ox, ty = tl.y + pr.oy;  // omega
+          const float om2 = fmaf(tx, tx, ty * ty);
+          const float iom2 = mufu_rcp(om2);
+          const float ur = pr.R * tx * iom2, ui = -pr.R * ty * iom2;  // tau = R / omega
+          const float2 uu = make_float2(ur, ur), ww = make_float2(ui, ui), mw = make_float2(-ui, -ui);
+          const MPMom* m = smom[buf] + qs * kLow;
+          float2 xr, xi, yr, yi;
+          int k = pr.code;
+          if (k >= kLow) {  // the few orders past the staged ones
+            const MPMom* hm = set.mom + mom_at(set.nsrc, s0 + qs, kLow);
+            const MPMom t = hm[k - kLow];
+            xr = t.abr, xi = t.abi, yr = t.aer, yi = t.aei;
+            for (--k; k >= kLow; --k) horner(xr, xi, yr, yi, hm[k - kLow], uu, ww, mw);
+            ++k;
+          } else {
+            const MPMom t = m[k];
+            xr = t.abr, xi = t.abi, yr = t.aer, yi = t.aei;
+          }
+          switch (k) {  // orders k - 1 .. 0, straight-line
+#define VES_MP_STEP(K) case K + 1: horner(xr, xi, yr, yi, m[K], uu, ww, mw);
+            VES_MP_STEP(12) VES_MP_STEP(11) VES_MP_STEP(10) VES_MP_STEP(9) VES_MP_STEP(8) VES_MP_STEP(7)
+            VES_MP_STEP(6) VES_MP_STEP(5) VES_MP_STEP(4) VES_MP_STEP(3) VES_MP_STEP(2) VES_MP_STEP(1) VES_MP_STEP(0)
+#undef VES_MP_STEP
+            default: break;
+          }
+          const float2 f0 = ssrc[buf][qs].f0;
+          const float lnom = (float)kHalfLn2 * mufu_lg2(om2);  // log|omega|
+          // (omega / conj(omega)) conj(hC) and conj(tau hE)
+          const float qr = (tx * tx - ty * ty) * iom2, qi = 2.f * tx * ty * iom2;
+          const float wcr = qr * yr.x + qi * yi.x, wci = qi * yr.x - qr * yi.x;
+          const float ter = ur * yr.y - ui * yi.y, tei = -(ur * yi.y + ui * yr.y);
+          v.x = fmaf(-lnom, f0.x, 0.5f * f0.x) + xr.x + xr.y + 0.5f * (wcr - ter);
+          v.y = fmaf(-lnom, f0.y, 0.5f * f0.y) + xi.x - xi.y + 0.5f * (wci - tei);
+        } else if (pr.code < 0) {
+          // direct rule over the upsampled points (FP32, log relative to the source centre)
+          const float4* R4 = set.rec + (long long)(s0 + qs) * set.ns;
+          bool ex = false;
+          if (pr.code < -1 && valid) {
+            const uint32_t w = excl[(long long)(-2 - pr.code) * p.nwords[g] + (i >> 5)];
+            ex = (w >> (i & 31)) & 1u;
+          }
+          const float tx = tl.x + pr.ox, ty = tl.y + pr.oy;
+          const float rc2 = fmaf(tx, tx, ty * ty);
+          const float irc2 = mufu_rcp(rc2);
+          float2 ac = make_float2(0.f, 0.f), al = make_float2(0.f, 0.f);
+          float4 nx = lane < set.ns ? R4[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int j0 = 0; j0 < set.ns; j0 += 32) {
+            __syncwarp();
+            drec[warp][lane] = nx;
+            __syncwarp();
+            if (j0 + 32 + lane < set.ns) nx = R4[j0 + 32 + lane];
+            const int nj = min(32, set.ns - j0);
+#pragma unroll 8
+            for (int j = 0; j < nj; ++j) {
+              const float4 r = drec[warp][j];
+              const float dx = tx - r.x, dy = ty - r.y;
+              const float r2 = fmaf(dx, dx, dy * dy);
+              const float inv = mufu_rcp(r2);
+              const float lg = mufu_lg2(r2 * irc2);
+              const float cc = fmaf(dx, r.z, dy * r.w) * inv;
+              ac = __ffma2_rn(make_float2(cc, cc), make_float2(dx, dy), ac);
+              al = __ffma2_rn(make_float2(lg, lg), make_float2(r.z, r.w), al);
+            }
+          }
+          if (!ex) {
+            const float2 f0 = ssrc[buf][qs].f0;
+            const float lgc = mufu_lg2(rc2);
+            v.x = ac.x - (float)kHalfLn2 * fmaf(lgc, f0.x, al.x);
+            v.y = ac.y - (float)kHalfLn2 * fmaf(lgc, f0.y, al.y);
+          }
+        }
+        if (S > 1)
+          part[buf][unit][qs][lane] = v;
+        else
+          two_sum(tot, cmp, v);  // points past the column's end add too; they are not stored
+      }
+      // nobody reads this stage any more (and every contribution is in)
+      failed = __syncthreads_or(failed ? 1 : 0) != 0;
+      if (S > 1) {
+        if (threadIdx.x < kUnits) turn[buf][threadIdx.x] = 0;
+        if (sub == 0)
+          for (int qs = 0; qs < n; ++qs) two_sum(tot, cmp, part[buf][unit][qs][lane]);
+      }
+      if (failed) {  // the copies in flight land before the CTA ends
+        if (threadIdx.x == 0) {
+          tc_mbar_wait(&bar[buf], (kst >> 1) & 1, nullptr, 0);
+          if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((kst + 1) >> 1) & 1, nullptr, 0);
+        }
+        break;
+      }
+      if (threadIdx.x == 0 && st + 2 < nstages) {
+        tc_fence_async_smem();
+        fetch(st + 2, buf);
+      }
+    }
   }
-  if (valid) {
+  if (p.work) {
+    const unsigned long long npt = live ? min(32, ntp - (i - lane)) : 0;
+    terms = __reduce_add_sync(0xffffffffu, terms);
+    ndirect = __reduce_add_sync(0xffffffffu, ndirect);
+    if (lane == 0 && sub == 0) {
+      atomicAdd(&p.work[0], terms * npt);
+      atomicAdd(&p.work[1], ndirect * npt);
+    }
+  }
+  if (valid && sub == 0) {
     const double scale = 1.0 / (4.0 * VES_PI);
-    double* o = p.out[g] + (long long)lc * 2 * ntp;
-    o[i] = ((double)tot_x + (double)cmp_x) * scale;
-    o[ntp + i] = ((double)tot_y + (double)cmp_y) * scale;
+    double* o = p.out[g] + (long long)col * 2 * ntp;
+    o[i] = ((double)tot.x + (double)cmp.x) * scale;
+    o[ntp + i] = ((double)tot.y + (double)cmp.y) * scale;
   }
+}
+
+// Warps per unit: one from nine units per SM on, four from two per SM, eight
+// below.  Measured (one sum, us; S = 1 / 4 / 8): 100 x N=32 (100 units) 195 /
+// 45 / 35, 61 x N=128 (244) 276 / 120 / 118, 600 x N=32 (600) 355 / 163 / 203,
+// 300 x N=128 (1200) 648 / 592 / 835, 1024 x N=128 (4096) 2050 / 2770 / 3990.
+int mp_launch(MPGroupArgs& a, cudaStream_t s) {
+  long long units = 0;
+  for (int g = 0; g < a.ng; ++g) {
+    a.upc[g] = (a.ntp[g] + 31) / 32;
+    units += (long long)a.nt[g] * a.upc[g];
+  }
+  const int S = units >= 152 * 9 ? 1 : units >= 152 * 2 ? 4 : 8;
+  const int per = S == 1 ? 4 : 1;  // units per CTA
+  a.cta0[0] = 0;
+  for (int g = 0; g < a.ng; ++g) a.cta0[g + 1] = a.cta0[g] + (int)(((long long)a.nt[g] * a.upc[g] + per - 1) / per);
+  const int grid = a.cta0[a.ng];
+  if (grid == 0) return VES_OK;
+  ves_count_launch();
+  if (S == 1)
+    mp_eval_kernel<4, 1><<<grid, 128, 0, s>>>(a);
+  else if (S == 4)
+    mp_eval_kernel<4, 4><<<grid, 128, 0, s>>>(a);
+  else
+    mp_eval_kernel<8, 8><<<grid, 256, 0, s>>>(a);
+  return ves_launch_check("farfield multipole");
 }
 
 }  // namespace
@@ -499,44 +585,36 @@ int farfield_mp_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, cons
     ves_record_error(VES_ERR_SHAPE, "farfield: near lists need N target points per column");
     return VES_ERR_SHAPE;
   }
-  const size_t dsmem = (size_t)std::min(ns, kDrecChunk) * sizeof(float4);
   ves_count_launch(2);
   mp_prep_kernel<<<nsrc, 256, 0, s>>>(ns, Xsrc, den, rec, src, mom);
   mp_prep_targets_kernel<<<nt, 256, 0, s>>>(ntp, Xtar, tloc, thi, tlo);
-  MPArgs a;
-  a.nsrc = nsrc;
-  a.ns = ns;
-  a.ntp = ntp;
-  a.rec = rec;
-  a.src = src;
-  a.mom = mom;
-  a.tloc = tloc;
-  a.thi = thi;
-  a.tlo = tlo;
-  a.self_idx = self_idx;
-  a.cand_count = nl ? nl->cand_count : nullptr;
-  a.cand_src = nl ? nl->cand_src : nullptr;
-  a.excl_mask = nl ? nl->excl_mask : nullptr;
-  a.maxc = nl ? nl->maxc : 0;
-  a.nwords = (env.N + 31) / 32;
-  a.out = out;
+  MPGroupArgs a;
+  memset(&a, 0, sizeof(a));
+  a.ng = 1;
+  a.set[0] = MPSet{nsrc, ns, rec, src, mom};
+  a.nt[0] = nt;
+  a.ntp[0] = ntp;
+  a.tloc[0] = tloc;
+  a.thi[0] = thi;
+  a.tlo[0] = tlo;
+  a.out[0] = out;
+  a.self_idx[0] = self_idx;
+  a.cand_count[0][0] = nl ? nl->cand_count : nullptr;
+  a.cand_src[0][0] = nl ? nl->cand_src : nullptr;
+  a.excl_mask[0][0] = nl ? nl->excl_mask : nullptr;
+  a.maxc[0][0] = nl ? nl->maxc : 0;
+  a.nwords[0] = (env.N + 31) / 32;
   a.work = (env.timing && env.timing->timing) ? env.timing->d_mp : nullptr;
-  if (dsmem > 32 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(mp_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem);
-    if (e != cudaSuccess) return ves_cuda_status(e, "farfield multipole smem attribute");
-  }
-  const int threads = ((ntp + 31) / 32) * 32;
-  ves_count_launch();
+  a.st = env.status;
   if (env.timing) ves_ff_timing_begin(env.timing, s);
-  mp_eval_kernel<<<nt, threads, dsmem, s>>>(a);
+  const int rc = mp_launch(a, s);
   if (env.timing) ves_ff_timing_end(env.timing, s, (double)total_pts * ns * (double)nsrc);
-  return ves_launch_check("farfield multipole");
+  return rc;
 }
 
 int farfield_mp_groups_run(const FFEnv& env, int ng, const int* nsrc, const int* ns, const double* const* Xsrc,
                            const double* const* den, const int* nt, const int* ntp, const double* const* Xtar,
                            const ves_near_lists* const* nl, double* const* out, WsCarver& ws, cudaStream_t s) {
-  (void)env;
   if (ng < 1 || ng > kMPSets) {
     if (!ws.sizing) ves_record_error(VES_ERR_ARG, "farfield groups: 1 to %d point sets", kMPSets);
     return VES_ERR_ARG;
@@ -546,14 +624,13 @@ int farfield_mp_groups_run(const FFEnv& env, int ng, const int* nsrc, const int*
   MPMom* mom[kMPSets];
   float2* tloc[kMPSets];
   long long cols = 0;
-  int nsmax = 0, ntpmax = 0;
+  int ntpmax = 0;
   for (int g = 0; g < ng; ++g) {
     rec[g] = ws.take<float4>((size_t)nsrc[g] * ns[g]);
     src[g] = ws.take<MPSrc>(nsrc[g]);
     mom[g] = ws.take<MPMom>((size_t)nsrc[g] * (kPMax + 1));
     tloc[g] = ws.take<float2>((size_t)nt[g] * ntp[g]);
     cols += nt[g];
-    nsmax = std::max(nsmax, ns[g]);
     ntpmax = std::max(ntpmax, ntp[g]);
   }
   float2* thi = ws.take<float2>((size_t)cols);
@@ -571,9 +648,8 @@ int farfield_mp_groups_run(const FFEnv& env, int ng, const int* nsrc, const int*
   MPGroupArgs a;
   memset(&a, 0, sizeof(a));
   a.ng = ng;
-  a.thi = thi;
-  a.tlo = tlo;
-  a.col0[0] = 0;
+  a.st = env.status;
+  int col0 = 0;
   for (int g = 0; g < ng; ++g) {
     if (nsrc[g] > 0) {
       ves_count_launch();
@@ -581,13 +657,17 @@ int farfield_mp_groups_run(const FFEnv& env, int ng, const int* nsrc, const int*
     }
     if (nt[g] > 0) {
       ves_count_launch();
-      mp_prep_targets_kernel<<<nt[g], 256, 0, s>>>(ntp[g], Xtar[g], tloc[g], thi + a.col0[g], tlo + a.col0[g]);
+      mp_prep_targets_kernel<<<nt[g], 256, 0, s>>>(ntp[g], Xtar[g], tloc[g], thi + col0, tlo + col0);
     }
     a.set[g] = MPSet{nsrc[g], ns[g], rec[g], src[g], mom[g]};
-    a.col0[g + 1] = a.col0[g] + nt[g];
+    a.nt[g] = nt[g];
     a.ntp[g] = ntp[g];
     a.tloc[g] = tloc[g];
+    a.thi[g] = thi + col0;
+    a.tlo[g] = tlo + col0;
     a.out[g] = out[g];
+    a.own[g] = 1;
+    col0 += nt[g];
     a.nwords[g] = (ntp[g] + 31) / 32;
     for (int q = 0; q < ng; ++q) {
       const ves_near_lists* L = nl ? nl[g * ng + q] : nullptr;
@@ -597,12 +677,5 @@ int farfield_mp_groups_run(const FFEnv& env, int ng, const int* nsrc, const int*
       a.maxc[g][q] = L ? L->maxc : 0;
     }
   }
-  const size_t dsmem = (size_t)std::min(nsmax, kDrecChunk) * sizeof(float4);
-  if (dsmem > 32 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(mp_eval_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem);
-    if (e != cudaSuccess) return ves_cuda_status(e, "farfield groups smem attribute");
-  }
-  ves_count_launch();
-  mp_eval_groups_kernel<<<(unsigned)cols, ((ntpmax + 31) / 32) * 32, dsmem, s>>>(a);
-  return ves_launch_check("farfield groups");
+  return mp_launch(a, s);
 }
