@@ -326,50 +326,75 @@ __global__ void __launch_bounds__(256) py_masks_kernel(int N, int Nup, int maxc,
   for (int i = threadIdx.x; i < wU; i += blockDim.x) hm[i] = hbits[i];
 }
 
-// py_hh correction: one warp per (t, candidate), lanes over hedgehog words
-__global__ void hh_apply_kernel(int nv, int N, int Nup, int maxc, const double* __restrict__ X,
-                                const double* __restrict__ Xup, const int* __restrict__ cand_count,
-                                const int* __restrict__ cand_src, const uint32_t* __restrict__ hh_mask,
-                                const double* __restrict__ vself, double* __restrict__ LP,
-                                double* __restrict__ near_only, int* __restrict__ counter) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  const int lane = threadIdx.x % 32;
-  const int t = gw / maxc, slot = gw % maxc;
-  if (t >= nv || slot >= cand_count[t]) return;
-  const int s = cand_src[(long long)t * maxc + slot];
+// py_hh correction: one CTA per vesicle t.  Latency-bound: a hedgehog point is
+// a search of the N coarse points (FP64 distances), and the points of a close
+// pair sit side by side, that is in one or two words of the mask.  So the
+// warps take the set bits in turn and the lanes share one point's search (a
+// lane per word ran all of a word's searches one after the other: 374 us a
+// call at 301 vesicles of N = 64, 30 us like this).
+__global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, int maxc, const double* __restrict__ X,
+                                                       const double* __restrict__ Xup,
+                                                       const int* __restrict__ cand_count,
+                                                       const int* __restrict__ cand_src,
+                                                       const uint32_t* __restrict__ hh_mask,
+                                                       const double* __restrict__ vself, double* __restrict__ LP,
+                                                       double* __restrict__ near_only) {
+  extern __shared__ double xk[];  // [2][N] coarse points of t (k1 of every pair)
+  const int t = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nc = cand_count[t];
+  if (nc == 0) return;
+  for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) xk[i] = X[(long long)t * 2 * N + i];
+  __syncthreads();
   const int wU = (Nup + 31) / 32;
-  const uint32_t* hm = hh_mask + ((long long)t * maxc + slot) * wU;
-  const double* Xk1 = X + (long long)t * 2 * N;  // k1 = t (coarse vesicle of the pair)
-  for (int w = lane; w < wU; w += 32) {
-    uint32_t bits = hm[w];
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      const int u = w * 32 + b;
-      const long long id1 = (long long)s * Nup + u;
-      const int k2 = (int)(id1 / N), J = (int)(id1 % N);
-      if (k2 >= nv || k2 == t) continue;
-      // closest coarse point of k1 to upsampled point J of vesicle k2 (first minimum)
-      const double px = Xup[(long long)k2 * 2 * Nup + J], py = Xup[(long long)k2 * 2 * Nup + Nup + J];
-      double best = 1e300;
-      int icp = 0;
-      for (int i = 0; i < N; ++i) {
-        const double dx = Xk1[i] - px, dy = Xk1[N + i] - py;
-        const double d2 = dx * dx + dy * dy;
-        if (d2 < best) {
-          best = d2;
-          icp = i;
+  int turn = 0;  // set bits so far: each belongs to one warp
+  for (int slot = 0; slot < nc; ++slot) {
+    const int s = cand_src[(long long)t * maxc + slot];
+    const uint32_t* hm = hh_mask + ((long long)t * maxc + slot) * wU;
+    for (int w0 = 0; w0 < wU; w0 += 32) {
+      const uint32_t word = w0 + lane < wU ? hm[w0 + lane] : 0u;
+      unsigned some = __ballot_sync(0xffffffffu, word != 0u);
+      while (some) {
+        const int wl = __ffs(some) - 1;
+        some &= some - 1;
+        uint32_t bits = __shfl_sync(0xffffffffu, word, wl);
+        while (bits) {
+          const int b = __ffs(bits) - 1;
+          bits &= bits - 1;
+          if (turn++ % nw != warp) continue;
+          const int u = (w0 + wl) * 32 + b;
+          const long long id1 = (long long)s * Nup + u;
+          const int k2 = (int)(id1 / N), J = (int)(id1 % N);
+          if (k2 >= nv || k2 == t) continue;
+          // closest coarse point of k1 to upsampled point J of vesicle k2 (first minimum)
+          const double px = Xup[(long long)k2 * 2 * Nup + J], py = Xup[(long long)k2 * 2 * Nup + Nup + J];
+          double best = 1e300;
+          int icp = 0x7fffffff;
+          for (int i = lane; i < N; i += 32) {
+            const double dx = xk[i] - px, dy = xk[N + i] - py;
+            const double d2 = dx * dx + dy * dy;
+            if (d2 < best) {
+              best = d2;
+              icp = i;
+            }
+          }
+          for (int o = 16; o > 0; o >>= 1) {
+            const double d2 = __shfl_xor_sync(0xffffffffu, best, o);
+            const int i2 = __shfl_xor_sync(0xffffffffu, icp, o);
+            if (d2 < best || (d2 == best && i2 < icp)) {
+              best = d2;
+              icp = i2;
+            }
+          }
+          if (icp == 0x7fffffff) icp = 0;  // no finite distance
+          const int pn0 = ((icp - 3) % N + N) % N;
+          if (lane < 2) {  // one component each
+            const double v = vself[(long long)t * 2 * N + lane * N + pn0];
+            atomicAdd(&LP[(long long)k2 * 2 * N + lane * N + J], v);
+            if (near_only) atomicAdd(&near_only[(long long)k2 * 2 * N + lane * N + J], v);
+          }
         }
       }
-      const int pn0 = ((icp - 3) % N + N) % N;
-      const double vx = vself[(long long)t * 2 * N + pn0], vy = vself[(long long)t * 2 * N + N + pn0];
-      atomicAdd(&LP[(long long)k2 * 2 * N + J], vx);
-      atomicAdd(&LP[(long long)k2 * 2 * N + N + J], vy);
-      if (near_only) {
-        atomicAdd(&near_only[(long long)k2 * 2 * N + J], vx);
-        atomicAdd(&near_only[(long long)k2 * 2 * N + N + J], vy);
-      }
-      if (counter) atomicAdd(counter, 1);
     }
   }
 }
@@ -829,11 +854,9 @@ int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const doubl
     // nearSingInt_rbf: the far field above plus the fits of the near pairs
     if ((rc = rbf_near_correct(c, nv, X, f, vself, nl, LP, ws, s))) return rc;
   } else if (scheme == VES_NEAR_PY_HH) {
-    const long long warps = (long long)nv * nl->maxc;
     ves_count_launch();
-    hh_apply_kernel<<<ceil_div(warps * 32, 256), 256, 0, s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
-                                                              nl->cand_src, nl->hh_mask, vself, LP, near_only,
-                                                              nullptr);
+    hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
+                                                                    nl->cand_src, nl->hh_mask, vself, LP, near_only);
   } else if (scheme == VES_NEAR_MATLAB) {
     const long long warps = nl->max_entries;
     ves_count_launch();
@@ -1021,11 +1044,9 @@ int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const do
                            s);
   if (rc) return rc;
   if (scheme == VES_NEAR_PY_HH) {
-    const long long warps = (long long)nv * nl->maxc;
     ves_count_launch();
-    hh_apply_kernel<<<ceil_div(warps * 32, 256), 256, 0, s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
-                                                              nl->cand_src, nl->hh_mask, vself, LP, near_only,
-                                                              nullptr);
+    hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
+                                                                    nl->cand_src, nl->hh_mask, vself, LP, near_only);
   } else if (scheme == VES_NEAR_MATLAB) {
     const long long warps = nl->max_entries;
     ves_count_launch();
