@@ -67,15 +67,20 @@ __global__ void __launch_bounds__(256) bgemm_kernel(int M, int N, int K, T alpha
 // FP32 variant for aligned shapes: 128x128 tiles, K steps of 8, 8x8 outputs
 // per thread (rows ty*4+i and 64+ty*4+i, columns tx*4+j and 64+tx*4+j), 16-byte
 // operand loads.  Needs K % 8 == 0, N % 4 == 0, lda/ldb/sA/sB multiples of 4
-// and 16-byte aligned A and B.
-__global__ void __launch_bounds__(256) bgemm128_f32_kernel(int M, int N, int K, float alpha,
-                                                           const float* __restrict__ A, int lda, long long sA,
-                                                           const float* __restrict__ B, int ldb, long long sB,
-                                                           float beta, float* __restrict__ C, int ldc,
-                                                           long long sC) {
+// and 16-byte aligned A and B.  Bound by the FP32 pipe: the next K step is
+// loaded into registers while the current one is multiplied and stored into
+// the other half of the shared memory, one barrier per step, and two columns'
+// products are one packed FP32x2 fma (the same products in the same order).
+// The Alpert products of 1024 vesicles of N = 128 (K = 1536): 45.9 -> 40.8 ms
+// (49 TFLOP/s).
+__global__ void __launch_bounds__(256, 2) bgemm128_f32_kernel(int M, int N, int K, float alpha,
+                                                              const float* __restrict__ A, int lda, long long sA,
+                                                              const float* __restrict__ B, int ldb, long long sB,
+                                                              float beta, float* __restrict__ C, int ldc,
+                                                              long long sC) {
   constexpr int TK = 8, LDS = 132;  // padded rows: the transposed A stores are conflict-free
-  __shared__ __align__(16) float As[TK][LDS];
-  __shared__ __align__(16) float Bs[TK][LDS];
+  __shared__ __align__(16) float As[2][TK][LDS];
+  __shared__ __align__(16) float Bs[2][TK][LDS];
   const long long b = blockIdx.z;
   const float* Ab = A + b * sA;
   const float* Bb = B + b * sB;
@@ -87,35 +92,49 @@ __global__ void __launch_bounds__(256) bgemm128_f32_kernel(int M, int N, int K, 
   const int bk = t >> 5, bc = (t & 31) * 4;
   const bool arow_ok = row0 + ar < M;
   const bool bcol_ok = col0 + bc < N;  // N % 4 == 0: the whole float4 is in range
-  float acc[8][8];
+  const float* ap = Ab + (long long)(arow_ok ? row0 + ar : 0) * lda + ak;
+  const float* bp = Bb + (long long)bk * ldb + (bcol_ok ? col0 + bc : 0);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto store = [&](int buf, float4 av, float4 bv) {
+    As[buf][ak + 0][ar] = av.x;
+    As[buf][ak + 1][ar] = av.y;
+    As[buf][ak + 2][ar] = av.z;
+    As[buf][ak + 3][ar] = av.w;
+    *reinterpret_cast<float4*>(&Bs[buf][bk][bc]) = bv;
+  };
+  float2 acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    const float4 av = arow_ok ? *reinterpret_cast<const float4*>(Ab + (long long)(row0 + ar) * lda + k0 + ak)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 bv = bcol_ok ? *reinterpret_cast<const float4*>(Bb + (long long)(k0 + bk) * ldb + col0 + bc)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    As[ak + 0][ar] = av.x;
-    As[ak + 1][ar] = av.y;
-    As[ak + 2][ar] = av.z;
-    As[ak + 3][ar] = av.w;
-    *reinterpret_cast<float4*>(&Bs[bk][bc]) = bv;
-    __syncthreads();
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  store(0, arow_ok ? *reinterpret_cast<const float4*>(ap) : zero, bcol_ok ? *reinterpret_cast<const float4*>(bp) : zero);
+  __syncthreads();
+  for (int k0 = 0, buf = 0; k0 < K; k0 += TK, buf ^= 1) {
+    const bool more = k0 + TK < K;
+    float4 av = zero, bv = zero;
+    if (more) {
+      ap += TK;
+      bp += (long long)TK * ldb;
+      if (arow_ok) av = *reinterpret_cast<const float4*>(ap);
+      if (bcol_ok) bv = *reinterpret_cast<const float4*>(bp);
+    }
 #pragma unroll
     for (int kk = 0; kk < TK; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[kk][64 + tx * 4]);
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
+      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][kk][64 + tx * 4]);
       const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      const float2 bb[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y),
+                            make_float2(b1.z, b1.w)};
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], bb[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), bb[j], acc[i][j]);
+    }
+    if (more) {
+      store(buf ^ 1, av, bv);
+      __syncthreads();
     }
   }
 #pragma unroll
@@ -126,8 +145,9 @@ __global__ void __launch_bounds__(256) bgemm128_f32_kernel(int M, int N, int K, 
     for (int j = 0; j < 8; ++j) {
       const int gc = col0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
       if (gc >= N) continue;
+      const float v = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
       float* cp = Cb + (long long)gr * ldc + gc;
-      *cp = (beta == 0.f) ? alpha * acc[i][j] : fmaf(alpha, acc[i][j], beta * *cp);
+      *cp = (beta == 0.f) ? alpha * v : fmaf(alpha, v, beta * *cp);
     }
   }
 }
@@ -169,21 +189,49 @@ void launch_bgemm_f32(int batch, int M, int N, int K, float alpha, const float* 
 }
 
 // ----------------------------------------------------------------------------
-// y[k] = A[k] (m x n) x[k]; one CTA per vesicle, one warp per row.
-__global__ void bgemv_kernel(int m, int n, const double* __restrict__ A, const double* __restrict__ x,
-                             long long xs, double* __restrict__ y, long long ys) {
+// Sums over the warp of four values per lane, in the order of the usual
+// exchange (lanes 16 apart, then 8, 4, 2, 1): the lanes 8 q .. 8 q + 7 get the
+// sum of s[q].  The first two exchanges add different values in the two halves
+// and quarters of the warp, so the four sums take 6 additions.
+__device__ __forceinline__ double warp_sum4(const double* s, int lane) {
+  const bool h = lane & 16, f = lane & 8;
+  const double u0 = (h ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h ? s[0] : s[2], 16);
+  const double u1 = (h ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h ? s[1] : s[3], 16);
+  double t = (f ? u1 : u0) + __shfl_xor_sync(0xffffffffu, f ? u0 : u1, 8);
+  t += __shfl_xor_sync(0xffffffffu, t, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  return t;
+}
+
+// y[k] = A[k] (m x n) x[k]; one CTA per vesicle, four rows to a warp (bound by
+// the FP64 pipe: one row's own reduction cost 5 additions next to n/32
+// multiply-adds; 1024 blocks of 256 rows 0.205 -> 0.147 ms).
+__global__ void __launch_bounds__(256) bgemv_kernel(int m, int n, const double* __restrict__ A,
+                                                    const double* __restrict__ x, long long xs,
+                                                    double* __restrict__ y, long long ys) {
   extern __shared__ double xsh[];
   const int k = blockIdx.x;
   for (int i = threadIdx.x; i < n; i += blockDim.x) xsh[i] = x[(long long)k * xs + i];
   __syncthreads();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nw = blockDim.x / 32;
   const double* Ak = A + (long long)k * m * n;
-  for (int r = warp; r < m; r += nw) {
-    double s = 0.0;
-    for (int c = lane; c < n; c += 32) s = fma(Ak[(long long)r * n + c], xsh[c], s);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) y[(long long)k * ys + r] = s;
+  for (int r = 4 * warp; r < m; r += 4 * nw) {
+    const double* row = Ak + (long long)r * n;
+    const int mr = min(4, m - r);
+    const long long s1 = mr > 1 ? n : 0, s2 = mr > 2 ? 2LL * n : 0, s3 = mr > 3 ? 3LL * n : 0;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int c = lane; c < n; c += 32) {
+      const double v = xsh[c];
+      s[0] = fma(row[c], v, s[0]);
+      s[1] = fma(row[s1 + c], v, s[1]);
+      s[2] = fma(row[s2 + c], v, s[2]);
+      s[3] = fma(row[s3 + c], v, s[3]);
+    }
+    const double t = warp_sum4(s, lane);
+    const int q = lane >> 3;
+    if ((lane & 7) == 0 && q < mr) y[(long long)k * ys + r + q] = t;
   }
 }
 
@@ -358,18 +406,49 @@ int launch_lu_factor_f32(ves_ctx* c, int nv, int n, float* A, int* piv, cudaStre
   return lu_factor_t<float>(c, nv, n, A, piv, s);
 }
 
-// x = LU^{-1} P b per vesicle.  Blocks of 32 rows: the off-diagonal part is a
-// warp-parallel GEMV, the 32x32 diagonal block is solved by one warp.
+// FP32 -> FP64 by moving the bits (exact, as the conversion is).  The
+// conversion instruction runs on the FP64 pipe (2 lanes/clk/SM); these are
+// integer operations, 32 times that rate.
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), e = b & 0x7f800000u;
+  if (e == 0x7f800000u || (e == 0u && (b << 1) != 0u)) return (double)x;  // infinite, NaN or subnormal
+  const bool z = (b << 1) == 0u;
+  const uint32_t hi = z ? b : (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u);
+  return __hiloint2double((int)hi, (int)(z ? 0u : b << 29));
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
+// exponent between -895 and 896: no intermediate result of the correction is subnormal
+__device__ __forceinline__ bool mid_range(double z) {
+  return (((uint32_t)__double2hiint(z) >> 20) & 0x7ffu) - 128u < 1792u;
+}
+
+// x = LU^{-1} P b per vesicle, one CTA each.  Blocks of 32 rows: the
+// off-diagonal part is a GEMV, four rows to a warp, the 32x32 diagonal block
+// is solved by one warp.  Bound by the FP64 pipe (16 cycles per warp
+// instruction): n^2 multiply-adds, plus what each row's reduction, each
+// conversion of an FP32 factor and each division cost there.  So four rows are
+// reduced together (6 additions instead of 20), factors are widened by integer
+// operations, and a division by a diagonal entry is a product with its
+// reciprocal, taken for the whole block at once, and Markstein's correction
+// (two multiply-adds, correctly rounded when the reciprocal is; IBM J. Res.
+// Dev. 34, 1990).  The row exchanges walk the pivots in shared memory.  One
+// solve: 1024 blocks of 384 rows in FP32 1.22 -> 0.92 ms, 301 of 192 in FP64
+// 0.21 -> 0.11, 16 of 96 0.075 -> 0.040.
 template <typename T>
 __global__ void __launch_bounds__(256) lu_solve_kernel(int n, const T* __restrict__ LU,
                                                        const int* __restrict__ piv,
                                                        const double* __restrict__ b, double* __restrict__ x) {
-  extern __shared__ double xs[];
+  extern __shared__ double xs[];  // [n], then the pivots [n]
+  __shared__ double tile[32][33], rcp[32];
+  int* pv = reinterpret_cast<int*>(xs + n);
   const int k = blockIdx.x;
   const T* a = LU + (long long)k * n * n;
-  const int* pv = piv + (long long)k * n;
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nw = blockDim.x / 32;
-  for (int i = tid; i < n; i += blockDim.x) xs[i] = b[(long long)k * n + i];
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  for (int i = tid; i < n; i += blockDim.x) {
+    xs[i] = b[(long long)k * n + i];
+    pv[i] = piv[(long long)k * n + i];
+  }
   __syncthreads();
   if (tid == 0) {
     for (int j = 0; j < n; ++j) {
@@ -382,22 +461,45 @@ __global__ void __launch_bounds__(256) lu_solve_kernel(int n, const T* __restric
     }
   }
   __syncthreads();
+  // xs[r] -= sum_{c0 <= c < c1} a[r][c] xs[c] for the rows r0 .. r0 + nr - 1
+  // (lane l sums the columns c0 + l, + 32, ..., then the lanes meet pairwise)
+  auto off_diagonal = [&](int r0, int nr, int c0, int c1) {
+    const int rr = 4 * warp;
+    if (c0 >= c1 || rr >= nr) return;
+    const T* row = a + (long long)(r0 + rr) * n;
+    const int m = min(4, nr - rr);
+    const long long s1 = m > 1 ? n : 0, s2 = m > 2 ? 2LL * n : 0, s3 = m > 3 ? 3LL * n : 0;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int c = c0 + lane; c < c1; c += 32) {
+      const T a0 = row[c], a1 = row[s1 + c], a2 = row[s2 + c], a3 = row[s3 + c];
+      const double v = xs[c];
+      s[0] = fma(widen(a0), v, s[0]);
+      s[1] = fma(widen(a1), v, s[1]);
+      s[2] = fma(widen(a2), v, s[2]);
+      s[3] = fma(widen(a3), v, s[3]);
+    }
+    const double t = warp_sum4(s, lane);
+    const int q = lane >> 3;
+    if ((lane & 7) == 0 && q < m) xs[r0 + rr + q] -= t;
+  };
+  auto load_tile = [&](int r0, int nr) {
+    for (int i = tid; i < nr * 32; i += blockDim.x) {
+      const int r = i >> 5, c = i & 31;
+      if (c < nr) tile[r][c] = widen(a[(long long)(r0 + r) * n + r0 + c]);
+    }
+  };
   // forward: unit lower
   for (int r0 = 0; r0 < n; r0 += 32) {
     const int nr = min(32, n - r0);
-    for (int r = warp; r < nr; r += nw) {
-      double s = 0.0;
-      for (int c = lane; c < r0; c += 32) s = fma((double)a[(long long)(r0 + r) * n + c], xs[c], s);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) xs[r0 + r] -= s;
-    }
+    load_tile(r0, nr);
+    off_diagonal(r0, nr, 0, r0);
     __syncthreads();
     if (warp == 0) {
       double v = (lane < nr) ? xs[r0 + lane] : 0.0;
       for (int j = 0; j < nr; ++j) {
         const double xj = __shfl_sync(0xffffffffu, v, j);
-        if (lane > j && lane < nr) v = fma(-(double)a[(long long)(r0 + lane) * n + r0 + j], xj, v);
+        if (lane > j && lane < nr) v = fma(-tile[lane][j], xj, v);
       }
       if (lane < nr) xs[r0 + lane] = v;
     }
@@ -406,23 +508,20 @@ __global__ void __launch_bounds__(256) lu_solve_kernel(int n, const T* __restric
   // backward: upper
   for (int r1 = n; r1 > 0; r1 -= 32) {
     const int r0 = max(0, r1 - 32), nr = r1 - r0;
-    for (int r = warp; r < nr; r += nw) {
-      double s = 0.0;
-      for (int c = r1 + lane; c < n; c += 32) s = fma((double)a[(long long)(r0 + r) * n + c], xs[c], s);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) xs[r0 + r] -= s;
-    }
+    load_tile(r0, nr);
+    off_diagonal(r0, nr, r1, n);
+    if (warp == 7) rcp[lane] = lane < nr ? 1.0 / widen(a[(long long)(r0 + lane) * n + r0 + lane]) : 1.0;
     __syncthreads();
     if (warp == 0) {
       double v = (lane < nr) ? xs[r0 + lane] : 0.0;
       for (int j = nr - 1; j >= 0; --j) {
-        double vj = __shfl_sync(0xffffffffu, v, j);
-        if (lane == j) {
-          v = v / (double)a[(long long)(r0 + j) * n + r0 + j];
-        }
-        vj = __shfl_sync(0xffffffffu, v, j);
-        if (lane < j) v = fma(-(double)a[(long long)(r0 + lane) * n + r0 + j], vj, v);
+        const double vj = __shfl_sync(0xffffffffu, v, j), d = tile[j][j], y = rcp[j];
+        const double q0 = vj * y;
+        const double q = fma(fma(-d, q0, vj), y, q0);
+        // zero, and what would leave the correction's range, is divided
+        const double xj = mid_range(q) && mid_range(vj) && mid_range(y) ? q : vj / d;
+        if (lane == j) v = xj;
+        if (lane < j) v = fma(-tile[lane][j], xj, v);
       }
       if (lane < nr) xs[r0 + lane] = v;
     }
@@ -435,7 +534,7 @@ void launch_lu_solve(int nv, int n, const double* LU, const int* piv, const doub
                      cudaStream_t s) {
   if (nv <= 0) return;
   ves_count_launch();
-  lu_solve_kernel<double><<<nv, 256, (size_t)n * sizeof(double), s>>>(n, LU, piv, b, x);
+  lu_solve_kernel<double><<<nv, 256, (size_t)n * (sizeof(double) + sizeof(int)), s>>>(n, LU, piv, b, x);
 }
 
 // the same solve with an FP32 factorisation (FP64 right-hand side, FP64 sums)
@@ -443,7 +542,7 @@ void launch_lu_solve_f32(int nv, int n, const float* LU, const int* piv, const d
                          cudaStream_t s) {
   if (nv <= 0) return;
   ves_count_launch();
-  lu_solve_kernel<float><<<nv, 256, (size_t)n * sizeof(double), s>>>(n, LU, piv, b, x);
+  lu_solve_kernel<float><<<nv, 256, (size_t)n * (sizeof(double) + sizeof(int)), s>>>(n, LU, piv, b, x);
 }
 
 // ----------------------------------------------------------------------------
