@@ -43,6 +43,7 @@
 //   unit length, is those 12 spacings, and its points are excluded).
 //   Sources without a contrast (visc == 1) have zero density and are skipped.
 #include "ves_internal.h"
+#include "ves_tc.cuh"
 
 namespace {
 
@@ -325,7 +326,7 @@ namespace {
 constexpr int kDLPMax = 24;          // highest expansion order
 constexpr float kDLRhoMax = 0.35f;   // expansion used for rho_pair <= this
 constexpr float kDLEps = 1e-10f;     // truncation bound relative to sum |c|, sum |e|
-constexpr int kDLStage = 16;         // source vesicles per shared-memory stage
+constexpr int kDLStage = 12;         // source vesicles per shared-memory stage (48 KB with eight warps)
 
 struct __align__(16) DLSrc {
   float2 chi, clo;  // centre, high and low FP32 parts
@@ -501,7 +502,7 @@ __global__ void __launch_bounds__(256) dl_mp_targets_kernel(int ntp, const doubl
 }
 
 struct DLMPArgs {
-  int nsrc, ns, ntp;
+  int nsrc, ns, nt, ntp;
   const float4* recA;  // [nsrc][ns] local x, y, normal x, y
   const float2* recB;  // [nsrc][ns] mean-free density
   const double* Xsrc;  // the FP64 sources (targets within 6 spacings)
@@ -519,6 +520,7 @@ struct DLMPArgs {
   const uint32_t* excl_mask;
   int maxc, nwords;
   double* out;
+  VesDeviceStatus* st;
 };
 
 // smallest P with rho^(P+1) ((P+2)(1-rho) + rho) / (1-rho)^2 <= eps (the
@@ -533,65 +535,123 @@ __device__ __forceinline__ int dl_order(float rp) {
   return kDLPMax;
 }
 
-// One CTA per target column (blockDim = ntp rounded up to a warp multiple, <= 128).
-// Dynamic shared memory: the direct-rule records of one source (ns float4 + ns float2).
-__global__ void __launch_bounds__(128) dl_mp_eval_kernel(DLMPArgs p) {
-  extern __shared__ __align__(16) float4 dA[];
-  float2* dB = reinterpret_cast<float2*>(dA + p.ns);
-  __shared__ DLSrc ssrc[kDLStage];
-  __shared__ DLMom smom[kDLStage][kDLPMax + 1];
-  __shared__ float rmax_w[4];
-  const int col = blockIdx.x, i = threadIdx.x;
-  const bool valid = i < p.ntp;
-  const float2 tl = valid ? p.tloc[(long long)col * p.ntp + i] : make_float2(0.f, 0.f);
+// A pair of target column and source as the warp's lanes read it: centre
+// offset and what to do (> 0: order of the expansion, 0: nothing, -1: direct
+// rule, -2 - place on the near list).
+struct __align__(16) DLPair {
+  float ox, oy;
+  int code, pad;
+};
+
+// A warp owns 32 points of one target column (one unit); the warps of a CTA
+// share the staged sources (all orders and one record each, by bulk copy, two
+// stages in flight).  One lane per source works out the pair's offset, order
+// and place on the near list.  S warps share a unit when there are few: they
+// take the sources of a stage in turn and leave the contributions in shared
+// memory, where the unit's first warp adds them in source order, so the sum
+// does not depend on S.  Latency-bound at small sizes: a close pair is a chain
+// of ns terms per point, and a column's warps ran all of a column's pairs one
+// after the other (301 x N = 64: 1.54 ms, now 1.15).
+template <int WARPS, int S>
+__global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eval_kernel(DLMPArgs p) {
+  constexpr int kUnits = WARPS / S;
+  __shared__ __align__(128) DLMom smom[2][kDLStage * (kDLPMax + 1)];
+  __shared__ __align__(16) DLSrc ssrc[2][kDLStage];
+  __shared__ DLPair pairs[WARPS][kDLStage];
+  __shared__ float4 dA[WARPS][32];
+  __shared__ float2 dB[WARPS][32];
+  __shared__ double2 part[S > 1 ? 2 : 1][S > 1 ? kUnits : 1][S > 1 ? kDLStage : 1][32];
+  __shared__ int turn[2][kUnits];
+  __shared__ uint64_t bar[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int unit = warp / S, sub = warp % S;
+  const int upc = (p.ntp + 31) / 32;
+  const long long u = (long long)blockIdx.x * kUnits + unit;
+  const bool live = u < (long long)p.nt * upc;
+  const int col = live ? (int)(u / upc) : 0;
+  const int i = (live ? (int)(u % upc) : 0) * 32 + lane;
+  const bool valid = live && i < p.ntp;
+  const float2* tl_col = p.tloc + (long long)col * p.ntp;
+  const float2 tl = valid ? tl_col[i] : make_float2(0.f, 0.f);
   const float2 thi = p.thi[col], tlo = p.tlo[col];
   const double txa = valid ? p.Xtar[(long long)col * 2 * p.ntp + i] : 0.0;
   const double tya = valid ? p.Xtar[(long long)col * 2 * p.ntp + p.ntp + i] : 0.0;
-  float rt = sqrtf(tl.x * tl.x + tl.y * tl.y);
-  for (int o = 16; o > 0; o >>= 1) rt = fmaxf(rt, __shfl_xor_sync(0xffffffffu, rt, o));
-  if ((i & 31) == 0) rmax_w[i >> 5] = rt;
-  __syncthreads();
   float RT = 0.f;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) RT = fmaxf(RT, rmax_w[w]);
+  for (int k = lane; k < p.ntp; k += 32) {
+    const float2 t = tl_col[k];
+    RT = fmaxf(RT, sqrtf(t.x * t.x + t.y * t.y));
+  }
+  for (int o = 16; o > 0; o >>= 1) RT = fmaxf(RT, __shfl_xor_sync(0xffffffffu, RT, o));
   RT *= 1.0f + 1e-6f;
+  if (threadIdx.x == 0) {
+    tc_mbar_init(&bar[0], 1);
+    tc_mbar_init(&bar[1], 1);
+    tc_mbar_fence_init();
+    tc_fence_async_smem();
+  }
+  if (threadIdx.x < 2 * kUnits) turn[threadIdx.x / kUnits][threadIdx.x % kUnits] = 0;
+  __syncthreads();
   const int self = p.self_idx ? p.self_idx[col] : -1;
   const int cend = p.cand_count ? min(p.cand_count[col], p.maxc) : 0;
   const int* cands = p.cand_src ? p.cand_src + (long long)col * p.maxc : nullptr;
-  int cur = 0;
+  const int nstages = (p.nsrc + kDLStage - 1) / kDLStage;
+  auto fetch = [&](int st) {  // thread 0
+    const int s0 = st * kDLStage, n = min(kDLStage, p.nsrc - s0), buf = st & 1;
+    tc_expect_tx(&bar[buf], (uint32_t)(n * ((kDLPMax + 1) * sizeof(DLMom) + sizeof(DLSrc))));
+    tc_bulk_g2s(smom[buf], p.mom + (long long)s0 * (kDLPMax + 1), (uint32_t)(n * (kDLPMax + 1) * sizeof(DLMom)),
+                &bar[buf]);
+    tc_bulk_g2s(ssrc[buf], p.src + s0, (uint32_t)(n * sizeof(DLSrc)), &bar[buf]);
+  };
+  if (threadIdx.x == 0)
+    for (int st = 0; st < 2 && st < nstages; ++st) fetch(st);
   double ax = 0.0, ay = 0.0;  // pi * u
-  for (int s0 = 0; s0 < p.nsrc; s0 += kDLStage) {
-    const int nst = min(kDLStage, p.nsrc - s0);
-    __syncthreads();
-    for (int q = i; q < nst; q += blockDim.x) ssrc[q] = p.src[s0 + q];
-    for (int q = i; q < nst * (kDLPMax + 1); q += blockDim.x)
-      (&smom[0][0])[q] = p.mom[(long long)s0 * (kDLPMax + 1) + q];
-    __syncthreads();
-    for (int q = 0; q < nst; ++q) {
-      const int s = s0 + q;
-      if (s == self) continue;
-      const DLSrc S = ssrc[q];
-      bool cand = false;
-      int cidx = 0;
-      if (cend > 0) {
-        while (cur < cend && cands[cur] < s) ++cur;
-        cand = cur < cend && cands[cur] == s;
-        cidx = cur;
+  for (int st = 0; st < nstages; ++st) {
+    const int buf = st & 1, s0 = st * kDLStage, n = min(kDLStage, p.nsrc - s0);
+    bool failed = !tc_mbar_wait(&bar[buf], (st >> 1) & 1, p.st, 31);
+    if (lane < n) {
+      const DLSrc Sq = ssrc[buf][lane];
+      const int s = s0 + lane;
+      int lo = 0, hi = cend;  // first candidate >= s
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cands[mid] < s) lo = mid + 1; else hi = mid;
       }
-      if (S.skip) continue;
-      const float ox = (thi.x - S.chi.x) + (tlo.x - S.clo.x);
-      const float oy = (thi.y - S.chi.y) + (tlo.y - S.clo.y);
+      const bool cand = lo < cend && cands[lo] == s;
+      const float ox = (thi.x - Sq.chi.x) + (tlo.x - Sq.clo.x);
+      const float oy = (thi.y - Sq.chi.y) + (tlo.y - Sq.clo.y);
       const float dc = sqrtf(ox * ox + oy * oy) - RT;
-      const float rp = dc > 0.f ? S.R / dc : 2.f;
-      if (!cand && rp <= kDLRhoMax) {
-        const int P = dl_order(rp);
-        const float wx = tl.x + ox, wy = tl.y + oy;  // omega
+      const float rp = dc > 0.f ? Sq.R / dc : 2.f;
+      int code;
+      if (s == self || Sq.skip)
+        code = 0;
+      else if (!cand && rp <= kDLRhoMax)
+        code = dl_order(rp);
+      else
+        code = cand ? -2 - lo : -1;
+      pairs[warp][lane] = DLPair{ox, oy, code, 0};
+    }
+    __syncwarp();
+    for (int qs = 0;; ++qs) {
+      if (S > 1) {  // the unit's warps take the stage's sources in turn
+        if (lane == 0) qs = atomicAdd(&turn[buf][unit], 1);
+        qs = __shfl_sync(0xffffffffu, qs, 0);
+      }
+      if (qs >= n || !live) break;
+      const DLPair pr = pairs[warp][qs];
+      const DLSrc& Sq = ssrc[buf][qs];
+      double vx = 0.0, vy = 0.0;
+      if (pr.code > 0) {
+        const int P = pr.code;
+        const DLMom* mq = smom[buf] + qs * (kDLPMax + 1);
+        const float wx = tl.x + pr.ox, wy = tl.y + pr.oy;  // omega
         const float om2 = fmaf(wx, wx, wy * wy);
         const float iom2 = 1.0f / om2;
         const float iwr = wx * iom2, iwi = -wy * iom2;       // 1 / omega
-        const float ur = S.R * iwr, ui = S.R * iwi;          // tau = R / omega
-        float2 h1 = smom[q][P].c, h2 = smom[q][P].e, h3 = smom[q][P].c1, h4 = smom[q][P].g1;
+        const float ur = Sq.R * iwr, ui = Sq.R * iwi;        // tau = R / omega
+        float2 h1 = mq[P].c, h2 = mq[P].e, h3 = mq[P].c1, h4 = mq[P].g1;
+#pragma unroll 2
         for (int k = P - 1; k >= 0; --k) {
-          const DLMom m = smom[q][k];
+          const DLMom m = mq[k];
           float2 n;
           n.x = fmaf(h1.x, ur, fmaf(-h1.y, ui, m.c.x));
           n.y = fmaf(h1.x, ui, fmaf(h1.y, ur, m.c.y));
@@ -615,33 +675,42 @@ __global__ void __launch_bounds__(128) dl_mp_eval_kernel(DLMPArgs p) {
         const float t3r = qr * h3.x + qi * h3.y, t3i = qi * h3.x - qr * h3.y;
         // t4 = R conj(h4 / omega^2)
         const float i2r = iwr * iwr - iwi * iwi, i2i = 2.f * iwr * iwi;   // 1/omega^2
-        const float t4r = S.R * (h4.x * i2r - h4.y * i2i), t4i = -S.R * (h4.x * i2i + h4.y * i2r);
-        if (valid) {
-          ax += 0.25 * (double)(t1r + t2r + t3r - t4r);
-          ay += 0.25 * (double)(t1i + t2i + t3i - t4i);
-        }
-      } else {
-        // direct rule over the upsampled points, FP32, coordinates relative to the source centre
-        __syncthreads();
+        const float t4r = Sq.R * (h4.x * i2r - h4.y * i2i), t4i = -Sq.R * (h4.x * i2i + h4.y * i2r);
+        vx = 0.25 * (double)(t1r + t2r + t3r - t4r);
+        vy = 0.25 * (double)(t1i + t2i + t3i - t4i);
+      } else if (pr.code < 0) {
+        // direct rule over the upsampled points, FP32, coordinates relative to
+        // the source centre; records staged 32 at a time
+        const int s = s0 + qs;
         const float4* A4 = p.recA + (long long)s * p.ns;
         const float2* B2 = p.recB + (long long)s * p.ns;
-        for (int j = i; j < p.ns; j += blockDim.x) {
-          dA[j] = A4[j];
-          dB[j] = B2[j];
-        }
-        __syncthreads();
         bool excl = !valid;
-        if (cand && valid) {
-          const uint32_t w = p.excl_mask[((long long)col * p.maxc + cidx) * p.nwords + (i >> 5)];
+        if (pr.code < -1 && valid) {
+          const uint32_t w = p.excl_mask[((long long)col * p.maxc + (-2 - pr.code)) * p.nwords + (i >> 5)];
           excl = (w >> (i & 31)) & 1u;
         }
-        if (!excl) {
-          const float tx = tl.x + ox, ty = tl.y + oy;
-          float bx = 0.f, by = 0.f, dmin = 3.0e38f;
+        const float tx = tl.x + pr.ox, ty = tl.y + pr.oy;
+        float bx = 0.f, by = 0.f, dmin = 3.0e38f;
+        float4 na = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 nb = make_float2(0.f, 0.f);
+        if (lane < p.ns) {
+          na = A4[lane];
+          nb = B2[lane];
+        }
+        for (int j0 = 0; j0 < p.ns; j0 += 32) {
+          __syncwarp();
+          dA[warp][lane] = na;
+          dB[warp][lane] = nb;
+          __syncwarp();
+          if (j0 + 32 + lane < p.ns) {
+            na = A4[j0 + 32 + lane];
+            nb = B2[j0 + 32 + lane];
+          }
+          const int nj = min(32, p.ns - j0);
 #pragma unroll 4
-          for (int j = 0; j < p.ns; ++j) {
-            const float4 a = dA[j];
-            const float2 b = dB[j];
+          for (int j = 0; j < nj; ++j) {
+            const float4 a = dA[warp][j];
+            const float2 b = dB[warp][j];
             const float dx = tx - a.x, dy = ty - a.y;
             const float d2 = fmaf(dx, dx, dy * dy);
             dmin = fminf(dmin, d2);
@@ -650,29 +719,55 @@ __global__ void __launch_bounds__(128) dl_mp_eval_kernel(DLMPArgs p) {
             bx = fmaf(c, dx, bx);
             by = fmaf(c, dy, by);
           }
-          if (dmin >= S.thr2) {
-            ax += (double)bx;
-            ay += (double)by;
+        }
+        if (!excl) {
+          if (dmin >= Sq.thr2) {
+            vx = (double)bx;
+            vy = (double)by;
           } else {  // within 12 spacings: the full density in FP64
             const double* xs = p.Xsrc + (long long)s * 2 * p.ns;
             const double* ts = p.tang + (long long)s * 2 * p.ns;
             const double* ds = p.den + (long long)s * 2 * p.ns;
-            double cx = 0.0, cy = 0.0;
             for (int j = 0; j < p.ns; ++j) {
               const double dx = txa - xs[j], dy = tya - xs[p.ns + j];
               const double d2 = dx * dx + dy * dy;
               const double c = ((dx * ts[p.ns + j] - dy * ts[j]) / (d2 * d2)) * (dx * ds[j] + dy * ds[p.ns + j]);
-              cx = fma(c, dx, cx);
-              cy = fma(c, dy, cy);
+              vx = fma(c, dx, vx);
+              vy = fma(c, dy, vy);
             }
-            ax += cx;
-            ay += cy;
           }
         }
       }
+      if (S > 1) {
+        part[buf][unit][qs][lane] = make_double2(vx, vy);
+      } else {  // points past the column's end add too; they are not stored
+        ax += vx;
+        ay += vy;
+      }
+    }
+    // nobody reads this stage any more (and every contribution is in)
+    failed = __syncthreads_or(failed ? 1 : 0) != 0;
+    if (S > 1) {
+      if (threadIdx.x < kUnits) turn[buf][threadIdx.x] = 0;
+      if (sub == 0)
+        for (int qs = 0; qs < n; ++qs) {
+          ax += part[buf][unit][qs][lane].x;
+          ay += part[buf][unit][qs][lane].y;
+        }
+    }
+    if (failed) {  // the copies in flight land before the CTA ends
+      if (threadIdx.x == 0) {
+        tc_mbar_wait(&bar[buf], (st >> 1) & 1, nullptr, 0);
+        if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((st + 1) >> 1) & 1, nullptr, 0);
+      }
+      break;
+    }
+    if (threadIdx.x == 0 && st + 2 < nstages) {
+      tc_fence_async_smem();
+      fetch(st + 2);
     }
   }
-  if (valid) {
+  if (valid && sub == 0) {
     p.out[(long long)col * 2 * p.ntp + i] = ax / VES_PI;
     p.out[(long long)col * 2 * p.ntp + p.ntp + i] = ay / VES_PI;
   }
@@ -715,17 +810,13 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
     ves_record_error(VES_ERR_SHAPE, "farfield_dl: %d source points per vesicle exceed the multipole path", ns);
     return VES_ERR_SHAPE;
   }
-  if (dsmem > 32 * 1024) {  // with the ~13 KB of static shared memory, past the 48 KB default
-    const int rc = ves_cuda_status(
-        cudaFuncSetAttribute(dl_mp_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem), "dl smem");
-    if (rc) return rc;
-  }
   ves_count_launch(3);
   dl_mp_prep_kernel<<<nsrc, 256, 0, s>>>(ns, Xsrc, tang, den, sa, visc, src, mom, recA, recB);
   dl_mp_targets_kernel<<<nt, 256, 0, s>>>(ntp, Xtar, tloc, thi, tlo);
   DLMPArgs a;
   a.nsrc = nsrc;
   a.ns = ns;
+  a.nt = nt;
   a.ntp = ntp;
   a.recA = recA;
   a.recB = recB;
@@ -745,7 +836,16 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
   a.maxc = nl ? nl->maxc : 0;
   a.nwords = (ntp + 31) / 32;
   a.out = out;
-  dl_mp_eval_kernel<<<nt, ((ntp + 31) / 32) * 32, dsmem, s>>>(a);
+  a.st = c ? c->status : nullptr;
+  // one warp per 32 points from nine such units per SM on, four from two per
+  // SM, eight below (the single layer's rule, the same pattern of work)
+  const long long units = (long long)nt * ((ntp + 31) / 32);
+  if (units >= 152 * 9)
+    dl_mp_eval_kernel<4, 1><<<(unsigned)((units + 3) / 4), 128, 0, s>>>(a);
+  else if (units >= 152 * 2)
+    dl_mp_eval_kernel<4, 4><<<(unsigned)units, 128, 0, s>>>(a);
+  else
+    dl_mp_eval_kernel<8, 8><<<(unsigned)units, 256, 0, s>>>(a);
   return ves_launch_check("farfield_dl multipole");
 }
 
