@@ -24,20 +24,31 @@
 //
 // Three kernels per block: "down" (conv pair 1, conv pair 2), "up1"
 // (transposed conv 1) and "up2" (transposed conv 2, mix, residual and
-// pass-through).  up1 works on tiles of V1 = 128 / (L/4) vesicles of one
-// group whose rows are interleaved (row q*V1 + j holds position q of the
-// tile's vesicle j), so that its MMAs use all 128 rows: a shift of the input
-// by u positions is a shift by u*V1 rows, and every row still only meets
-// rows of its own vesicle.  down writes the intermediate in that layout.
-// down itself works on tiles of vd = 2 vesicles at L = 128 (conv pair 1
-// then fills 128 rows, conv pair 2 64), one vesicle at L = 256.  The block input and output stay FP32 in global memory
-// ([nv][groups*channels][L]); the intermediates between the kernels are BF16
-// in the K-major layout.  Kernels are persistent: each CTA walks a contiguous
-// range of (group, vesicle) items, loading a group's weight image into shared
-// memory once per group it meets, and runs several warp groups, each on its
-// own items (3, 4 and 3 when TMEM and shared memory allow): while one waits
-// for its MMAs the others run their epilogues.  Splitting the transposed
-// convs over two kernels keeps each weight image small enough for that.
+// pass-through).  All work on tiles of V vesicles of one group whose rows are
+// interleaved (row q*V + j holds position q of the tile's vesicle j), so that
+// the MMAs use all 128 rows: a shift of the input by u positions is a shift
+// by u*V rows, and every row still only meets rows of its own vesicle.  down:
+// two vesicles at L = 128 (conv pair 1 fills 128 rows, conv pair 2 64), one at
+// L = 256; up1: 128 / (L/4); up2: two at L = 128, one at L = 256.  down and
+// up1 write the intermediate in the next kernel's layout.  The block input and
+// output stay FP32 in global memory ([nv][groups*channels][L]); the
+// intermediates between the kernels are BF16 in the K-major layout.  Kernels
+// are persistent: each CTA walks a contiguous range of (group, tile) items,
+// loading a group's weight image into shared memory once per group it meets,
+// and runs two or three warp groups of eight warps (as TMEM and shared memory
+// allow), each on its own items: while one waits for its MMAs the others run
+// their epilogues.
+//
+// What bounds them, from clock stamps in a copy: the tensor core's reads of its
+// operands from shared memory (an M = 128, N = 128, K = 16 MMA reads 8 KB in
+// its 64 cycles, the whole shared-memory rate) next to the epilogues' own
+// reads and writes there.  With every epilogue access left out of the copy
+// the kernels still took 75-95% of their time.  One network pass, 1024
+// vesicles, before (one warp per lane quarter, one vesicle per up2 item, its
+// block input staged in shared memory, MMAs issued from per-thread values) and
+// now, ms: advection 56.1 -> 49.3, near field 48.7 -> 34.9, advection-tension
+// 42.5 -> 31.8.  The near field's kernels: down 1.20 -> 0.92, up1 0.45 -> 0.33,
+// up2 1.83 -> 1.23; the advection's 1.67 -> 1.41, 0.62 -> 0.51, 2.05 -> 1.86.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -52,7 +63,7 @@
 
 namespace tcnet {
 
-constexpr int kGroupThreads = 128;
+constexpr int kGroupThreads = 256;  // eight warps: two on each TMEM lane quarter
 constexpr int kMinSmem = 117 * 1024;
 constexpr int kOffsets = 11;  // input shifts of a conv pair: -6..6 without +-5
 __host__ __device__ constexpr int shift_of(int oi) { return oi < 2 ? -6 + 2 * oi : (oi < 9 ? oi - 5 : 2 * oi - 14); }
@@ -80,13 +91,13 @@ struct Geo {
   // up2 image (transposed conv 2 and mix): W (u2merge = 1: [5][kcd][2*kcd*8][16B],
   // both output parities in one operand of N = 2*kcd*8 rows, parity r at row
   // r*kcd*8; u2merge = 0: as up1), M [3][kcd][cmix][16B], consts [7][128] f32;
-  // arrays of warp group 0: cs [kcd][L/2+4][16B], ds [kcd][L+2][16B] (at least
-  // cin*L*4 bytes: it first receives the block input)
+  // arrays of warp group 0: cs [kcd][(L/2+4)*vu][16B], ds [kcd][(L+2)*vu][16B]
   int u2merge, u2w, u2wm, u2cst, u2size, u2cs, u2ds, u2grp;
   // down -> up1 per tile of v1 vesicles: [kcd][L/4][v1][16B] (mid_bytes per
-  // vesicle); up1 -> up2 per (vesicle, group) item: [kcd][L/2][16B]
+  // vesicle); up1 -> up2 per tile of vu vesicles: [kcd][L/2][vu][16B]
   int mid_bytes, mid2_bytes, mid_stride;
   int v1;  // vesicles per up1 tile (v1 * L/4 = 128 rows)
+  int vu;  // vesicles per up2 tile (2 at L = 128 when two tiles fit on an SM)
   int vd;  // vesicles per down tile (2 at L = 128: the block input is read
            // from global memory (L2-prefetched) with no FP32 staging copy)
 };
@@ -159,20 +170,22 @@ inline Geo make_geo(const ves_net_block& b, int L) {
   g.u1bs = g.u1size;
   g.v1 = 128 / (L / 4);
   g.u1grp = g.kcd * (L / 4 + 4) * g.v1 * 16;
-  // up2: merged image (both parities in one operand of N = 2*Nd rows) when it
-  // still leaves room for three warp groups
-  g.u2grp = g.kcd * (L / 2 + 4) * 16 + std::max(g.kcd * (L + 2) * 16, rup(g.cin * L * 4, 16));
-  for (g.u2merge = 1; g.u2merge >= 0; --g.u2merge) {
-    const int dbytes = g.u2merge ? 5 * g.kcd * 2 * g.kcd * 8 * 16 : dec_unmerged;
+  // up2: tiles of two vesicles at L = 128 (128 rows) when two warp groups of
+  // them fit in shared memory and TMEM; merged image (both parities in one
+  // operand of N = 2*Nd rows) when two groups fit next to it
+  auto lay_up2 = [&](int vu, int merge) {
+    g.vu = vu;
+    g.u2merge = merge;
     g.u2w = 0;
-    g.u2wm = dbytes;
+    g.u2wm = merge ? 5 * g.kcd * 2 * g.kcd * 8 * 16 : dec_unmerged;
     g.u2cst = g.u2wm + 3 * g.kcd * g.cmix * 16;
     g.u2size = g.u2cst + 7 * 128 * 4;
-    if (g.u2size + 3 * g.u2grp + kTail <= kMaxSmem) break;
-  }
-  if (g.u2merge < 0) g.u2merge = 0;
+    g.u2grp = g.kcd * (L / 2 + 4 + L + 2) * vu * 16;
+    return g.u2size + 2 * g.u2grp + kTail <= kMaxSmem;
+  };
+  if (!(L == 128 && 2 * (2 * g.kcd * 8 + 64) <= 512 && lay_up2(2, 1)) && !lay_up2(1, 1)) lay_up2(1, 0);
   g.u2cs = g.u2size;
-  g.u2ds = g.u2cs + g.kcd * (L / 2 + 4) * 16;
+  g.u2ds = g.u2cs + g.kcd * (L / 2 + 4) * g.vu * 16;
   g.mid_bytes = g.kcd * (L / 4) * 16;
   g.mid2_bytes = g.kcd * (L / 2) * 16;
   g.mid_stride = g.mid_bytes + g.mid2_bytes;
@@ -182,14 +195,13 @@ inline Geo make_geo(const ves_net_block& b, int L) {
 struct KArgs {
   Geo g;
   int G, nv;
-  int m64;                   // layers of at most 64 positions use M = 64 MMAs
   long long items;
   const unsigned char* img;  // group 0 image of this block; group stride = image size
   const float* x;            // block input [nv][G*cin][L]
   float* out;                // block output [nv][G*cout][L]
   unsigned char* mid;        // down -> up1: [ntiles][G][v1 * mid_bytes]
-  unsigned char* mid2;       // up1 -> up2: [nv][G][mid2_bytes]
-  int per_grp;               // items per channel group (nv, or up1 tiles)
+  unsigned char* mid2;       // up1 -> up2: [tiles of vu][G][vu * mid2_bytes]
+  int per_grp;               // items per channel group (tiles of the kernel's vesicles)
   VesDeviceStatus* st;
 };
 
@@ -204,7 +216,7 @@ __device__ __forceinline__ void zero16(unsigned char* dst, int bytes) {
   for (int i = threadIdx.x; i < bytes / 16; i += blockDim.x) d[i] = z;
 }
 
-// barrier of one warp group (named barrier 1 + group, 128 threads)
+// barrier of one warp group (named barrier 1 + group)
 __device__ __forceinline__ void group_sync(int wg) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + wg), "r"(kGroupThreads) : "memory");
 }
@@ -226,7 +238,25 @@ __device__ __forceinline__ bool group_wait_one(uint64_t* bar, unsigned phase, Ve
   return *(volatile int*)flag == 0;
 }
 
-// MMA issue sequences.  The issuing lane runs them as straight-line code:
+// The tensor core takes MMAs in the order they are issued.  Groups that issue
+// at the same time share its rate, finish together and then all run their
+// epilogues while it idles; a group that issues its whole batch before the
+// next one starts leaves the others' epilogues to overlap with it.  The
+// issuing threads therefore take turns through a flag in shared memory.  It
+// orders issue only: one that waits too long issues anyway.
+__device__ __forceinline__ void batch_begin(int* flag) {
+  for (int it = 0; it < (1 << 14); ++it)
+    if (*(volatile int*)flag == 0 && atomicCAS(flag, 0, 1) == 0) return;
+}
+__device__ __forceinline__ void batch_end(int* flag) { atomicExch(flag, 0); }
+
+// MMA issue sequences.  One elected thread of a group's first warp issues;
+// the operands are computed from values that are the same across the warp
+// (the group's index and the TMEM base by a shuffle, everything else from
+// kernel arguments), which lets descriptors stay in uniform registers: from
+// per-thread values an issue took 65-75 cycles whatever the shape, like this
+// 37-51 where the tensor core takes 32-44.  The issuing lane runs the
+// sequences as straight-line code:
 // each is a template on the number of 16-channel K steps (NK), picked by one
 // switch, so that no loop branch sits between two tcgen05.mma (a branching
 // loop in the single issuing lane costs more than the tensor core's time per
@@ -259,14 +289,14 @@ __device__ __forceinline__ void issue_deconv(uint32_t d, uint64_t a0, uint64_t b
     for (int j = 0; j < NK; ++j) tc_mma_bf16(d, ad + j * stepA, bd + j * stepB, idesc, (u | j) ? 1u : 0u);
   }
 }
-// mix of one 128-position half: 3 taps t (A rows t) x NK K steps, onto the
+// mix of 128 rows: 3 taps t (A rows t * tapRows) x NK K steps, onto the
 // preset accumulator
 template <int NK>
 __device__ __forceinline__ void issue_mix(uint32_t d, uint64_t a0, uint64_t b0, uint32_t bTap, uint32_t stepA,
-                                          uint32_t stepB, uint32_t idesc) {
+                                          uint32_t stepB, uint32_t idesc, uint32_t tapRows) {
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
-    const uint64_t ad = a0 + (uint32_t)t, bd = b0 + (uint32_t)t * bTap;
+    const uint64_t ad = a0 + (uint32_t)t * tapRows, bd = b0 + (uint32_t)t * bTap;
 #pragma unroll
     for (int j = 0; j < NK; ++j) tc_mma_bf16(d, ad + j * stepA, bd + j * stepB, idesc, 1u);
   }
@@ -333,26 +363,6 @@ __device__ __forceinline__ uint4 act8(const float* v, const float* cst, int kc, 
   return make_uint4(pack_bf2(y[0], y[1]), pack_bf2(y[2], y[3]), pack_bf2(y[4], y[5]), pack_bf2(y[6], y[7]));
 }
 
-// Rows of an accumulator of M rows in TMEM: M = 128 puts row r on lane r;
-// M = 64 (half the A tile per MMA, for layers of at most 64 positions) puts
-// rows 16 q .. 16 q + 15 on lanes 32 q .. 32 q + 15 (measured on a GB300).
-// The row this thread's lane holds, or -1.
-__device__ __forceinline__ int acc_row(int M, int qd, int lane) {
-  return M == 128 ? 32 * qd + lane : (lane < 16 ? 16 * qd + lane : -1);
-}
-// first row held by warp quarter qd (uniform across the warp)
-__device__ __forceinline__ int acc_row0(int M, int qd) { return M == 128 ? 32 * qd : 16 * qd; }
-
-// accumulators of at most 64 rows use M = 64 MMAs (VES_TC_M64=0 turns this off; read once)
-inline bool tcnet_m64() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("VES_TC_M64");
-    v = (e && atoi(e) == 0) ? 0 : 1;
-  }
-  return v != 0;
-}
-
 // ---------------------------------------------------------------------------
 // Segments: the CTA's contiguous item range split where the channel group
 // changes; the weight image is reloaded (whole CTA) at each segment start and
@@ -367,12 +377,13 @@ __device__ __forceinline__ Seg next_seg(long long lo, long long hi, int nv) {
   return {lo, end < hi ? end : hi, grp};
 }
 
-// KC1 / KCD: compile-time K chunk counts of the two conv pairs' outputs (0:
-// read them from the geometry); fixed counts let every epilogue and issue
-// loop unroll.  NG: warp groups per CTA, each running its own items (2: 256
-// TMEM columns each; 3 or 4: 128 columns each, when N1 + N2 <= 128 and the
-// groups' arrays fit in shared memory).
-template <int KC1, int KCD, int NG>
+// down: conv pairs 1 and 2 on tiles of VD vesicles with interleaved rows (128
+// rows of conv pair 1, 64 of conv pair 2).  KC1 / KCD: compile-time K chunk
+// counts of the two conv pairs' outputs (0: read them from the geometry), so
+// that every epilogue and issue loop unrolls.  NG warp groups of eight warps,
+// each running its own tiles (2: 256 TMEM columns each; 3: 128, when N1 + N2
+// <= 128 and the groups' arrays fit in shared memory).
+template <int KC1, int KCD, int NG, int VD>
 __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bar[NG], xbar[NG];  // per warp group: MMA completion, input arrival
@@ -381,11 +392,10 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   const Geo& g = a.g;
   const int kc1 = KC1 ? KC1 : g.kc1, kcd = KCD ? KCD : g.kcd;
   const int L = g.L, L2 = L / 2, L4 = L / 4;
-  const int VD = g.vd;          // vesicles per item (tile), rows interleaved
   const int ntl = a.per_grp;    // tiles per channel group
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wg = tid / kGroupThreads, gt = tid % kGroupThreads;  // warp group, thread within it
-  const int qd = warp & 3;                                       // TMEM lane quarter = position block
+  const int wg = tid / kGroupThreads, gt = tid % kGroupThreads;    // warp group, thread within it
+  const int qd = warp & 3, hw = gt >> 7;   // TMEM lane quarter; which of the two warps on it
   const Range rg = my_items(a.items);
   if (rg.lo >= rg.hi) return;
   const uint32_t ncols = 512;  // all of TMEM (one CTA per SM)
@@ -404,10 +414,13 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   __syncthreads();
   tc_fence_after_sync();
   const int N1 = kc1 * 8, N2 = kcd * 8;
-  const uint32_t tcol = tbase + (NG == 2 ? 256 : 128) * wg;
+  const int wgu = __shfl_sync(0xffffffffu, wg, 0);  // uniform across the warp
+  const bool issuer = __shfl_sync(0xffffffffu, gt >> 5, 0) == 0 && tc_elect();
+  const uint32_t tcol = __shfl_sync(0xffffffffu, tbase, 0) + (NG == 2 ? 256 : 128) * wgu;
   const uint32_t d1 = tcol, d2 = tcol + N1;
+  const uint32_t lanes = (uint32_t)(32 * qd) << 16;
   const uint32_t sbase = tc_smem_u32(sm);
-  const int goff = wg * g.dgrp;
+  const int goff = wgu * g.dgrp;
   const float* cst = reinterpret_cast<const float*>(sm + g.dcst);
   const int P1 = (L2 + 6) * VD, P2 = (L4 + 6) * VD;  // rows per K chunk (circular halos of 3 positions)
   uint4* xs = reinterpret_cast<uint4*>(sm + g.dxs + goff);
@@ -416,16 +429,14 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   const uint32_t xbytes = (uint32_t)(g.cin * L * 4);
   unsigned phase = 0, xphase = 0;
   bool xpend = false;  // a bulk copy into xf is in flight
-  // block input x[v][grp*cin + c][pos] (cin*L contiguous floats) of the
-  // item's vesicles: one vesicle -> xf by bulk copy; a tile of two -> L2
+  // block input x[v][grp*cin + c][pos] (cin*L contiguous floats) of a tile's
+  // vesicles: one vesicle -> xf by bulk copy; a tile of two -> L2
   // (read by convert_x straight from global memory)
-  auto fetch_x = [&](long long item) {
-    const int grp = (int)(item / ntl);
-    const long long t = item % ntl;
+  auto fetch_x = [&](int grp, long long t) {
     if (VD == 1) {
       if (gt == 0) {
         tc_expect_tx(&xbar[wg], xbytes);
-        tc_bulk_g2s(xf, a.x + ((long long)t * a.G + grp) * (long long)g.cin * L, xbytes, &xbar[wg]);
+        tc_bulk_g2s(xf, a.x + (t * a.G + grp) * (long long)g.cin * L, xbytes, &xbar[wg]);
       }
       xpend = true;
     } else if (gt < VD && t * VD + gt < a.nv) {
@@ -437,6 +448,7 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   // (8-channel chunk, vesicle, position pair 2m, 2m+1)
   auto convert_x = [&](long long t, int grp) {
     const int lg2 = g.lgL - 1;
+#pragma unroll 2
     for (int i = gt; i < g.kcin * VD * L2; i += kGroupThreads) {
       const int m = i & (L2 - 1), kj = i >> lg2, kc = kj / VD, j = kj - kc * VD;
       const long long v = t * VD + j;
@@ -474,13 +486,14 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
   bool failed = false, stuck = false;  // stuck: this warp group's own MMA wait timed out
   for (long long lo = rg.lo; lo < rg.hi && !failed;) {
     const Seg sg = next_seg(lo, rg.hi, ntl);
+    const long long t0 = (long long)sg.grp * ntl;  // first item of the group
     __syncthreads();
     copy16(sm, a.img + (size_t)sg.grp * g.dsize, g.dsize);  // whole CTA
-    tc_fence_async_smem();  // weights (and the zeroed padding) -> tensor core, for both groups
+    tc_fence_async_smem();  // weights (and the zeroed padding) -> tensor core, for every group
     __syncthreads();
-    if (sg.lo + wg < sg.hi) fetch_x(sg.lo + wg);
+    if (sg.lo + wg < sg.hi) fetch_x(sg.grp, sg.lo + wg - t0);
     for (long long it = sg.lo + wg; it < sg.hi; it += NG) {
-      const long long t = it % ntl;
+      const long long t = it - t0;
       if (VD == 1) {
         if (!group_wait_one(&xbar[wg], xphase, a.st, 20, wg, gt, &fail[wg])) {
           failed = true;
@@ -491,18 +504,17 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
       }
       convert_x(t, sg.grp);
       group_sync_for_mma(wg);  // xs complete; xf fully read
-      if (it + NG < sg.hi) fetch_x(it + NG);
       // conv pair 1: D1[r][o], rows r = p*VD + j (p < L/2) on the lanes, o < n1 in the columns
-      const int M1 = (a.m64 && L2 * VD <= 64) ? 64 : 128, M2 = (a.m64 && L4 * VD <= 64) ? 64 : 128;
-      if (gt == 0) {
-        const uint32_t idesc = tc_idesc_bf16(M1, N1);
+      if (issuer) {
+        const uint32_t idesc = tc_idesc_bf16(128, N1);
         const uint32_t lboA = P1 * 16, lboB = g.n1 * 16;
         const uint64_t a0 = tc_desc(sbase + g.dxs + goff, lboA, 128), b0 = tc_desc(sbase + g.dw1, lboB, 128);
 #define VES_CONV1(NK) issue_conv<NK>(d1, a0, b0, (g.kcin * lboA) >> 4, (g.kcin * lboB) >> 4, (2 * lboA) >> 4, (2 * lboB) >> 4, idesc, (uint32_t)VD)
         VES_TC_NK_SWITCH(g.kcin / 2, VES_CONV1)
 #undef VES_CONV1
-        tc_commit(&bar[wg]);
+        tc_commit(&bar[wgu]);
       }
+      if (it + NG < sg.hi) fetch_x(sg.grp, t + NG);
       if (!group_wait_one(&bar[wg], phase, a.st, 21, wg, gt, &fail[wg])) {
         failed = stuck = true;
         break;
@@ -511,39 +523,22 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
       tc_fence_after_sync();
       // the epilogue's row r holds position p = r / VD of the tile's vesicle j = r % VD;
       // conv pair 2 reads position q of parity par at row (q + 3)*VD + j
-      if (KC1 != 0 && M1 == 64) {
-        // M = 64: threads 0-15 and 16-31 of a warp take the two halves of the
-        // channel chunks of the same 16 rows (16x32bx2 loads)
-        const int r = 16 * qd + (lane & 15), p = r / VD, j = r - p * VD, par = p & 1, q = p >> 1;
-        const int kb = (lane >> 4) * (KC1 / 2);
-        float vv[32];
-        tc_ld16x2_32<4 * KC1>(d1 + ((uint32_t)(32 * qd) << 16), vv);
-        if (p < L2) {
+      if (32 * qd < L2 * VD) {  // uniform per warp: the TMEM loads are warp-wide
+        const int r = 32 * qd + lane, p = r / VD, j = r % VD, par = p & 1, q = p >> 1;
+        const bool own = p < L2;
+        const int k1 = hw ? kc1 : kc1 / 2;
 #pragma unroll
-          for (int k = 0; k < KC1 / 2; ++k) {
-            const int kc = kb + k;
-            const uint4 val = act8(vv + 8 * k, cst, kc, g.n1, 0, 128, 256);
-            uint4* base = as + (size_t)(par * kc1 + kc) * P2 + j;
-            base[(q + 3) * VD] = val;
-            if (q >= L4 - 3) base[(q + 3 - L4) * VD] = val;
-            if (q < 3) base[(q + 3 + L4) * VD] = val;
-          }
-        }
-      } else if (acc_row0(M1, qd) < L2 * VD) {  // uniform per warp: the TMEM loads are warp-wide
-        const int r = acc_row(M1, qd, lane), p = r / VD, j = r - p * VD;
-        const bool own = r >= 0 && p < L2;
-        const int par = p & 1, q = p >> 1;
-#pragma unroll
-        for (int k0 = 0; k0 < kc1; k0 += 4) {
+        for (int kk = 0; kk < (KC1 ? KC1 / 2 : 8); kk += 4) {
+          const int k0 = hw * (kc1 / 2) + kk;
+          if (k0 >= k1) break;
           float vv[32];
-          tc_ld32(d1 + ((uint32_t)(32 * qd) << 16) + 8 * k0, vv);
+          tc_ld32(d1 + lanes + 8 * k0, vv);
           if (own) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              const int kc = k0 + k;
-              if (kc >= kc1) break;
-              const uint4 val = act8(vv + 8 * k, cst, kc, g.n1, 0, 128, 256);
-              uint4* base = as + (size_t)(par * kc1 + kc) * P2 + j;
+              if ((KC1 != 0 && kk + k >= KC1 / 2) || k0 + k >= k1) break;
+              const uint4 val = act8(vv + 8 * k, cst, k0 + k, g.n1, 0, 128, 256);
+              uint4* base = as + (size_t)(par * kc1 + k0 + k) * P2 + j;
               base[(q + 3) * VD] = val;
               if (q >= L4 - 3) base[(q + 3 - L4) * VD] = val;
               if (q < 3) base[(q + 3 + L4) * VD] = val;
@@ -552,15 +547,17 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
         }
       }
       group_sync_for_mma(wg);
-      // conv pair 2: D2[p][o], p < L/4, o < d
-      if (gt == 0) {
+      // conv pair 2: D2[r][o], rows r = p*VD + j (p < L/4, 64 rows), o < d; M = 64
+      // halves the operand read per MMA
+      constexpr int M2 = KCD ? 64 : 128;
+      if (issuer) {
         const uint32_t idesc = tc_idesc_bf16(M2, N2);
         const uint32_t lboA = P2 * 16, lboB = g.d * 16;
         const uint64_t a0 = tc_desc(sbase + g.das + goff, lboA, 128), b0 = tc_desc(sbase + g.dw2, lboB, 128);
 #define VES_CONV2(NK) issue_conv<NK>(d2, a0, b0, (kc1 * lboA) >> 4, (kc1 * lboB) >> 4, (2 * lboA) >> 4, (2 * lboB) >> 4, idesc, (uint32_t)VD)
         VES_TC_NK_SWITCH(kc1 / 2, VES_CONV2)
 #undef VES_CONV2
-        tc_commit(&bar[wg]);
+        tc_commit(&bar[wgu]);
       }
       if (!group_wait_one(&bar[wg], phase, a.st, 22, wg, gt, &fail[wg])) {
         failed = stuck = true;
@@ -570,39 +567,42 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
       tc_fence_after_sync();
       // the intermediate goes straight to global memory: row (kc, p) of
       // vesicle v = t*VD + j sits in its up1 tile (v / v1) at ((kc * L/4 + p) * v1 + v % v1)
-      if (KCD != 0 && M2 == 64) {
-        // M = 64, the two halves of the chunks on the two half-warps, as above
-        if (16 * qd < L4 * VD) {  // uniform per warp
-          const int r = 16 * qd + (lane & 15), p = r / VD, j = r - p * VD;
-          const long long v = t * VD + j;
-          const int V1 = g.v1, kb = (lane >> 4) * (KCD / 2);
-          const long long vs = v < a.nv ? v : 0;
-          uint4* gmid = reinterpret_cast<uint4*>(a.mid + ((size_t)(vs / V1) * a.G + sg.grp) * (size_t)V1 * g.mid_bytes) +
-                        (vs % V1);
-          float vv[32];
-          tc_ld16x2_32<4 * KCD>(d2 + ((uint32_t)(32 * qd) << 16), vv);
-          if (p < L4 && v < a.nv) {
-#pragma unroll
-            for (int k = 0; k < KCD / 2; ++k)
-              gmid[((size_t)(kb + k) * L4 + p) * V1] = act8(vv + 8 * k, cst, kb + k, g.d, 384, 512, 640);
-          }
-        }
-      } else if (acc_row0(M2, qd) < L4 * VD) {
-        const int r = acc_row(M2, qd, lane), p = r / VD, j = r - p * VD;
+      const int V1 = g.v1;
+      if (KCD != 0) {
+        // rows 16 qd .. + 15 of this quarter; the half-warps take the two
+        // halves of the channel chunks (16x32bx2 loads), the two warps parts of each half
+        const int r = 16 * qd + (lane & 15), p = r / VD, j = r % VD;
         const long long v = t * VD + j;
-        const bool own = r >= 0 && p < L4 && v < a.nv;
-        const int V1 = g.v1;
+        const int kb = (lane >> 4) * (KCD / 2);
+        const long long vs = v < a.nv ? v : 0;
+        uint4* gmid = reinterpret_cast<uint4*>(a.mid + ((size_t)(vs / V1) * a.G + sg.grp) * (size_t)V1 * g.mid_bytes) +
+                      (vs % V1);
+        float vv[32];
+        tc_ld16x2_32<4 * KCD>(d2 + lanes, vv);
+        if (p < L4 && v < a.nv) {
+#pragma unroll
+          for (int k = 0; k < KCD / 2; ++k)
+            if ((k < (KCD / 2 + 1) / 2) == (hw == 0))
+              gmid[((size_t)(kb + k) * L4 + p) * V1] = act8(vv + 8 * k, cst, kb + k, g.d, 384, 512, 640);
+        }
+      } else if (32 * qd < L4 * VD) {
+        const int r = 32 * qd + lane, p = r / VD, j = r % VD;
+        const long long v = t * VD + j;
+        const bool own = p < L4 && v < a.nv;
         const long long vs = own ? v : 0;
         uint4* gmid = reinterpret_cast<uint4*>(a.mid + ((size_t)(vs / V1) * a.G + sg.grp) * (size_t)V1 * g.mid_bytes) +
                       (vs % V1);
+        const int k1 = hw ? kcd : kcd / 2;
 #pragma unroll
-        for (int k0 = 0; k0 < kcd; k0 += 4) {
+        for (int kk = 0; kk < 8; kk += 4) {
+          const int k0 = hw * (kcd / 2) + kk;
+          if (k0 >= k1) break;
           float vv[32];
-          tc_ld32(d2 + ((uint32_t)(32 * qd) << 16) + 8 * k0, vv);
+          tc_ld32(d2 + lanes + 8 * k0, vv);
           if (own) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              if (k0 + k < kcd)
+              if (k0 + k < k1)
                 gmid[((size_t)(k0 + k) * L4 + p) * V1] = act8(vv + 8 * k, cst, k0 + k, g.d, 384, 512, 640);
           }
         }
@@ -624,99 +624,37 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
 // ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // The transposed convolutions, split in two kernels so that their weight
-// images and per-group arrays are small enough for more warp groups per SM:
+// images and per-group arrays are small enough for several warp groups per SM:
 //   up1: transposed conv 1 (intermediate [kcd][L/4] -> [kcd][L/2], BF16 rows
 //        to global memory);
 //   up2: transposed conv 2, mix, residual and pass-through channels.
-// Both M-split a transposed conv when its two output parities fit in 128
-// lanes (2*npos <= 128): parity r's operand starts r*npos rows early, so its
-// valid rows land on lanes [r*npos, (r+1)*npos) and every warp has epilogue
-// work; otherwise both parities share one MMA of N = 2*Nd (merged image) or
-// run as two MMAs on the same lanes.  Parity r accumulates in TMEM columns
-// [r*Nd, (r+1)*Nd) either way.
+// Both output parities share one MMA of N = 2*Nd (merged image) or run as two
+// MMAs on the same lanes; parity r accumulates in TMEM columns [r*Nd, (r+1)*Nd)
+// either way.
 
 // Issue one transposed conv (thread 0 of the group).  w0/w1: byte offsets of
 // parity 0/1 weights (tap 0, chunk 0, row 0), bTap: tap stride (16-byte
 // units), lboB: K-chunk stride of B in bytes, merged: both parities in one
-// operand of N = 2*Nd rows at w0.
+// operand of N = 2*Nd rows at w0; tapRows: vesicles per tile, rows interleaved.
 template <int KCD>
-__device__ __forceinline__ void deconv_issue(uint32_t dt, uint32_t sbase, uint32_t a_off, uint32_t lboA, int npos,
-                                             int Nd, int kcd, bool merged, uint32_t w0, uint32_t w1, uint32_t bTap,
-                                             uint32_t lboB, bool allow_split = true, int Mrows = 128,
-                                             uint32_t tapRows = 1) {
-  const bool msplit = allow_split && 2 * npos <= 128;
+__device__ __forceinline__ void deconv_issue(uint32_t dt, uint32_t sbase, uint32_t a_off, uint32_t lboA, int Nd,
+                                             int kcd, bool merged, uint32_t w0, uint32_t w1, uint32_t bTap,
+                                             uint32_t lboB, uint32_t tapRows) {
   const uint32_t stepA = (2 * lboA) >> 4;
-  if (merged && !msplit) {
-    const uint32_t idesc = tc_idesc_bf16(Mrows, 2 * Nd);
-    const uint64_t a0 = tc_desc(sbase + a_off, lboA, 128), b0 = tc_desc(sbase + w0, lboB, 128);
+  const uint64_t a0 = tc_desc(sbase + a_off, lboA, 128);
+  if (merged) {
+    const uint32_t idesc = tc_idesc_bf16(128, 2 * Nd);
+    const uint64_t b0 = tc_desc(sbase + w0, lboB, 128);
 #define VES_DEC(NK) issue_deconv<NK>(dt, a0, b0, bTap, stepA, (2 * lboB) >> 4, idesc, tapRows)
     VES_TC_NK_SWITCH(kcd / 2, VES_DEC)
 #undef VES_DEC
   } else {
     const uint32_t idesc = tc_idesc_bf16(128, Nd);
     for (int r = 0; r < 2; ++r) {
-      const int lift = msplit ? r * npos * 16 : 0;
-      const uint64_t a0 = tc_desc(sbase + a_off - lift, lboA, 128);
       const uint64_t b0 = tc_desc(sbase + (r ? w1 : w0), lboB, 128);
 #define VES_DEC(NK) issue_deconv<NK>(dt + r * Nd, a0, b0, bTap, stepA, (2 * lboB) >> 4, idesc, tapRows)
       VES_TC_NK_SWITCH(kcd / 2, VES_DEC)
 #undef VES_DEC
-    }
-  }
-}
-
-// Epilogue of a transposed conv over npos input rows: 8 channels of output
-// position 2q + r for this thread's lane go to dst[kc * pitch + 2q + r + row0].
-template <int KCD>
-__device__ __forceinline__ void deconv_epilogue(uint32_t dt, int qd, int lane, int npos, int Nd, int kcd, int nreal,
-                                                const float* cst, int ob, int os, int ot, uint4* dst, int pitch,
-                                                int row0, bool allow_split = true, int Mrows = 128) {
-  const bool msplit = allow_split && 2 * npos <= 128;
-  const int lane0 = 32 * qd;
-  if (!msplit) {
-    // both parities on this lane: one wait for the two parities' columns
-    if (acc_row0(Mrows, qd) >= npos) return;  // uniform per warp
-    const int q = acc_row(Mrows, qd, lane);
-    const bool own = q >= 0 && q < npos;
-#pragma unroll
-    for (int k0 = 0; k0 < (KCD ? KCD : 8); k0 += 4) {
-      if (k0 >= kcd) break;
-      float vv[64];
-      tc_ld32x2(dt + ((uint32_t)lane0 << 16) + 8 * k0, dt + ((uint32_t)lane0 << 16) + Nd + 8 * k0, vv);
-      if (own) {
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k0 + k < kcd)
-              dst[(size_t)(k0 + k) * pitch + 2 * q + r + row0] = act8(vv + 32 * r + 8 * k, cst, k0 + k, nreal, ob, os, ot);
-      }
-    }
-    return;
-  }
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    int q;
-    bool own = true;
-    if (msplit) {
-      if (lane0 < r * npos || lane0 >= (r + 1) * npos) continue;  // uniform per warp
-      q = lane0 + lane - r * npos;
-    } else {
-      if (acc_row0(Mrows, qd) >= npos) continue;  // uniform per warp
-      q = acc_row(Mrows, qd, lane);
-      own = q >= 0 && q < npos;
-    }
-#pragma unroll
-    for (int k0 = 0; k0 < (KCD ? KCD : 8); k0 += 4) {
-      if (k0 >= kcd) break;
-      float vv[32];
-      tc_ld32(dt + ((uint32_t)lane0 << 16) + r * Nd + 8 * k0, vv);
-      if (own) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (k0 + k < kcd)
-            dst[(size_t)(k0 + k) * pitch + 2 * q + r + row0] = act8(vv + 8 * k, cst, k0 + k, nreal, ob, os, ot);
-      }
     }
   }
 }
@@ -726,19 +664,23 @@ __device__ __forceinline__ void deconv_epilogue(uint32_t dt, int qd, int lane, i
 // image) or two MMAs on the same lanes.  KCD compile-time K chunk count (0:
 // from the geometry); NG warp groups (TMEM columns [128*wg, 128*wg + 2*Nd)
 // each).  Items are (group, tile) pairs, a.per_grp tiles per group.
+// The two warps on a lane quarter take one output parity each.  Its MMAs are
+// all math-bound (N = 2*Nd), so the groups issue whole batches in turn: 304 ->
+// 262 us (advection), 194 -> 175 us (near field) at 512 vesicles; in down and
+// up2, whose batches wait for shared memory, taking turns cost time.
 template <int KCD, int NG>
 __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bar[NG], mbar[NG];  // per warp group: MMA completion, intermediate arrival
   __shared__ uint32_t tbase;
-  __shared__ int fail[NG];
+  __shared__ int fail[NG], turn;
   const Geo& g = a.g;
   const int kcd = KCD ? KCD : g.kcd;
   const int L = g.L, L2 = L / 2, L4 = L / 4, V1 = g.v1;
   const int ntiles = a.per_grp;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wg = tid / kGroupThreads, gt = tid % kGroupThreads;
-  const int qd = warp & 3;
+  const int qd = warp & 3, r = gt >> 7;  // TMEM lane quarter; the output parity of this warp's epilogue
   const Range rg = my_items(a.items);
   if (rg.lo >= rg.hi) return;
   const uint32_t ncols = 512;
@@ -748,6 +690,7 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
       tc_mbar_init(&mbar[k], 1);
       fail[k] = 0;
     }
+    turn = 0;
     tc_mbar_fence_init();
   }
   if (warp == 0) tc_tmem_alloc(&tbase, ncols);
@@ -756,7 +699,9 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t dt = tbase + 128 * wg;
+  const int wgu = __shfl_sync(0xffffffffu, wg, 0);  // uniform across the warp
+  const bool issuer = __shfl_sync(0xffffffffu, gt >> 5, 0) == 0 && tc_elect();
+  const uint32_t dt = __shfl_sync(0xffffffffu, tbase, 0) + (NG == 2 ? 256 : 128) * wgu;
   const uint32_t sbase = tc_smem_u32(sm);
   const float* cst = reinterpret_cast<const float*>(sm + g.u1cst);
   const int PB = (L4 + 4) * V1;  // rows per K chunk: 2*v1 zero rows, the tile's L4*v1 rows, 2*v1 zero rows
@@ -771,10 +716,8 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
   unsigned phase = 0, mphase = 0;
   bool mpend = false;  // a bulk copy into bs is in flight
   // intermediate of a tile [kcd][L/4 * v1][16B] -> bs rows 2*v1 .. (L/4 + 2)*v1 - 1 of each chunk
-  auto fetch_mid = [&](long long item) {
+  auto fetch_mid = [&](int grp, long long t) {
     if (gt == 0) {
-      const int grp = (int)(item / ntiles);
-      const long long t = item % ntiles;
       const unsigned char* src = a.mid + ((size_t)t * a.G + grp) * (size_t)V1 * g.mid_bytes;
       tc_expect_tx(&mbar[wg], chunk * (uint32_t)kcd);
       for (int kc = 0; kc < kcd; ++kc) tc_bulk_g2s(bs + kc * PB + 2 * V1, src + (size_t)kc * chunk, chunk, &mbar[wg]);
@@ -788,9 +731,10 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
     copy16(sm, a.img + (size_t)sg.grp * g.u1size, g.u1size);
     tc_fence_async_smem();
     __syncthreads();
-    if (sg.lo + wg < sg.hi) fetch_mid(sg.lo + wg);
+    const long long t0 = (long long)sg.grp * ntiles;  // first item of the group
+    if (sg.lo + wg < sg.hi) fetch_mid(sg.grp, sg.lo + wg - t0);
     for (long long it = sg.lo + wg; it < sg.hi; it += NG) {
-      const long long t = it % ntiles;
+      const long long t = it - t0;
       if (!group_wait_one(&mbar[wg], mphase, a.st, 26, wg, gt, &fail[wg])) {
         failed = true;
         break;
@@ -798,10 +742,12 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
       mphase ^= 1;
       mpend = false;
       tc_fence_after_sync();
-      if (gt == 0) {
-        deconv_issue<KCD>(dt, sbase, g.u1bs + wg * g.u1grp, PB * 16, 128, Nd, kcd, g.u1merge != 0, g.u1w, w1, bTap,
-                          lboB1, false, 128, (uint32_t)V1);
-        tc_commit(&bar[wg]);
+      if (issuer) {
+        batch_begin(&turn);
+        deconv_issue<KCD>(dt, sbase, g.u1bs + wgu * g.u1grp, PB * 16, Nd, kcd, g.u1merge != 0, g.u1w, w1, bTap, lboB1,
+                          (uint32_t)V1);
+        tc_commit(&bar[wgu]);
+        batch_end(&turn);
       }
       if (!group_wait_one(&bar[wg], phase, a.st, 23, wg, gt, &fail[wg])) {
         failed = stuck = true;
@@ -810,24 +756,24 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
       phase ^= 1;
       tc_fence_after_sync();
       // bs is free once the MMAs have completed: this group's next item
-      if (it + NG < sg.hi) fetch_mid(it + NG);
-      // output positions 2q + r of vesicle t*v1 + j -> its up1 -> up2 record
+      if (it + NG < sg.hi) fetch_mid(sg.grp, t + NG);
+      // output positions 2q + r of vesicle t*v1 + j -> the record of its up2 tile
       const long long v = t * V1 + j;
       const bool own = v < a.nv;
-      uint4* dst = reinterpret_cast<uint4*>(a.mid2 + ((size_t)(own ? v : 0) * a.G + sg.grp) * g.mid2_bytes);
+      const int VU = g.vu;
+      const long long vs = own ? v : 0;
+      uint4* dst = reinterpret_cast<uint4*>(a.mid2 + ((size_t)(vs / VU) * a.G + sg.grp) * (size_t)VU * g.mid2_bytes) +
+                   (vs % VU);
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
+      for (int k0 = 0; k0 < (KCD ? KCD : 16); k0 += 4) {
+        if (k0 >= kcd) break;
+        float vv[32];
+        tc_ld32(dt + ((uint32_t)(32 * qd) << 16) + r * Nd + 8 * k0, vv);
+        if (own) {
 #pragma unroll
-        for (int k0 = 0; k0 < (KCD ? KCD : 8); k0 += 4) {
-          if (k0 >= kcd) break;
-          float vv[32];
-          tc_ld32(dt + ((uint32_t)(32 * qd) << 16) + r * Nd + 8 * k0, vv);
-          if (own) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (k0 + k < kcd)
-                dst[(size_t)(k0 + k) * L2 + 2 * q + r] = act8(vv + 8 * k, cst, k0 + k, g.d, 0, 128, 256);
-          }
+          for (int k = 0; k < 4; ++k)
+            if (k0 + k < kcd)
+              dst[((size_t)(k0 + k) * L2 + 2 * q + r) * VU] = act8(vv + 8 * k, cst, k0 + k, g.d, 0, 128, 256);
         }
       }
       tc_fence_before_sync();
@@ -843,12 +789,25 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
   if (warp == 0) tc_tmem_dealloc(tbase, ncols);
 }
 
-// up2: transposed conv 2, mix, residual and pass-through.  NG warp groups,
-// TMEM columns [cstride*wg, cstride*wg + 2*Nd + nh*Nm) each.
-template <int KCD, int NG>
+// up2: transposed conv 2, mix, residual and pass-through, on tiles of VU
+// vesicles with interleaved rows (row q*VU + j holds position q of the tile's
+// vesicle j).  At L = 128 a tile of two vesicles fills the 128 rows of a
+// transposed-conv MMA (one vesicle alone ran M = 64 MMAs at half the math
+// rate) and its mix is two MMAs of 128 rows; at L = 256 one vesicle is such a
+// tile.
+//
+// NG warp groups, TMEM columns [cstride*wg, + cstride) each.  The two warps on
+// a lane quarter take half of the channel chunks and one of the two mix
+// accumulators each.  The residual and the bias go into the mix accumulators
+// while the transposed conv runs, straight from global memory (prefetched into
+// L2 one item ahead), so the block input needs no shared memory.  The two
+// halves of the mix are issued by two threads.  Loading the residual one item
+// ahead into registers was slower (671 against 645 us at 512 vesicles of the
+// near field), as was one thread issuing both halves.
+template <int KCD, int NG, int VU>
 __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
-  __shared__ uint64_t bar[NG], mbar[NG], rbar[NG];  // per warp group: MMA completion, intermediate, block input
+  __shared__ uint64_t bar[NG], mbar[NG], xbar[NG];  // per warp group: transposed conv, intermediate, mix
   __shared__ uint32_t tbase;
   __shared__ int fail[NG];
   const Geo& g = a.g;
@@ -856,7 +815,8 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
   const int L = g.L, L2 = L / 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wg = tid / kGroupThreads, gt = tid % kGroupThreads;
-  const int qd = warp & 3;
+  const int qd = warp & 3, hw = gt >> 7;  // TMEM lane quarter; which of the two warps on it
+  const int nhalf = VU * L / 128;         // mix accumulators of 128 rows: 2, or 1 (L = 128, VU = 1)
   const Range rg = my_items(a.items);
   if (rg.lo >= rg.hi) return;
   const uint32_t ncols = 512;
@@ -864,7 +824,7 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
     for (int k = 0; k < NG; ++k) {
       tc_mbar_init(&bar[k], 1);
       tc_mbar_init(&mbar[k], 1);
-      tc_mbar_init(&rbar[k], 1);
+      tc_mbar_init(&xbar[k], nhalf);
       fail[k] = 0;
     }
     tc_mbar_fence_init();
@@ -875,165 +835,173 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t dt = tbase + (NG == 2 ? 256 : 160) * wg;
-  const uint32_t sbase = tc_smem_u32(sm);
-  const int goff = wg * g.u2grp;
-  const float* cst = reinterpret_cast<const float*>(sm + g.u2cst);
-  const int PC = L2 + 4, PD = L + 2;
   const int Nd = kcd * 8, Nm = rup(g.cmix, 16);
+  const int mcol = 2 * Nd;  // mix accumulators: 32 columns each, after the transposed conv's
+  // issue from uniform values with tiles of two vesicles only: at L = 256 the
+  // faster issue of three groups slowed the kernel (946 -> 1104 us at 512 vesicles)
+  constexpr bool kUniform = VU == 2;
+  const int wgu = kUniform ? __shfl_sync(0xffffffffu, wg, 0) : wg;
+  const int wiu = kUniform ? __shfl_sync(0xffffffffu, gt >> 5, 0) : 0;
+  const bool leader = kUniform ? tc_elect() : (gt & 127) == 0;
+  const uint32_t dt = (kUniform ? __shfl_sync(0xffffffffu, tbase, 0) : tbase) + (uint32_t)((2 * Nd + 32 * nhalf) * wgu);
+  const uint32_t lanes = (uint32_t)(32 * qd) << 16;
+  const uint32_t sbase = tc_smem_u32(sm);
+  const int goff = wgu * g.u2grp;
+  const float* cst = reinterpret_cast<const float*>(sm + g.u2cst);
+  const int PC = (L2 + 4) * VU, PD = (L + 2) * VU;
   const int cout = g.cmix + g.npass;
-  const int nh = L / 128;   // 128-position halves of the mix
-  const int mcol = 2 * Nd;  // first TMEM column of the mix accumulators (after the transposed conv's)
   uint4* cs = reinterpret_cast<uint4*>(sm + g.u2cs + goff);
   uint4* ds = reinterpret_cast<uint4*>(sm + g.u2ds + goff);
-  const float* xf = reinterpret_cast<const float*>(ds);  // block input while it sits in ds
   const bool need_x = g.residual || g.npass > 0;
-  // transposed conv of at most 64 input positions on the merged image: one
-  // M = 64 MMA per (tap, K step) with both parities on N
-  const bool m64dec = KCD != 0 && g.u2merge && L2 <= 64;
-  const uint32_t xbytes = (uint32_t)(g.cin * L * 4);
   const uint32_t bTap = (uint32_t)((g.u2merge ? 2 * Nd : g.d) * kcd * 16) >> 4;
   const uint32_t lboB = (uint32_t)((g.u2merge ? 2 * Nd : g.d) * 16);
   const uint32_t w1 = g.u2merge ? (uint32_t)(g.u2w + Nd * 16) : (uint32_t)(g.u2w + 5 * kcd * g.d * 16);
-  unsigned phase = 0, mphase = 0, rphase = 0;
-  bool mpend = false, rpend = false;  // bulk copies into cs / ds in flight
-  // up1 output [kcd][L/2][16B] of an item -> cs rows 2 .. L/2+1 of each chunk
-  auto fetch_mid = [&](long long item) {
+  // this thread's accumulator row: in the transposed conv input position q of
+  // the tile's vesicle j, in mix half hw output position pm of the same vesicle
+  const int row = 32 * qd + lane, q = row / VU, j = row % VU;
+  const int pm = (128 * hw + row) / VU;
+  const int ntl = a.per_grp;
+  unsigned phase = 0, mphase = 0, xphase = 0;
+  bool mpend = false, dpend = false, xpend = false;  // bulk copy into cs, transposed conv, mix in flight
+  // up1 output [kcd][L/2 * VU][16B] of tile t -> cs rows 2*VU .. (L/2 + 2)*VU - 1 of each chunk
+  auto fetch_mid = [&](int grp, long long t) {
     if (gt == 0) {
-      const int grp = (int)(item / a.nv);
-      const long long v = item % a.nv;
-      const unsigned char* src = a.mid2 + ((size_t)v * a.G + grp) * g.mid2_bytes;
-      tc_expect_tx(&mbar[wg], (uint32_t)g.mid2_bytes);
-      for (int kc = 0; kc < kcd; ++kc) tc_bulk_g2s(cs + kc * PC + 2, src + kc * L2 * 16, L2 * 16, &mbar[wg]);
+      const unsigned char* src = a.mid2 + ((size_t)t * a.G + grp) * (size_t)VU * g.mid2_bytes;
+      tc_expect_tx(&mbar[wg], (uint32_t)(VU * g.mid2_bytes));
+      for (int kc = 0; kc < kcd; ++kc)
+        tc_bulk_g2s(cs + kc * PC + 2 * VU, src + (size_t)kc * L2 * VU * 16, (uint32_t)(L2 * VU * 16), &mbar[wg]);
     }
     mpend = true;
   };
-  // block input x[v][grp*cin + c][pos] of an item -> ds (free once the
-  // group's previous mix has completed)
-  auto fetch_x = [&](long long item) {
-    if (gt == 0) {
-      const int grp = (int)(item / a.nv);
-      const long long v = item % a.nv;
-      tc_expect_tx(&rbar[wg], xbytes);
-      tc_bulk_g2s(ds, a.x + ((long long)v * a.G + grp) * (long long)g.cin * L, xbytes, &rbar[wg]);
-    }
-    rpend = true;
+  // block input x[v][grp*cin + c][pos] of tile t -> L2
+  auto fetch_x = [&](int grp, long long t) {
+    const long long v = t * VU + (gt - 32);
+    if (gt >= 32 && gt < 32 + VU && v < a.nv)
+      tc_prefetch_l2(a.x + (v * a.G + grp) * (long long)g.cin * L, (uint32_t)(g.cin * L * 4));
   };
-  bool failed = false, stuck = false;
+  bool failed = false;
   for (long long lo = rg.lo; lo < rg.hi && !failed;) {
-    const Seg sg = next_seg(lo, rg.hi, a.nv);
+    const Seg sg = next_seg(lo, rg.hi, ntl);
     __syncthreads();
     copy16(sm, a.img + (size_t)sg.grp * g.u2size, g.u2size);
     tc_fence_async_smem();
     __syncthreads();
+    const long long t0 = (long long)sg.grp * ntl;  // first item of the group
     if (sg.lo + wg < sg.hi) {
-      fetch_mid(sg.lo + wg);
-      if (need_x) fetch_x(sg.lo + wg);
+      fetch_mid(sg.grp, sg.lo + wg - t0);
+      if (need_x) fetch_x(sg.grp, sg.lo + wg - t0);
     }
     for (long long it = sg.lo + wg; it < sg.hi; it += NG) {
-      const long long v = it % a.nv;
-      float* __restrict__ op = a.out + ((long long)v * a.G + sg.grp) * (long long)cout * L;
-      if (need_x) {
-        if (!group_wait_one(&rbar[wg], rphase, a.st, 27, wg, gt, &fail[wg])) {
-          failed = true;
-          break;
-        }
-        rphase ^= 1;
-        rpend = false;
-        // pass-through channels
-        const float4* src = reinterpret_cast<const float4*>(xf + (size_t)(g.cin - g.npass) * L);
-        float4* dst = reinterpret_cast<float4*>(op + (size_t)g.cmix * L);
-        for (int i = gt; i < g.npass * L / 4; i += kGroupThreads) dst[i] = src[i];
-      }
-      {
-        // mix accumulators preset to residual + bias (columns [mcol, mcol + nh*Nm))
-        const int p0 = 32 * qd + lane;
-        for (int h = 0; h < nh; ++h) {
-          float r0[32];
-#pragma unroll
-          for (int o = 0; o < 32; ++o) {
-            const bool on = o < g.cmix;
-            r0[o] = (on && g.residual ? xf[o * L + 128 * h + p0] : 0.f) + (on ? cst[768 + o] : 0.f);
-          }
-          tc_st32(dt + ((uint32_t)(32 * qd) << 16) + mcol + h * Nm, r0);
-        }
-        tc_wait_st();
-      }
+      const long long v = (it - t0) * VU + j;
+      const bool on = hw < nhalf && v < a.nv;
+      const long long vs = v < a.nv ? v : 0;
+      const float* __restrict__ xp = a.x + (vs * a.G + sg.grp) * (long long)g.cin * L + pm;
+      float* __restrict__ op = a.out + (vs * a.G + sg.grp) * (long long)cout * L + pm;
       if (!group_wait_one(&mbar[wg], mphase, a.st, 26, wg, gt, &fail[wg])) {
         failed = true;
         break;
       }
       mphase ^= 1;
       mpend = false;
-      group_sync_for_mma(wg);  // also: every read of the block input in ds is done
-      if (gt == 0) {
-        deconv_issue<KCD>(dt, sbase, g.u2cs + goff, PC * 16, L2, Nd, kcd, g.u2merge != 0, g.u2w, w1, bTap, lboB,
-                          !m64dec, m64dec ? 64 : 128);
-        tc_commit(&bar[wg]);
+      tc_fence_after_sync();  // every TMEM read of the previous item is done
+      if (kUniform ? wiu == 0 && leader : gt == 0) {
+        deconv_issue<KCD>(dt, sbase, g.u2cs + goff, PC * 16, Nd, kcd, g.u2merge != 0, g.u2w, w1, bTap, lboB, VU);
+        tc_commit(&bar[wgu]);
+      }
+      dpend = true;
+      if (need_x && it + NG < sg.hi) fetch_x(sg.grp, it + NG - t0);
+      if (hw < nhalf) {
+        // mix accumulator hw preset to residual + bias while the transposed conv runs
+        float r0[32];
+#pragma unroll
+        for (int o = 0; o < 32; ++o) r0[o] = (o < g.cmix && g.residual && on) ? __ldg(xp + o * L) : 0.f;
+#pragma unroll
+        for (int o = 0; o < 32; ++o) r0[o] = r0[o] + (o < g.cmix ? cst[768 + o] : 0.f);
+        tc_st32(dt + lanes + mcol + 32 * hw, r0);
+        // pass-through channels
+        if (on)
+          for (int c = 0; c < g.npass; ++c) op[(g.cmix + c) * L] = __ldg(xp + (g.cin - g.npass + c) * L);
+        tc_wait_st();
       }
       if (!group_wait_one(&bar[wg], phase, a.st, 24, wg, gt, &fail[wg])) {
-        failed = stuck = true;
+        failed = true;
         break;
       }
       phase ^= 1;
+      dpend = false;
       tc_fence_after_sync();
       // cs is free once the transposed conv has completed: this group's next item
-      if (it + NG < sg.hi) fetch_mid(it + NG);
-      if (m64dec) {
-        // M = 64 rows (input positions q), parity r = lane / 16 at TMEM columns r*Nd (16x32bx2 loads)
-        const int q = 16 * qd + (lane & 15), r = lane >> 4;
+      if (it + NG < sg.hi) fetch_mid(sg.grp, it + NG - t0);
+      if (32 * qd < L2 * VU) {  // uniform per warp
+        const bool own = row < L2 * VU;
+        const int k1 = hw ? kcd : kcd / 2;
+        if (VU == 2) {
+          // both parities of two chunks at a time: one read of the constants serves both
 #pragma unroll
-        for (int k0 = 0; k0 < (KCD ? KCD : 8); k0 += 4) {
-          float vv[32];
-          tc_ld16x2_32<(KCD ? KCD : 8) * 8>(dt + ((uint32_t)(32 * qd) << 16) + 8 * k0, vv);
+          for (int kk = 0; kk < (KCD ? KCD / 2 : 8); kk += 2) {
+            const int k0 = hw * (kcd / 2) + kk;
+            if (k0 >= k1) break;
+            float vv[32];
+            tc_ld16x2(dt + lanes + 8 * k0, dt + lanes + Nd + 8 * k0, vv);
+            if (own) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k0 + k < kcd) ds[(size_t)(k0 + k) * PD + 2 * q + r + 1] = act8(vv + 8 * k, cst, k0 + k, g.d, 384, 512, 640);
+              for (int k = 0; k < 2; ++k)
+                if ((KCD == 0 || kk + k < KCD / 2) && k0 + k < k1) {
+                  const uint4 e0 = act8(vv + 8 * k, cst, k0 + k, g.d, 384, 512, 640);
+                  const uint4 e1 = act8(vv + 16 + 8 * k, cst, k0 + k, g.d, 384, 512, 640);
+                  uint4* o = ds + (size_t)(k0 + k) * PD + (2 * q + 1) * VU + j;
+                  o[0] = e0;
+                  o[VU] = e1;
+                }
+            }
+          }
+        } else {
+          // one parity at a time (80 registers with three groups)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int kk = 0; kk < (KCD ? KCD / 2 : 8); kk += 4) {
+              const int k0 = hw * (kcd / 2) + kk;
+              if (k0 >= k1) break;
+              float vv[32];
+              tc_ld32(dt + lanes + r * Nd + 8 * k0, vv);
+              if (own) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  if ((KCD == 0 || kk + k < KCD / 2) && k0 + k < k1)
+                    ds[(size_t)(k0 + k) * PD + (2 * q + r + 1) * VU + j] = act8(vv + 8 * k, cst, k0 + k, g.d, 384, 512, 640);
+              }
+            }
+          }
         }
-      } else {
-        deconv_epilogue<KCD>(dt, qd, lane, L2, Nd, kcd, g.d, cst, 384, 512, 640, ds, PD, 1);
       }
-      // the halo rows of ds (zero padding of the mix) held block input
-      if (gt < 2 * kcd) ds[(gt >> 1) * PD + ((gt & 1) ? L + 1 : 0)] = make_uint4(0, 0, 0, 0);
       group_sync_for_mma(wg);
-      // mix: D[p][o] = sum_t d[p + t - 1] M_t; positions in halves of 128 rows
-      if (gt == 0) {
+      // mix: D[p][o] = sum_t d[p + t - 1] M_t onto residual + bias, 128 rows per issuing thread
+      if (leader && hw < nhalf && (!kUniform || (wiu & 3) == 0)) {
         const uint32_t idesc = tc_idesc_bf16(128, Nm);
         const uint32_t lboA = PD * 16, lboM = g.cmix * 16;
         const uint64_t a0 = tc_desc(sbase + g.u2ds + goff, lboA, 128), b0 = tc_desc(sbase + g.u2wm, lboM, 128);
-        for (int h = 0; h < nh; ++h) {  // onto residual + bias
-#define VES_MIX(NK) issue_mix<NK>(dt + mcol + h * Nm, a0 + (uint32_t)(128 * h), b0, (kcd * lboM) >> 4, (2 * lboA) >> 4, (2 * lboM) >> 4, idesc)
-          VES_TC_NK_SWITCH(kcd / 2, VES_MIX)
+        const uint32_t hh = kUniform ? (uint32_t)wiu >> 2 : (uint32_t)hw;
+#define VES_MIX(NK) issue_mix<NK>(dt + mcol + 32 * hh, a0 + 128 * hh, b0, (kcd * lboM) >> 4, (2 * lboA) >> 4, (2 * lboM) >> 4, idesc, VU)
+        VES_TC_NK_SWITCH(kcd / 2, VES_MIX)
 #undef VES_MIX
-        }
-        tc_commit(&bar[wg]);
+        tc_commit(&xbar[wgu]);
       }
-      if (!group_wait_one(&bar[wg], phase, a.st, 25, wg, gt, &fail[wg])) {
-        failed = stuck = true;
+      xpend = true;
+      if (!group_wait_one(&xbar[wg], xphase, a.st, 25, wg, gt, &fail[wg])) {
+        failed = true;
         break;
       }
-      phase ^= 1;
+      xphase ^= 1;
+      xpend = false;
       tc_fence_after_sync();
-      // ds is free once the mix has completed: the block input of this group's next item
-      if (need_x && it + NG < sg.hi) fetch_x(it + NG);
-      if (nh == 2) {  // both 128-position halves, one wait
-        const int p = 32 * qd + lane;
-        float vv[64];
-        tc_ld32x2(dt + ((uint32_t)(32 * qd) << 16) + mcol, dt + ((uint32_t)(32 * qd) << 16) + mcol + Nm, vv);
-#pragma unroll
-        for (int o = 0; o < 32; ++o)
-          if (o < g.cmix) {
-            op[(size_t)o * L + p] = vv[o];
-            op[(size_t)o * L + 128 + p] = vv[32 + o];
-          }
-      } else {
-        for (int h = 0; h < nh; ++h) {
-          const int p = 128 * h + 32 * qd + lane;
-          float vv[32];
-          tc_ld32(dt + ((uint32_t)(32 * qd) << 16) + mcol + h * Nm, vv);
+      if (hw < nhalf) {
+        float vv[32];
+        tc_ld32(dt + lanes + mcol + 32 * hw, vv);
+        if (on) {
 #pragma unroll
           for (int o = 0; o < 32; ++o)
-            if (o < g.cmix) op[(size_t)o * L + p] = vv[o];
+            if (o < g.cmix) op[o * L] = vv[o];
         }
       }
       tc_fence_before_sync();
@@ -1043,9 +1011,9 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
     failed = __syncthreads_or(failed ? 1 : 0) != 0;  // every thread takes part
   }
   // bounded drains: this group's MMAs and bulk copies still in flight after a failure
-  if (stuck) tc_mbar_wait(&bar[wg], phase, nullptr, 0);
+  if (dpend) tc_mbar_wait(&bar[wg], phase, nullptr, 0);
+  if (xpend) tc_mbar_wait(&xbar[wg], xphase, nullptr, 0);
   if (mpend) tc_mbar_wait(&mbar[wg], mphase, nullptr, 0);
-  if (rpend) tc_mbar_wait(&rbar[wg], rphase, nullptr, 0);
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tc_tmem_dealloc(tbase, ncols);
@@ -1204,44 +1172,36 @@ int tcnet_pack(const ves_net_block& b, int G, int L, const float* const* p, std:
   return VES_OK;
 }
 
-// Warp groups allowed in the down kernel (VES_TC_DOWN_GROUPS=2 or 3 caps
-// them; read once).
-static int tcnet_down_groups_max() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("VES_TC_DOWN_GROUPS");
-    const int k = e ? atoi(e) : 4;
-    v = (k == 2 || k == 3) ? k : 4;
-  }
-  return v;
-}
-
 namespace {
 
 // compiled chunk-count variants; others run the generic kernels
-void (*pick_down(int kc1, int kcd, int ng))(tcnet::KArgs) {
+void (*pick_down(int kc1, int kcd, int ng, int vd))(tcnet::KArgs) {
   using namespace tcnet;
-#define VES_DK(A, B) return ng == 4 ? down_kernel<A, B, 4> : (ng == 3 ? down_kernel<A, B, 3> : down_kernel<A, B, 2>)
-  if (kc1 == 4 && kcd == 6) VES_DK(4, 6);
-  if (kc1 == 6 && kcd == 6) VES_DK(6, 6);
-  if (kc1 == 6 && kcd == 8) VES_DK(6, 8);
-  if (kc1 == 8 && kcd == 8) VES_DK(8, 8);
-  VES_DK(0, 0);
+#define VES_DK(A, B, V) return ng == 3 ? down_kernel<A, B, 3, V> : down_kernel<A, B, 2, V>
+  if (vd == 1) {
+    if (kc1 == 4 && kcd == 6) VES_DK(4, 6, 1);
+    VES_DK(0, 0, 1);
+  }
+  if (kc1 == 6 && kcd == 6) VES_DK(6, 6, 2);
+  if (kc1 == 6 && kcd == 8) VES_DK(6, 8, 2);
+  if (kc1 == 8 && kcd == 8) VES_DK(8, 8, 2);
+  VES_DK(0, 0, 2);
 #undef VES_DK
 }
 
 void (*pick_up1(int kcd, int ng))(tcnet::KArgs) {
   using namespace tcnet;
-  if (kcd == 6) return ng == 4 ? up1_kernel<6, 4> : up1_kernel<6, 2>;
-  if (kcd == 8) return ng == 4 ? up1_kernel<8, 4> : up1_kernel<8, 2>;
-  return ng == 4 ? up1_kernel<0, 4> : up1_kernel<0, 2>;
+  if (kcd == 6) return ng == 3 ? up1_kernel<6, 3> : up1_kernel<6, 2>;
+  if (kcd == 8) return ng == 3 ? up1_kernel<8, 3> : up1_kernel<8, 2>;
+  return ng == 3 ? up1_kernel<0, 3> : up1_kernel<0, 2>;
 }
 
-void (*pick_up2(int kcd, int ng))(tcnet::KArgs) {
+void (*pick_up2(int kcd, int ng, int vu))(tcnet::KArgs) {
   using namespace tcnet;
-  if (kcd == 6) return ng == 3 ? up2_kernel<6, 3> : up2_kernel<6, 2>;
-  if (kcd == 8) return ng == 3 ? up2_kernel<8, 3> : up2_kernel<8, 2>;
-  return ng == 3 ? up2_kernel<0, 3> : up2_kernel<0, 2>;
+  if (vu == 2) return kcd == 6 ? (ng == 3 ? up2_kernel<6, 3, 2> : up2_kernel<6, 2, 2>)
+                               : (kcd == 8 ? up2_kernel<8, 2, 2> : up2_kernel<0, 2, 2>);
+  if (kcd == 6 && ng > 1) return ng == 3 ? up2_kernel<6, 3, 1> : up2_kernel<6, 2, 1>;
+  return ng == 1 ? up2_kernel<0, 1, 1> : up2_kernel<0, 2, 1>;
 }
 
 bool autotune_log() {
@@ -1269,7 +1229,6 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
   const Geo& g = a.g;
   a.G = G;
   a.nv = nv;
-  a.m64 = 0;
   a.items = (long long)G * nv;
   a.x = x;
   a.out = out;
@@ -1283,23 +1242,21 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int kc1 = g.kc1, kcd = g.kcd, Nd = kcd * 8;
   // warp groups per CTA that fit: TMEM (512 columns) and shared memory
-  const int down3 = g.dxs + 3 * g.dgrp + kTail, down4 = g.dxs + 4 * g.dgrp + kTail,
-            up1_4 = g.u1size + 4 * g.u1grp + kTail, up2_3 = g.u2size + 3 * g.u2grp + kTail;
+  const int down3 = g.dxs + 3 * g.dgrp + kTail, up1_3 = g.u1size + 3 * g.u1grp + kTail, up2_3 = g.u2size + 3 * g.u2grp + kTail;
+  const int ucols = 2 * Nd + 32 * (g.vu * g.L / 128);  // TMEM columns per up2 group
   const bool dn3 = (kc1 + kcd) * 8 <= 128 && down3 <= kMaxSmem;
-  const bool dn4 = dn3 && down4 <= kMaxSmem;
-  const bool u14 = 2 * Nd <= 128 && up1_4 <= kMaxSmem;
-  const bool u23 = 2 * Nd + (g.L / 128) * rup(g.cmix, 16) <= 160 && up2_3 <= kMaxSmem;
+  const bool u13 = 2 * Nd <= 128 && up1_3 <= kMaxSmem;
+  const bool u22 = 2 * ucols <= 512, u23 = kcd == 6 && 3 * ucols <= 512 && up2_3 <= kMaxSmem;
   const int grid = (int)std::min<long long>(a.items, (long long)nsm);
   // one CTA per SM (it allocates all 512 TMEM columns): at least 117 KB of
   // shared memory per CTA keeps a second one off the SM
-  auto launch = [&](int which, int ng, int m64) -> int {
+  auto launch = [&](int which, int ng) -> int {
     KArgs b = a;
-    b.m64 = m64;
     void (*fn)(KArgs);
     int smem;
     int nblk = grid;
     if (which == 0) {
-      fn = pick_down(kc1, kcd, ng);
+      fn = pick_down(kc1, kcd, ng, g.vd);
       smem = std::max(g.dxs + ng * g.dgrp + kTail, kMinSmem);
       b.img = d_down;
       b.per_grp = (nv + g.vd - 1) / g.vd;  // items: (group, tile of vd vesicles)
@@ -1313,9 +1270,12 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
       b.items = (long long)G * ntiles;
       nblk = (int)std::min<long long>(b.items, (long long)nsm);
     } else {
-      fn = pick_up2(kcd, ng);
+      fn = pick_up2(kcd, ng, g.vu);
       smem = std::max(g.u2size + ng * g.u2grp + kTail, kMinSmem);
       b.img = d_up2;
+      b.per_grp = (nv + g.vu - 1) / g.vu;  // items: (group, tile of vu vesicles)
+      b.items = (long long)G * b.per_grp;
+      nblk = (int)std::min<long long>(b.items, (long long)nsm);
     }
     int rc = ves_cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "tc smem attribute");
@@ -1324,11 +1284,8 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
     fn<<<nblk, ng * kGroupThreads, smem, s>>>(b);
     return ves_launch_check("tc net block");
   };
-  // the fixed rule: the most warp groups that fit, M = 64 MMAs where allowed
-  const int m64_default = tcnet_m64() ? 1 : 0;
-  const int dmax = tcnet_down_groups_max();
-  TcPlan plan{nv, (dn4 && dmax >= 4) ? 4 : ((dn3 && dmax >= 3) ? 3 : 2), m64_default, u14 ? 4 : 2, m64_default,
-              u23 ? 3 : 2};
+  // the fixed rule: the most warp groups that fit
+  TcPlan plan{nv, dn3 ? 3 : 2, u13 ? 3 : 2, u23 ? 3 : (u22 ? 2 : 1)};
   const TcPlan* found = nullptr;
   for (const TcPlan& p : tb.plans)
     if (p.nv == nv) found = &p;
@@ -1339,11 +1296,11 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
     int rc = ves_cuda_status(cudaEventCreate(&e0), "tune event");
     if (!rc) rc = ves_cuda_status(cudaEventCreate(&e1), "tune event");
     if (rc) return rc;
-    auto timed = [&](int which, int ng, int m64, float& ms) -> int {
+    auto timed = [&](int which, int ng, float& ms) -> int {
       ms = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
         int r = ves_cuda_status(cudaEventRecord(e0, s), "tune record");
-        if (!r) r = launch(which, ng, m64);
+        if (!r) r = launch(which, ng);
         if (!r) r = ves_cuda_status(cudaEventRecord(e1, s), "tune record");
         if (!r) r = ves_cuda_status(cudaEventSynchronize(e1), "tune sync");
         float t = 0.f;
@@ -1355,29 +1312,23 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
     };
     float best = 1e30f, t = 0.f;
     // each kernel in the order the block runs them, so that the next one reads a valid input
-    const int ngd[3] = {2, 3, 4};
-    for (int i = 0; i < 3 && !rc; ++i) {
-      const int ng = ngd[i];
-      if ((ng == 3 && !dn3) || (ng == 4 && !dn4)) continue;
-      for (int m = 0; m < 2 && !rc; ++m) {
-        if ((rc = timed(0, ng, m, t))) break;
-        if (t < best) best = t, plan.ng_down = ng, plan.m64_down = m;
-      }
+    for (int ng = 2; ng <= 3 && !rc; ++ng) {
+      if (ng == 3 && !dn3) continue;
+      if ((rc = timed(0, ng, t))) break;
+      if (t < best) best = t, plan.ng_down = ng;
     }
-    if (!rc) rc = launch(0, plan.ng_down, plan.m64_down);
-    best = 1e30f;
-    for (int ng = 2; ng <= 4 && !rc; ng += 2) {
-      if (ng == 4 && !u14) continue;
-      for (int m = 0; m < 1 && !rc; ++m) {
-        if ((rc = timed(1, ng, m, t))) break;
-        if (t < best) best = t, plan.ng_up1 = ng, plan.m64_up1 = m;
-      }
-    }
-    if (!rc) rc = launch(1, plan.ng_up1, plan.m64_up1);
+    if (!rc) rc = launch(0, plan.ng_down);
     best = 1e30f;
     for (int ng = 2; ng <= 3 && !rc; ++ng) {
-      if (ng == 3 && !u23) continue;
-      if ((rc = timed(2, ng, 0, t))) break;
+      if (ng == 3 && !u13) continue;
+      if ((rc = timed(1, ng, t))) break;
+      if (t < best) best = t, plan.ng_up1 = ng;
+    }
+    if (!rc) rc = launch(1, plan.ng_up1);
+    best = 1e30f;
+    for (int ng = u22 ? 2 : 1; ng <= 3 && !rc; ++ng) {
+      if ((ng == 2 && !u22) || (ng == 3 && !u23)) continue;
+      if ((rc = timed(2, ng, t))) break;
       if (t < best) best = t, plan.ng_up2 = ng;
     }
     cudaEventDestroy(e0);
@@ -1385,11 +1336,11 @@ int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_dow
     if (rc) return rc;
     tb.plans.push_back(plan);
     if (autotune_log())
-      fprintf(stderr, "tcnet autotune: L=%d kc1=%d kcd=%d nv=%d -> down %d groups m64 %d, up1 %d groups m64 %d, up2 %d groups\n",
-              g.L, kc1, kcd, nv, plan.ng_down, plan.m64_down, plan.ng_up1, plan.m64_up1, plan.ng_up2);
+      fprintf(stderr, "tcnet autotune: L=%d kc1=%d kcd=%d nv=%d -> down %d groups, up1 %d groups, up2 %d groups\n", g.L,
+              kc1, kcd, nv, plan.ng_down, plan.ng_up1, plan.ng_up2);
   }
-  int rc = launch(0, plan.ng_down, plan.m64_down);
-  if (!rc) rc = launch(1, plan.ng_up1, plan.m64_up1);
-  if (!rc) rc = launch(2, plan.ng_up2, 0);
+  int rc = launch(0, plan.ng_down);
+  if (!rc) rc = launch(1, plan.ng_up1);
+  if (!rc) rc = launch(2, plan.ng_up2);
   return rc;
 }

@@ -5,11 +5,10 @@
 
 #include "ves_internal.h"
 
-// Launch shape of one block's three kernels: warp groups per CTA and M = 64
-// MMAs (for layers of at most 64 positions) in down and up1.
+// Launch shape of one block's three kernels: warp groups per CTA.
 struct TcPlan {
   int nv;
-  int ng_down, m64_down, ng_up1, m64_up1, ng_up2;
+  int ng_down, ng_up1, ng_up2;
 };
 
 struct TcBlock {
@@ -28,8 +27,7 @@ int tcnet_pack(const ves_net_block& b, int G, int L, const float* const* params,
 // One block: x [nv][G*cin][L] -> out [nv][G*cout][L] (FP32), mid = scratch of
 // (nv rounded up to a multiple of 4)*G*mid_bytes.
 // autotune: on the first call for a vesicle count, time every launch shape
-// that fits (warp groups per CTA, M = 64 MMAs on or off) of each kernel on
-// this input and keep the fastest for later calls with that count (the
+// that fits (warp groups per CTA) of each kernel on this input and keep the fastest for later calls with that count (the
 // stream is synchronised during the timing); otherwise the fixed rule.
 int tcnet_run_block(const TcBlock& tb, int G, int nv, const unsigned char* d_down, const unsigned char* d_up1,
                     const unsigned char* d_up2, const float* x, float* out, unsigned char* mid,
