@@ -27,6 +27,7 @@
 //   reduction over the ranges produces the result (deterministic).
 // * The FP64 rule (parity) has its own kernel, ff64_kernel below.
 #include "ves_internal.h"
+#include "ves_log_table.cuh"
 
 namespace {
 
@@ -373,16 +374,51 @@ __global__ void ff_reduce_kernel(long long total_pts, int ntp, int nsplit, const
 }
 
 // --------------------------------------------------------------------------
-// FP64 direct rule.  Bound by the FP64 pipe (2 fma/clk/SM: a pair costs ~70
-// FP64 instructions in log2 and the divide, 16 cycles each per warp), so the
-// operands need no staging: what matters is that every SM has several warps.
-// One thread per target point, and the sources are cut into pieces of a
-// vesicle (``chunk`` points), ``per_split`` pieces per CTA row; a small
-// suspension then spreads over the chip where whole source vesicles staged
-// two at a time left it to a single CTA (16 vesicles of N = 32: 43 ms per sum
-// on one SM, 0.17 ms like this).  Each piece is summed relative to
-// its vesicle's centre as in the FP32 kernel, the centre's log times the
-// vesicle's density sum being added with the first piece.
+// FP64 direct rule.  Bound by the FP64 pipe (2 fma/clk/SM, 16 cycles per warp
+// instruction), so what counts is the instructions per pair: the reciprocal
+// and the logarithm share one table look-up and one reduced argument
+// (rcp_log), ~30 in all where 1 / x and log2 of the library brought it to ~72;
+// the operands need no staging.  One thread per target point, and the sources
+// are cut into pieces of a vesicle (``chunk`` points), ``per_split`` pieces per
+// CTA row, so that a small suspension spreads over the chip where whole source
+// vesicles staged two at a time left it to a single CTA.  One sum, 16 vesicles
+// of N = 32: 43 ms on one SM, 0.170 ms in pieces, 0.104 ms with the shared
+// look-up.  Against 113-bit sums (16 to 64 points, 10 to 40 vesicles) the
+// relative error is 2.7-3.6e-16, as it was (2.7-4.9e-16).  Each piece is summed relative to its vesicle's centre as in
+// the FP32 kernel, the centre's log times the vesicle's density sum being
+// added with the first piece.
+//
+// 1 / x and ln x of a positive normal x = 2^k m, m in [sqrt(1/2), sqrt(2)):
+// with the table's y near 1 / m and r = m y - 1 (|r| < 2^-6.9, exact up to
+// rounding), ln x = k ln 2 - ln y + ln(1 + r) by the series to r^8, and 1 / m
+// = y (1 - r)(1 + r^2) corrected by one Newton step.  Both within 1.3 units in
+// the last place on 2e4 arguments against 50 digits.  Anything else (0,
+// subnormal, infinite, NaN) takes the library's functions.
+__device__ __forceinline__ void rcp_log(double x, const double2* __restrict__ tab, double& inv, double& lg) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  if (h - 0x00100000u >= 0x7fe00000u) {
+    inv = 1.0 / x;
+    lg = log(x);
+    return;
+  }
+  const uint32_t hx = h + (0x3ff00000u - 0x3fe6a09eu);
+  const int k = (int)(hx >> 20) - 0x3ff;
+  const uint32_t hm = (hx & 0xfffffu) + 0x3fe6a09eu;
+  const double m = __hiloint2double((int)hm, __double2loint(x));
+  const double2 t = tab[(hm - 0x3fe6a09eu) >> 13];
+  const double r = fma(m, t.x, -1.0), r2 = r * r;
+  double y = fma(-r, t.x, t.x);
+  y = fma(y, r2, y);
+  y = fma(y, fma(-m, y, 1.0), y);
+  // y 2^-k by its exponent (1 / x is subnormal only where x is not below 2^1022)
+  inv = k < 1020 && k > -1020 ? __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y)) : 1.0 / x;
+  const double kd = __hiloint2double(0x43300000, (int)((uint32_t)k ^ 0x80000000u)) - 4503601774854144.0;  // k
+  double q = fma(r2, -0.125, fma(r, 1.0 / 7, -1.0 / 6));
+  q = fma(r2, q, fma(r, 0.2, -0.25));
+  q = fma(r2, q, fma(r, 1.0 / 3, -0.5));
+  lg = fma(kd, 0.69314718055994530942, t.y) + fma(r2, q, r);
+}
+
 struct FF64Args {
   int nsrc, ns, ntp;
   long long total_pts;
@@ -404,6 +440,10 @@ struct FF64Args {
 constexpr int FF64_THREADS = 128;
 
 __global__ void __launch_bounds__(FF64_THREADS) ff64_kernel(FF64Args p) {
+  __shared__ double2 tab[128];
+  static_assert(FF64_THREADS == 128, "one table entry per thread");
+  tab[threadIdx.x] = kLogTab[threadIdx.x];
+  __syncthreads();
   const long long pt = (long long)blockIdx.x * FF64_THREADS + threadIdx.x;
   const bool valid = pt < p.total_pts;
   const long long pq = valid ? pt : 0;
@@ -441,19 +481,19 @@ __global__ void __launch_bounds__(FF64_THREADS) ff64_kernel(FF64Args p) {
       const double2 b = __ldg(reinterpret_cast<const double2*>(S + j) + 1);
       const double dx = tx - a.x, dy = ty - a.y;
       const double r2 = fma(dx, dx, dy * dy);
-      const double inv = 1.0 / r2;
-      const double lg = log2(r2 * irc2);
-      const double cc = fma(dx, b.x, dy * b.y) * inv;
+      double inv, lg;
+      rcp_log(r2 * irc2, tab, inv, lg);
+      const double cc = fma(dx, b.x, dy * b.y) * (inv * irc2);
       acx = fma(cc, dx, acx);
       acy = fma(cc, dy, acy);
       alx = fma(lg, b.x, alx);
       aly = fma(lg, b.y, aly);
     }
     if (use) {
-      double px = acx - FF_HALF_LN2 * alx, py = acy - FF_HALF_LN2 * aly;
+      double px = acx - 0.5 * alx, py = acy - 0.5 * aly;
       if (c == 0) {
         const double2 ds = p.src_dsum[s];
-        const double lgc = FF_HALF_LN2 * log2(rc2);
+        const double lgc = 0.5 * log(rc2);
         px = fma(-lgc, ds.x, px);
         py = fma(-lgc, ds.y, py);
       }
