@@ -426,39 +426,41 @@ void launch_geom_prop(const ves_ctx* c, int nv, const double* X, double* ra, dou
 }
 
 // ----------------------------------------------------------------------------
-// tracJump (capsules.py:54-80): f = -kappa (isa D)^4 X + isa D (sigma X_s)
-__global__ void trac_jump_kernel(int N, const double* __restrict__ dstencil, double kappa,
-                                 const double* __restrict__ isa, const double* __restrict__ tang,
-                                 const double* __restrict__ X, long long xs,
-                                 const double* __restrict__ sig, long long ss,
-                                 double* __restrict__ f) {
+// tracJump (capsules.py:54-80): f = -kappa (isa D)^4 X + isa D (sigma X_s);
+// one half of the CTA per component (the five derivatives of a component
+// follow one another, the two components do not: 16 vesicles of N = 32 39 ->
+// 20 us; large suspensions are bound by the FP64 pipe either way)
+__global__ void __launch_bounds__(512) trac_jump_kernel(int N, const double* __restrict__ dstencil, double kappa,
+                                                        const double* __restrict__ isa,
+                                                        const double* __restrict__ tang,
+                                                        const double* __restrict__ X, long long xs,
+                                                        const double* __restrict__ sig, long long ss,
+                                                        double* __restrict__ f) {
   extern __shared__ double sh[];
+  const int half = blockDim.x / 2, comp = threadIdx.x >= half, t = threadIdx.x - comp * half;
   double* d = sh;
-  double* a = d + N;
+  double* is = d + N;
+  double* a = is + N + comp * 2 * N;
   double* b = a + N;
-  double* is = b + N;
   const int k = blockIdx.x;
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     d[i] = dstencil[i];
     is[i] = isa[(long long)k * N + i];
   }
-  for (int comp = 0; comp < 2; ++comp) {
+  for (int i = t; i < N; i += half) a[i] = X[(long long)k * xs + comp * N + i];
+  __syncthreads();
+  for (int it = 0; it < 2; ++it) {
+    for (int j = t; j < N; j += half) b[j] = is[j] * circ_apply(d, a, N, j);
     __syncthreads();
-    for (int i = threadIdx.x; i < N; i += blockDim.x) a[i] = X[(long long)k * xs + comp * N + i];
-    for (int it = 0; it < 4; ++it) {
-      __syncthreads();
-      for (int j = threadIdx.x; j < N; j += blockDim.x) b[j] = is[j] * circ_apply(d, a, N, j);
-      __syncthreads();
-      for (int j = threadIdx.x; j < N; j += blockDim.x) a[j] = b[j];
-    }
+    for (int j = t; j < N; j += half) a[j] = is[j] * circ_apply(d, b, N, j);
     __syncthreads();
-    for (int j = threadIdx.x; j < N; j += blockDim.x)
-      b[j] = sig[(long long)k * ss + j] * tang[(long long)k * 2 * N + comp * N + j];
-    __syncthreads();
-    for (int j = threadIdx.x; j < N; j += blockDim.x) {
-      const double ten = is[j] * circ_apply(d, b, N, j);
-      f[(long long)k * 2 * N + comp * N + j] = -kappa * a[j] + ten;
-    }
+  }
+  for (int j = t; j < N; j += half)
+    b[j] = sig[(long long)k * ss + j] * tang[(long long)k * 2 * N + comp * N + j];
+  __syncthreads();
+  for (int j = t; j < N; j += half) {
+    const double ten = is[j] * circ_apply(d, b, N, j);
+    f[(long long)k * 2 * N + comp * N + j] = -kappa * a[j] + ten;
   }
 }
 
@@ -466,34 +468,40 @@ void launch_trac_jump(const ves_ctx* c, int nv, double kappa, const double* isa,
                       const double* X, long long xs, const double* sig, long long ss, double* f,
                       cudaStream_t s) {
   if (nv <= 0) return;
-  const int threads = c->N < 256 ? ((c->N + 31) / 32) * 32 : 256;
+  const int threads = c->N < 256 ? ((c->N + 31) / 32) * 32 : 256;  // per component
+  const size_t sh = (size_t)6 * c->N * sizeof(double);
+  if (sh > 48 * 1024) cudaFuncSetAttribute(trac_jump_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   ves_count_launch();
-  trac_jump_kernel<<<nv, threads, (size_t)4 * c->N * sizeof(double), s>>>(c->N, c->d1N, kappa, isa,
-                                                                            tang, X, xs, sig, ss, f);
+  trac_jump_kernel<<<nv, 2 * threads, sh, s>>>(c->N, c->d1N, kappa, isa, tang, X, xs, sig, ss, f);
 }
 
-// surfaceDiv (capsules.py:82-89)
-__global__ void surface_div_kernel(int N, const double* __restrict__ dstencil,
-                                   const double* __restrict__ isa, const double* __restrict__ tang,
-                                   const double* __restrict__ f, long long fs, double* __restrict__ out,
-                                   long long os) {
+// surfaceDiv (capsules.py:82-89), one half of the CTA per component
+__global__ void __launch_bounds__(512) surface_div_kernel(int N, const double* __restrict__ dstencil,
+                                                          const double* __restrict__ isa,
+                                                          const double* __restrict__ tang,
+                                                          const double* __restrict__ f, long long fs,
+                                                          double* __restrict__ out, long long os) {
   extern __shared__ double sh[];
+  const int half = blockDim.x / 2, comp = threadIdx.x >= half, t = threadIdx.x - comp * half;
   double* d = sh;
-  double* fx = d + N;
-  double* fy = fx + N;
+  double* fc = d + N + comp * N;  // this half's component
+  double* ayv = d + 3 * N;
   const int k = blockIdx.x;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    d[i] = dstencil[i];
-    fx[i] = f[(long long)k * fs + i];
-    fy[i] = f[(long long)k * fs + N + i];
-  }
+  for (int i = threadIdx.x; i < N; i += blockDim.x) d[i] = dstencil[i];
+  for (int i = t; i < N; i += half) fc[i] = f[(long long)k * fs + comp * N + i];
   __syncthreads();
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double is = isa[(long long)k * N + j];
-    const double ax = is * circ_apply(d, fx, N, j);
-    const double ay = is * circ_apply(d, fy, N, j);
-    out[(long long)k * os + j] =
-        ax * tang[(long long)k * 2 * N + j] + ay * tang[(long long)k * 2 * N + N + j];
+  const int rounds = (N + half - 1) / half;
+  for (int q = 0; q < rounds; ++q) {  // every thread takes part in the barriers
+    const int j = t + q * half;
+    double v = 0.0;
+    if (j < N) v = isa[(long long)k * N + j] * circ_apply(d, fc, N, j);
+    if (comp && j < N) ayv[j] = v;
+    __syncthreads();
+    if (!comp && j < N) {
+      const double ax = v, ay = ayv[j];
+      out[(long long)k * os + j] =
+          ax * tang[(long long)k * 2 * N + j] + ay * tang[(long long)k * 2 * N + N + j];
+    }
   }
 }
 
@@ -502,8 +510,7 @@ void launch_surface_div(const ves_ctx* c, int nv, const double* isa, const doubl
   if (nv <= 0) return;
   const int threads = c->N < 256 ? ((c->N + 31) / 32) * 32 : 256;
   ves_count_launch();
-  surface_div_kernel<<<nv, threads, (size_t)3 * c->N * sizeof(double), s>>>(c->N, c->d1N, isa, tang,
-                                                                              f, fs, out, os);
+  surface_div_kernel<<<nv, 2 * threads, (size_t)4 * c->N * sizeof(double), s>>>(c->N, c->d1N, isa, tang, f, fs, out, os);
 }
 
 // ----------------------------------------------------------------------------
