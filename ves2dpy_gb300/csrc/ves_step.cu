@@ -47,6 +47,73 @@ __global__ void __launch_bounds__(512) mgs_axpy_kernel(long long n, const double
     w[i] -= h * v[i];
 }
 
+// One Arnoldi column of a short vector in one CTA: ||w||, modified
+// Gram-Schmidt against V[0..col], ||w|| again and vn = w / ||w||, in the sums'
+// and updates' order of dot_partials_kernel, finalize_dot_kernel,
+// mgs_axpy_kernel and scale_inv_kernel (256-element blocks as a tree, then the
+// blocks as a tree), so that it gives the same bits.  Those are 2 (col + 3)
+// launches of ~4 us each with little work; here every warp keeps one block of
+// 256 elements in registers, one barrier per sum.  One SM's FP64 pipe bounds it
+// (~33 instructions of 16 cycles per warp and sum, 4 us at 16 warps), hence
+// the limit.  16 vesicles of N = 32 (6 warps): ~80 us a column -> 27.
+constexpr int kMgsSmall = 4096;
+
+__global__ void __launch_bounds__(kMgsSmall / 8) mgs_small_kernel(int n, int col, const double* __restrict__ V,
+                                                         const double* __restrict__ win, double* __restrict__ h0out,
+                                                         double* __restrict__ hout, double* __restrict__ vn, double eps) {
+  __shared__ double part[2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = warp * 256 + lane;
+  double w[8], v[8], nx[8];
+  auto load = [&](const double* src, double* x) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = i0 + 32 * k < n ? src[i0 + 32 * k] : 0.0;
+  };
+  int flip = 0;
+  if (threadIdx.x < 32) part[0][threadIdx.x] = part[1][threadIdx.x] = 0.0;  // blocks past the end
+  __syncthreads();
+  auto dot = [&](const double* a, const double* b) {
+    double x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = fma(a[k], b[k], 0.0);
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < h) x[k] += x[k + h];
+    double s = x[0];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) part[flip][warp] = s;
+    __syncthreads();
+    s = part[flip][lane];
+    flip ^= 1;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    return __shfl_sync(0xffffffffu, s, 0);
+  };
+  load(win, w);
+  load(V, nx);
+  const double h0 = sqrt(dot(w, w));
+  for (int k = 0; k <= col; ++k) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = nx[e];
+    if (k < col) load(V + (long long)(k + 1) * n, nx);
+    const double h = dot(v, w);
+    if (threadIdx.x == 0) hout[k] = h;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[e] -= h * v[e];
+  }
+  const double h1 = sqrt(dot(w, w));
+  if (threadIdx.x == 0) {
+    *h0out = h0;
+    hout[col + 1] = h1;
+  }
+  const bool brk = h1 <= eps * h0;
+  const double inv = 1.0 / h1;
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (i0 + 32 * k < n) vn[i0 + 32 * k] = brk ? w[k] : w[k] * inv;
+}
+
 // dst = src * (1/scal) unless skip(scal, ref): the "v *= 1/tmp" of SciPy
 __global__ void scale_inv_kernel(long long n, double* __restrict__ dst, const double* __restrict__ src,
                                  const double* __restrict__ scal, const double* __restrict__ ref, double eps) {
@@ -489,15 +556,20 @@ int gmres(St& S, GmresBufs& B, ves_step_result* res) {
       double* vn = B.V + (long long)(col + 1) * n;
       if ((rc = matvec(S, vc, B.t))) return rc;
       if ((rc = psolve(S, B.t, B.w))) return rc;
-      if ((rc = device_norm(S, B, B.w, h0))) return rc;
-      for (int k = 0; k <= col; ++k) {
-        launch_dot_partials(n, B.V + (long long)k * n, B.w, B.partials, S.s);
+      if (n <= kMgsSmall) {
         ves_count_launch();
-        mgs_axpy_kernel<<<g, 512, 0, S.s>>>(n, B.partials, dot_partial_blocks(), B.w, B.V + (long long)k * n, hcol + k);
+        mgs_small_kernel<<<1, 32 * (unsigned)((n + 255) / 256), 0, S.s>>>((int)n, col, B.V, B.w, h0, hcol, vn, eps);
+      } else {
+        if ((rc = device_norm(S, B, B.w, h0))) return rc;
+        for (int k = 0; k <= col; ++k) {
+          launch_dot_partials(n, B.V + (long long)k * n, B.w, B.partials, S.s);
+          ves_count_launch();
+          mgs_axpy_kernel<<<g, 512, 0, S.s>>>(n, B.partials, dot_partial_blocks(), B.w, B.V + (long long)k * n, hcol + k);
+        }
+        if ((rc = device_norm(S, B, B.w, hcol + col + 1))) return rc;
+        ves_count_launch();
+        scale_inv_kernel<<<g, 512, 0, S.s>>>(n, vn, B.w, hcol + col + 1, h0, eps);
       }
-      if ((rc = device_norm(S, B, B.w, hcol + col + 1))) return rc;
-      ves_count_launch();
-      scale_inv_kernel<<<g, 512, 0, S.s>>>(n, vn, B.w, hcol + col + 1, h0, eps);
       if ((rc = ves_launch_check("mgs"))) return rc;
       if ((rc = read_scalars(S, B, B.dsc, restart + 3))) return rc;
       for (int k = 0; k <= col + 1; ++k) H(col, k) = B.hsc[k];
