@@ -42,6 +42,8 @@
 //   full density (only without near lists: the near zone of the step, 1/N for
 //   unit length, is those 12 spacings, and its points are excluded).
 //   Sources without a contrast (visc == 1) have zero density and are skipped.
+#include <type_traits>
+
 #include "ves_internal.h"
 #include "ves_tc.cuh"
 
@@ -345,7 +347,12 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
 }
 
 // One CTA (256 threads) per source vesicle: centre, radius, weighted mean of
-// the density, FP64 moments of the mean-free density, stored in FP32.
+// the density, FP64 moments of the mean-free density, stored in FP32.  Bound
+// by the FP64 pipe (~18 instructions per order and point): what all orders
+// need of a point is worked out once, 256 points at a time, and left in shared
+// memory for the warps, which take the orders in turn (301 vesicles, ns = 512:
+// 293 -> 186 us).
+constexpr int kPrepBytes = 12 * 256 * 16;
 __global__ void __launch_bounds__(256) dl_mp_prep_kernel(int ns, const double* __restrict__ X,
                                                          const double* __restrict__ tang,
                                                          const double* __restrict__ den,
@@ -417,34 +424,56 @@ __global__ void __launch_bounds__(256) dl_mp_prep_kernel(int ns, const double* _
   // moments: warp w takes orders k = w, w + 8, ... (<= kDLPMax); lanes split the points
   const int warp = t >> 5, lane = t & 31;
   constexpr int kPer = (kDLPMax + 8) / 8;
+  const bool all = warp + 8 * (kPer - 1) <= kDLPMax;  // else the last order is past the highest one
   double2 C[kPer], E[kPer], G[kPer];
 #pragma unroll
   for (int q = 0; q < kPer; ++q) C[q] = E[q] = G[q] = make_double2(0.0, 0.0);
   const double iR = 1.0 / R;
-  for (int j = lane; j < ns; j += 32) {
-    const double2 v = make_double2((x[j] - ccx) * iR, (x[ns + j] - ccy) * iR);
-    const double w = js[j] * wscale;
-    const double2 dj = make_double2(d[j] - fbx * w, d[ns + j] - fby * w);  // mean-free density
-    const double2 nj = make_double2(tg[ns + j], -tg[j]);                     // n = (ty, -tx)
-    const double2 cj = zmul(nj, dj);
-    const double ej = 2.0 * (nj.x * dj.x + nj.y * dj.y);                     // 2 Re(conj(n) d)
-    const double2 cvb = zmul(cj, make_double2(v.x, -v.y));                   // c conj(v)
-    double2 pw = make_double2(1.0, 0.0), v8 = v;
-    for (int e = 0; e < warp; ++e) pw = zmul(pw, v);
-    v8 = zmul(v8, v8);
-    v8 = zmul(v8, v8);
-    v8 = zmul(v8, v8);
+  extern __shared__ __align__(16) double2 prep_pt[];  // per point: v^0..v^7, v^8, c, c conj(v), (2 Re(conj(n) d), 0)
+  double2 (*pt)[256] = reinterpret_cast<double2(*)[256]>(prep_pt);
+  for (int j0 = 0; j0 < ns; j0 += 256) {
+    const int jt = j0 + t;
+    __syncthreads();
+    if (jt < ns) {  // what the orders share, once per point
+      const double2 v = make_double2((x[jt] - ccx) * iR, (x[ns + jt] - ccy) * iR);
+      const double w = js[jt] * wscale;
+      const double2 dj = make_double2(d[jt] - fbx * w, d[ns + jt] - fby * w);  // mean-free density
+      const double2 nj = make_double2(tg[ns + jt], -tg[jt]);                   // n = (ty, -tx)
+      const double2 cj = zmul(nj, dj);
+      const double ej = 2.0 * (nj.x * dj.x + nj.y * dj.y);                     // 2 Re(conj(n) d)
+      double2 pw = make_double2(1.0, 0.0), v8 = v;
+      pt[0][t] = pw;
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const double2 a = zmul(cj, pw);
-      const double2 g = zmul(cvb, pw);
-      C[q].x += a.x;
-      C[q].y += a.y;
-      E[q].x += ej * pw.x;
-      E[q].y += ej * pw.y;
-      G[q].x += g.x;
-      G[q].y += g.y;
-      pw = zmul(pw, v8);
+      for (int e = 1; e < 8; ++e) {
+        pw = zmul(pw, v);
+        pt[e][t] = pw;
+      }
+      v8 = zmul(v8, v8);
+      v8 = zmul(v8, v8);
+      pt[8][t] = zmul(v8, v8);
+      pt[9][t] = cj;
+      pt[10][t] = zmul(cj, make_double2(v.x, -v.y));
+      pt[11][t] = make_double2(ej, 0.0);
+    }
+    __syncthreads();
+    for (int j = lane; j < min(256, ns - j0); j += 32) {
+      double2 pw = pt[warp][j];
+      const double2 v8 = pt[8][j], cj = pt[9][j], cvb = pt[10][j];
+      const double ej = pt[11][j].x;
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        if (q + 1 < kPer || all) {
+          const double2 a = zmul(cj, pw);
+          const double2 g = zmul(cvb, pw);
+          C[q].x += a.x;
+          C[q].y += a.y;
+          E[q].x += ej * pw.x;
+          E[q].y += ej * pw.y;
+          G[q].x += g.x;
+          G[q].y += g.y;
+          pw = zmul(pw, v8);
+        }
+      }
     }
   }
 #pragma unroll
@@ -549,20 +578,45 @@ struct __align__(16) DLPair {
 // and place on the near list.  S warps share a unit when there are few: they
 // take the sources of a stage in turn and leave the contributions in shared
 // memory, where the unit's first warp adds them in source order, so the sum
-// does not depend on S.  Latency-bound at small sizes: a close pair is a chain
-// of ns terms per point, and a column's warps ran all of a column's pairs one
-// after the other (301 x N = 64: 1.54 ms, now 1.15).
+// does not depend on S.  What bounds it are the close pairs, a chain of ns
+// terms per point each: their FP32 divisions overlap eight at a time
+// (rcp_normal), and the points that need FP64 share a warp's lanes.  301
+// vesicles of N = 64, ns = 512, with contrast: 1.15 ms -> 0.33 ms per launch,
+// the same bits (FP64 shared out 0.69, branch-free reciprocal 0.41, four close
+// points at a time instead of eight, which leaves room for a fourth CTA, 0.33).
+// 1 / x, correctly rounded, for kRcpMin <= x <= kRcpMax: the hardware's
+// approximation (within an ulp) and one residual step in FMA (P. Markstein,
+// IBM J. Res. Dev. 34(1), 1990).  The general division has a branch of its own
+// for each call, so several of them do not overlap.
+constexpr float kRcpMin = 1e-30f, kRcpMax = 1e30f;
+__device__ __forceinline__ float rcp_normal(float x) {
+  const float r = mufu_rcp(x);
+  return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+constexpr int kNear = 4;    // close points of a pair summed together
+constexpr int kDLRow = 33;  // doubles per row of their terms: rows start on different banks
+
 template <int WARPS, int S>
-__global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eval_kernel(DLMPArgs p) {
+struct DLShared {
+  static constexpr int kUnits = WARPS / S;
+  DLMom mom[2][kDLStage * (kDLPMax + 1)];
+  DLSrc src[2][kDLStage];
+  DLPair pairs[WARPS][kDLStage];
+  float4 dA[WARPS][32];
+  float2 dB[WARPS][32];
+  double tar[WARPS][2][32];              // the unit's points
+  double near[WARPS][kNear][3][kDLRow];  // terms of close points: factor, dx, dy
+  double2 part[S > 1 ? 2 : 1][S > 1 ? kUnits : 1][S > 1 ? kDLStage : 1][32];
+  uint64_t bar[2];
+  int turn[2][kUnits];
+};
+
+template <int WARPS, int S>
+__global__ void __launch_bounds__(WARPS * 32, S == 1 ? 4 : 16 / WARPS) dl_mp_eval_kernel(DLMPArgs p) {
   constexpr int kUnits = WARPS / S;
-  __shared__ __align__(128) DLMom smom[2][kDLStage * (kDLPMax + 1)];
-  __shared__ __align__(16) DLSrc ssrc[2][kDLStage];
-  __shared__ DLPair pairs[WARPS][kDLStage];
-  __shared__ float4 dA[WARPS][32];
-  __shared__ float2 dB[WARPS][32];
-  __shared__ double2 part[S > 1 ? 2 : 1][S > 1 ? kUnits : 1][S > 1 ? kDLStage : 1][32];
-  __shared__ int turn[2][kUnits];
-  __shared__ uint64_t bar[2];
+  extern __shared__ __align__(128) unsigned char dl_sm[];
+  DLShared<WARPS, S>& sh = *reinterpret_cast<DLShared<WARPS, S>*>(dl_sm);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = warp / S, sub = warp % S;
   const int upc = (p.ntp + 31) / 32;
@@ -576,6 +630,8 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
   const float2 thi = p.thi[col], tlo = p.tlo[col];
   const double txa = valid ? p.Xtar[(long long)col * 2 * p.ntp + i] : 0.0;
   const double tya = valid ? p.Xtar[(long long)col * 2 * p.ntp + p.ntp + i] : 0.0;
+  sh.tar[warp][0][lane] = txa;
+  sh.tar[warp][1][lane] = tya;
   float RT = 0.f;
   for (int k = lane; k < p.ntp; k += 32) {
     const float2 t = tl_col[k];
@@ -584,12 +640,12 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
   for (int o = 16; o > 0; o >>= 1) RT = fmaxf(RT, __shfl_xor_sync(0xffffffffu, RT, o));
   RT *= 1.0f + 1e-6f;
   if (threadIdx.x == 0) {
-    tc_mbar_init(&bar[0], 1);
-    tc_mbar_init(&bar[1], 1);
+    tc_mbar_init(&sh.bar[0], 1);
+    tc_mbar_init(&sh.bar[1], 1);
     tc_mbar_fence_init();
     tc_fence_async_smem();
   }
-  if (threadIdx.x < 2 * kUnits) turn[threadIdx.x / kUnits][threadIdx.x % kUnits] = 0;
+  if (threadIdx.x < 2 * kUnits) sh.turn[threadIdx.x / kUnits][threadIdx.x % kUnits] = 0;
   __syncthreads();
   const int self = p.self_idx ? p.self_idx[col] : -1;
   const int cend = p.cand_count ? min(p.cand_count[col], p.maxc) : 0;
@@ -597,19 +653,19 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
   const int nstages = (p.nsrc + kDLStage - 1) / kDLStage;
   auto fetch = [&](int st) {  // thread 0
     const int s0 = st * kDLStage, n = min(kDLStage, p.nsrc - s0), buf = st & 1;
-    tc_expect_tx(&bar[buf], (uint32_t)(n * ((kDLPMax + 1) * sizeof(DLMom) + sizeof(DLSrc))));
-    tc_bulk_g2s(smom[buf], p.mom + (long long)s0 * (kDLPMax + 1), (uint32_t)(n * (kDLPMax + 1) * sizeof(DLMom)),
-                &bar[buf]);
-    tc_bulk_g2s(ssrc[buf], p.src + s0, (uint32_t)(n * sizeof(DLSrc)), &bar[buf]);
+    tc_expect_tx(&sh.bar[buf], (uint32_t)(n * ((kDLPMax + 1) * sizeof(DLMom) + sizeof(DLSrc))));
+    tc_bulk_g2s(sh.mom[buf], p.mom + (long long)s0 * (kDLPMax + 1), (uint32_t)(n * (kDLPMax + 1) * sizeof(DLMom)),
+                &sh.bar[buf]);
+    tc_bulk_g2s(sh.src[buf], p.src + s0, (uint32_t)(n * sizeof(DLSrc)), &sh.bar[buf]);
   };
   if (threadIdx.x == 0)
     for (int st = 0; st < 2 && st < nstages; ++st) fetch(st);
   double ax = 0.0, ay = 0.0;  // pi * u
   for (int st = 0; st < nstages; ++st) {
     const int buf = st & 1, s0 = st * kDLStage, n = min(kDLStage, p.nsrc - s0);
-    bool failed = !tc_mbar_wait(&bar[buf], (st >> 1) & 1, p.st, 31);
+    bool failed = !tc_mbar_wait(&sh.bar[buf], (st >> 1) & 1, p.st, 31);
     if (lane < n) {
-      const DLSrc Sq = ssrc[buf][lane];
+      const DLSrc Sq = sh.src[buf][lane];
       const int s = s0 + lane;
       int lo = 0, hi = cend;  // first candidate >= s
       while (lo < hi) {
@@ -628,21 +684,21 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
         code = dl_order(rp);
       else
         code = cand ? -2 - lo : -1;
-      pairs[warp][lane] = DLPair{ox, oy, code, 0};
+      sh.pairs[warp][lane] = DLPair{ox, oy, code, 0};
     }
     __syncwarp();
     for (int qs = 0;; ++qs) {
       if (S > 1) {  // the unit's warps take the stage's sources in turn
-        if (lane == 0) qs = atomicAdd(&turn[buf][unit], 1);
+        if (lane == 0) qs = atomicAdd(&sh.turn[buf][unit], 1);
         qs = __shfl_sync(0xffffffffu, qs, 0);
       }
       if (qs >= n || !live) break;
-      const DLPair pr = pairs[warp][qs];
-      const DLSrc& Sq = ssrc[buf][qs];
+      const DLPair pr = sh.pairs[warp][qs];
+      const DLSrc& Sq = sh.src[buf][qs];
       double vx = 0.0, vy = 0.0;
       if (pr.code > 0) {
         const int P = pr.code;
-        const DLMom* mq = smom[buf] + qs * (kDLPMax + 1);
+        const DLMom* mq = sh.mom[buf] + qs * (kDLPMax + 1);
         const float wx = tl.x + pr.ox, wy = tl.y + pr.oy;  // omega
         const float om2 = fmaf(wx, wx, wy * wy);
         const float iom2 = 1.0f / om2;
@@ -699,47 +755,102 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
         }
         for (int j0 = 0; j0 < p.ns; j0 += 32) {
           __syncwarp();
-          dA[warp][lane] = na;
-          dB[warp][lane] = nb;
+          sh.dA[warp][lane] = na;
+          sh.dB[warp][lane] = nb;
           __syncwarp();
           if (j0 + 32 + lane < p.ns) {
             na = A4[j0 + 32 + lane];
             nb = B2[j0 + 32 + lane];
           }
           const int nj = min(32, p.ns - j0);
-#pragma unroll 4
-          for (int j = 0; j < nj; ++j) {
-            const float4 a = dA[warp][j];
-            const float2 b = dB[warp][j];
-            const float dx = tx - a.x, dy = ty - a.y;
-            const float d2 = fmaf(dx, dx, dy * dy);
-            dmin = fminf(dmin, d2);
-            const float inv = 1.0f / d2;
-            const float c = fmaf(dx, a.z, dy * a.w) * fmaf(dx, b.x, dy * b.y) * (inv * inv);
-            bx = fmaf(c, dx, bx);
-            by = fmaf(c, dy, by);
-          }
+          auto terms = [&](int j, auto count) {  // count terms from j on; their divisions overlap
+            constexpr int n = decltype(count)::value;
+            float4 a[n];
+            float2 b[n];
+            float dx[n], dy[n], d2[n], inv[n], lo = 3.0e38f, hi = 0.f;
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+              a[q] = sh.dA[warp][j + q];
+              b[q] = sh.dB[warp][j + q];
+              dx[q] = tx - a[q].x;
+              dy[q] = ty - a[q].y;
+              d2[q] = fmaf(dx[q], dx[q], dy[q] * dy[q]);
+              lo = fminf(lo, d2[q]);
+              hi = fmaxf(hi, d2[q]);
+            }
+            dmin = fminf(dmin, lo);
+            if (lo >= kRcpMin && hi <= kRcpMax) {
+#pragma unroll
+              for (int q = 0; q < n; ++q) inv[q] = rcp_normal(d2[q]);
+            } else {
+              for (int q = 0; q < n; ++q) inv[q] = 1.0f / d2[q];
+            }
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+              const float c =
+                  fmaf(dx[q], a[q].z, dy[q] * a[q].w) * fmaf(dx[q], b[q].x, dy[q] * b[q].y) * (inv[q] * inv[q]);
+              bx = fmaf(c, dx[q], bx);
+              by = fmaf(c, dy[q], by);
+            }
+          };
+          int j = 0;
+          for (; j + 8 <= nj; j += 8) terms(j, std::integral_constant<int, 8>());
+          for (; j < nj; ++j) terms(j, std::integral_constant<int, 1>());
         }
-        if (!excl) {
-          if (dmin >= Sq.thr2) {
-            vx = (double)bx;
-            vy = (double)by;
-          } else {  // within 12 spacings: the full density in FP64
-            const double* xs = p.Xsrc + (long long)s * 2 * p.ns;
-            const double* ts = p.tang + (long long)s * 2 * p.ns;
-            const double* ds = p.den + (long long)s * 2 * p.ns;
-            for (int j = 0; j < p.ns; ++j) {
-              const double dx = txa - xs[j], dy = tya - xs[p.ns + j];
-              const double d2 = dx * dx + dy * dy;
-              const double c = ((dx * ts[p.ns + j] - dy * ts[j]) / (d2 * d2)) * (dx * ds[j] + dy * ds[p.ns + j]);
-              vx = fma(c, dx, vx);
-              vy = fma(c, dy, vy);
+        const bool close = !excl && !(dmin >= Sq.thr2);
+        if (!excl && !close) {
+          vx = (double)bx;
+          vy = (double)by;
+        }
+        // Points within 12 spacings: the full density in FP64.  A term takes ~20
+        // FP64 instructions, the pipe 16 cycles for each however many lanes
+        // are on, and few lanes of a warp are that close.  So the lanes share
+        // out 32 terms of one point at a time, and then 2 kNear of them add
+        // the terms of kNear points in order, one coordinate each.
+        unsigned todo = __ballot_sync(0xffffffffu, close);
+        while (todo) {
+          const double* xs = p.Xsrc + (long long)s * 2 * p.ns;
+          const double* ts = p.tang + (long long)s * 2 * p.ns;
+          const double* ds = p.den + (long long)s * 2 * p.ns;
+          double (*nt)[3][kDLRow] = sh.near[warp];
+          const unsigned batch = todo;
+          double acc = 0.0;
+          for (int j0 = 0; j0 < p.ns; j0 += 32) {
+            const int j = j0 + lane;
+            __syncwarp();
+            if (j < p.ns) {
+              const double sx = xs[j], sy = xs[p.ns + j], tx2 = ts[j], ty2 = ts[p.ns + j];
+              const double gx = ds[j], gy = ds[p.ns + j];
+              unsigned left = batch;
+              for (int k = 0; k < kNear && left; ++k, left &= left - 1) {
+                const int l = __ffs(left) - 1;
+                const double dx = sh.tar[warp][0][l] - sx, dy = sh.tar[warp][1][l] - sy;
+                const double d2 = dx * dx + dy * dy;
+                const double c = ((dx * ty2 - dy * tx2) / (d2 * d2)) * (dx * gx + dy * gy);
+                nt[k][0][lane] = c;
+                nt[k][1][lane] = dx;
+                nt[k][2][lane] = dy;
+              }
+            }
+            __syncwarp();
+            const double* tc = nt[lane % kNear][0];
+            const double* td = nt[lane % kNear][1 + (lane / kNear & 1)];
+            const int nj = min(32, p.ns - j0);
+            if (lane < 2 * kNear)
+              for (int q = 0; q < nj; ++q) acc = fma(tc[q], td[q], acc);
+          }
+          __syncwarp();
+          for (int k = 0; k < kNear && todo; ++k, todo &= todo - 1) {
+            const double rx = __shfl_sync(0xffffffffu, acc, k), ry = __shfl_sync(0xffffffffu, acc, kNear + k);
+            if (lane == __ffs(todo) - 1) {
+              vx = rx;
+              vy = ry;
             }
           }
         }
       }
       if (S > 1) {
-        part[buf][unit][qs][lane] = make_double2(vx, vy);
+        sh.part[buf][unit][qs][lane] = make_double2(vx, vy);
       } else {  // points past the column's end add too; they are not stored
         ax += vx;
         ay += vy;
@@ -748,17 +859,17 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
     // nobody reads this stage any more (and every contribution is in)
     failed = __syncthreads_or(failed ? 1 : 0) != 0;
     if (S > 1) {
-      if (threadIdx.x < kUnits) turn[buf][threadIdx.x] = 0;
+      if (threadIdx.x < kUnits) sh.turn[buf][threadIdx.x] = 0;
       if (sub == 0)
         for (int qs = 0; qs < n; ++qs) {
-          ax += part[buf][unit][qs][lane].x;
-          ay += part[buf][unit][qs][lane].y;
+          ax += sh.part[buf][unit][qs][lane].x;
+          ay += sh.part[buf][unit][qs][lane].y;
         }
     }
     if (failed) {  // the copies in flight land before the CTA ends
       if (threadIdx.x == 0) {
-        tc_mbar_wait(&bar[buf], (st >> 1) & 1, nullptr, 0);
-        if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((st + 1) >> 1) & 1, nullptr, 0);
+        tc_mbar_wait(&sh.bar[buf], (st >> 1) & 1, nullptr, 0);
+        if (st + 1 < nstages) tc_mbar_wait(&sh.bar[buf ^ 1], ((st + 1) >> 1) & 1, nullptr, 0);
       }
       break;
     }
@@ -771,6 +882,19 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) dl_mp_eva
     p.out[(long long)col * 2 * p.ntp + i] = ax / VES_PI;
     p.out[(long long)col * 2 * p.ntp + p.ntp + i] = ay / VES_PI;
   }
+}
+
+template <int WARPS, int S>
+int dl_mp_start(const DLMPArgs& a, long long grid, cudaStream_t s) {
+  constexpr int bytes = (int)sizeof(DLShared<WARPS, S>);
+  if (bytes > 48 * 1024) {
+    const int rc = ves_cuda_status(
+        cudaFuncSetAttribute(dl_mp_eval_kernel<WARPS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
+        "farfield_dl smem attribute");
+    if (rc) return rc;
+  }
+  dl_mp_eval_kernel<WARPS, S><<<(unsigned)grid, WARPS * 32, bytes, s>>>(a);
+  return ves_launch_check("farfield_dl multipole");
 }
 
 }  // namespace
@@ -810,8 +934,12 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
     ves_record_error(VES_ERR_SHAPE, "farfield_dl: %d source points per vesicle exceed the multipole path", ns);
     return VES_ERR_SHAPE;
   }
+  const int rc = ves_cuda_status(
+      cudaFuncSetAttribute(dl_mp_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepBytes),
+      "farfield_dl smem attribute");
+  if (rc) return rc;
   ves_count_launch(3);
-  dl_mp_prep_kernel<<<nsrc, 256, 0, s>>>(ns, Xsrc, tang, den, sa, visc, src, mom, recA, recB);
+  dl_mp_prep_kernel<<<nsrc, 256, kPrepBytes, s>>>(ns, Xsrc, tang, den, sa, visc, src, mom, recA, recB);
   dl_mp_targets_kernel<<<nt, 256, 0, s>>>(ntp, Xtar, tloc, thi, tlo);
   DLMPArgs a;
   a.nsrc = nsrc;
@@ -840,13 +968,9 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
   // one warp per 32 points from nine such units per SM on, four from two per
   // SM, eight below (the single layer's rule, the same pattern of work)
   const long long units = (long long)nt * ((ntp + 31) / 32);
-  if (units >= 152 * 9)
-    dl_mp_eval_kernel<4, 1><<<(unsigned)((units + 3) / 4), 128, 0, s>>>(a);
-  else if (units >= 152 * 2)
-    dl_mp_eval_kernel<4, 4><<<(unsigned)units, 128, 0, s>>>(a);
-  else
-    dl_mp_eval_kernel<8, 8><<<(unsigned)units, 256, 0, s>>>(a);
-  return ves_launch_check("farfield_dl multipole");
+  if (units >= 152 * 9) return dl_mp_start<4, 1>(a, (units + 3) / 4, s);
+  if (units >= 152 * 2) return dl_mp_start<4, 4>(a, units, s);
+  return dl_mp_start<8, 8>(a, units, s);
 }
 
 int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const double* tang, const double* den,
