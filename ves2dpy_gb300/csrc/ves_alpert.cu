@@ -21,6 +21,16 @@ __device__ __forceinline__ float tlog<float>(float x) { return logf(x); }
 template <>
 __device__ __forceinline__ double tlog<double>(double x) { return log(x); }
 
+// FP64 -> T, and 1 / x for the kernel's regularised square distances
+template <typename T>
+__device__ __forceinline__ T to(double x);
+template <>
+__device__ __forceinline__ float to<float>(double x) { return narrow(x); }
+template <>
+__device__ __forceinline__ double to<double>(double x) { return x; }
+__device__ __forceinline__ float inverse(float x) { return x >= kRcpMin && x <= kRcpMax ? rcp_normal(x) : 1.0f / x; }
+__device__ __forceinline__ double inverse(double x) { return 1.0 / x; }
+
 // Kernel A: per (vesicle, target s) the 14 off-grid node field values.
 template <typename T>
 __global__ void alpert_dense_nodes_kernel(int N, int Nup, int m, int nquad, const double* __restrict__ X,
@@ -60,63 +70,90 @@ __global__ void alpert_dense_nodes_kernel(int N, int Nup, int m, int nquad, cons
 }
 
 // Kernel B: rows of Gup (three fields G11, G12, G22) for ROWS targets per CTA.
-template <typename T, int ROWS>
-__global__ void __launch_bounds__(256) alpert_rows_kernel(int Nup, int nquad, const double* __restrict__ Xup,
-                                                          const double* __restrict__ sa_up,
-                                                          const T* __restrict__ adense,
-                                                          const double* __restrict__ qw,
-                                                          const T* __restrict__ Fd, T* __restrict__ Gup,
-                                                          int k0) {
-  __shared__ T fd[ROWS][56];
+// In FP32 an entry is 28 packed multiply-adds, a logarithm, a reciprocal and two
+// FP64 differences; those, 32 cycles of the FP64 pipe per warp, bound it from
+// below (0.57 ms for 73 vesicles of Nup = 1536), instruction issue does now.
+// The conversions to FP32 took 48 cycles more there, so they are done in
+// integers, the jacobian's once per CTA, and the division is branch-free: 1.55
+// -> 1.14 ms.  One column per thread and one row at a time, 36 warps per SM: two
+// or three columns or eight rows in flight need registers that cost more warps
+// than they save loads (1.25 .. 1.8 ms).
+template <typename T, int ROWS, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) alpert_rows_kernel(int Nup, int nquad,
+                                                                    const double* __restrict__ Xup,
+                                                                    const double* __restrict__ sa_up,
+                                                                    const T* __restrict__ adense,
+                                                                    const double* __restrict__ qw,
+                                                                    const T* __restrict__ Fd, T* __restrict__ Gup,
+                                                                    int k0) {
+  __shared__ __align__(16) T fd[ROWS][56];
   __shared__ double txs[ROWS], tys[ROWS];
+  extern __shared__ float saf[];    // [Nup], FP32 only
   const int kl = blockIdx.y;        // vesicle within chunk
   const int k = k0 + kl;            // global vesicle
   const int s0 = blockIdx.x * ROWS;
-  for (int idx = threadIdx.x; idx < ROWS * 56; idx += blockDim.x) {
+  const double* xk = Xup + (long long)k * 2 * Nup;
+  const double* sak = sa_up + (long long)k * Nup;
+  for (int idx = threadIdx.x; idx < ROWS * 56; idx += THREADS) {
     const int r = idx / 56, e = idx % 56;
     fd[r][e] = (s0 + r < Nup) ? Fd[((long long)k * Nup + s0 + r) * 56 + e] : T(0);
   }
   if (threadIdx.x < ROWS) {
-    const int s = min(s0 + threadIdx.x, Nup - 1);
-    txs[threadIdx.x] = Xup[(long long)k * 2 * Nup + s];
-    tys[threadIdx.x] = Xup[(long long)k * 2 * Nup + Nup + s];
+    const int s = min(s0 + (int)threadIdx.x, Nup - 1);
+    txs[threadIdx.x] = xk[s];
+    tys[threadIdx.x] = xk[Nup + s];
   }
+  if (sizeof(T) == 4)
+    for (int i = threadIdx.x; i < Nup; i += THREADS) saf[i] = narrow(sak[i]);
   __syncthreads();
   const T wg = (T)qw[7];  // on-grid weight h/(4 pi)
-  const double* xk = Xup + (long long)k * 2 * Nup;
-  const double* sak = sa_up + (long long)k * Nup;
   const long long NN = (long long)Nup * Nup;
   T* G11 = Gup + (long long)kl * 3 * NN;
   T* G12 = G11 + NN;
   T* G22 = G12 + NN;
-  for (int i = threadIdx.x; i < Nup; i += blockDim.x) {
+  for (int i = threadIdx.x; i < Nup; i += THREADS) {
     T a[14];
 #pragma unroll
     for (int q = 0; q < 14; ++q) a[q] = adense[(long long)q * Nup + i];
     const bool grid = (i >= 5 && i <= Nup - 5);
-#pragma unroll
+#pragma unroll(sizeof(T) == 4 ? 1 : ROWS)
     for (int r = 0; r < ROWS; ++r) {
       const int s = s0 + r;
       if (s >= Nup) break;
       T wl = 0, wxx = 0, wxy = 0, wyy = 0;
+      if constexpr (sizeof(T) == 4) {
+        float2 w0 = make_float2(0.f, 0.f), w1 = w0;
 #pragma unroll
-      for (int q = 0; q < 14; ++q) {
-        wl += a[q] * fd[r][q * 4 + 0];
-        wxx += a[q] * fd[r][q * 4 + 1];
-        wxy += a[q] * fd[r][q * 4 + 2];
-        wyy += a[q] * fd[r][q * 4 + 3];
+        for (int q = 0; q < 14; ++q) {
+          const float4 f = *reinterpret_cast<const float4*>(&fd[r][q * 4]);
+          const float2 aa = make_float2(a[q], a[q]);
+          w0 = __ffma2_rn(aa, make_float2(f.x, f.y), w0);
+          w1 = __ffma2_rn(aa, make_float2(f.z, f.w), w1);
+        }
+        wl = w0.x;
+        wxx = w0.y;
+        wxy = w1.x;
+        wyy = w1.y;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 14; ++q) {
+          wl += a[q] * fd[r][q * 4 + 0];
+          wxx += a[q] * fd[r][q * 4 + 1];
+          wxy += a[q] * fd[r][q * 4 + 2];
+          wyy += a[q] * fd[r][q * 4 + 3];
+        }
       }
       int col = s + i;
       if (col >= Nup) col -= Nup;
       if (grid) {
-        const T dx = (T)(txs[r] - xk[col]), dy = (T)(tys[r] - xk[Nup + col]);
-        const T rho = T(1) / (dx * dx + dy * dy + T(1e-7));
+        const T dx = to<T>(txs[r] - xk[col]), dy = to<T>(tys[r] - xk[Nup + col]);
+        const T rho = inverse(dx * dx + dy * dy + T(1e-7));
         wl += T(0.5) * wg * tlog<T>(rho);
         wxx += wg * dx * dx * rho;
         wxy += wg * dx * dy * rho;
         wyy += wg * dy * dy * rho;
       }
-      const T sa = (T)sak[col];
+      const T sa = sizeof(T) == 4 ? (T)saf[col] : (T)sak[col];
       const long long o = (long long)s * Nup + col;
       G11[o] = (wl + wxx) * sa;
       G12[o] = wxy * sa;
@@ -327,7 +364,11 @@ static int alpert_impl(ves_ctx* c, int nv, const double* X, double* G, WsCarver&
     const int nk = min(chunk, nv - k0);
     dim3 grid(ceil_div(Nup, ROWS), nk);
     ves_count_launch();
-    alpert_rows_kernel<T, ROWS><<<grid, 256, 0, s>>>(Nup, c->nquad, Xup, sa_up, adense, c->qw, Fd, Gup, k0);
+    if (sizeof(T) == 4)
+      alpert_rows_kernel<T, ROWS, 128, 9>
+          <<<grid, 128, Nup * sizeof(float), s>>>(Nup, c->nquad, Xup, sa_up, adense, c->qw, Fd, Gup, k0);
+    else
+      alpert_rows_kernel<T, ROWS, 256, 1><<<grid, 256, 0, s>>>(Nup, c->nquad, Xup, sa_up, adense, c->qw, Fd, Gup, k0);
     const long long NN = (long long)Nup * Nup;
     // T = Gup * P for the 3*nk fields; Gf = R * T
     const int pairs = sizeof(T) == 8 ? interp_pairs(N, Nup) : 0;

@@ -406,18 +406,6 @@ int launch_lu_factor_f32(ves_ctx* c, int nv, int n, float* A, int* piv, cudaStre
   return lu_factor_t<float>(c, nv, n, A, piv, s);
 }
 
-// FP32 -> FP64 by moving the bits (exact, as the conversion is).  The
-// conversion instruction runs on the FP64 pipe (2 lanes/clk/SM); these are
-// integer operations, 32 times that rate.
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t b = __float_as_uint(x), e = b & 0x7f800000u;
-  if (e == 0x7f800000u || (e == 0u && (b << 1) != 0u)) return (double)x;  // infinite, NaN or subnormal
-  const bool z = (b << 1) == 0u;
-  const uint32_t hi = z ? b : (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u);
-  return __hiloint2double((int)hi, (int)(z ? 0u : b << 29));
-}
-__device__ __forceinline__ double widen(double x) { return x; }
-
 // exponent between -895 and 896: no intermediate result of the correction is subnormal
 __device__ __forceinline__ bool mid_range(double z) {
   return (((uint32_t)__double2hiint(z) >> 20) & 0x7ffu) - 128u < 1792u;
@@ -433,7 +421,7 @@ __device__ __forceinline__ bool mid_range(double z) {
 // reciprocal, taken for the whole block at once, and Markstein's correction
 // (two multiply-adds, correctly rounded when the reciprocal is; IBM J. Res.
 // Dev. 34, 1990).  The row exchanges walk the pivots in shared memory.  One
-// solve: 1024 blocks of 384 rows in FP32 1.22 -> 0.92 ms, 301 of 192 in FP64
+// solve: 1024 blocks of 384 rows in FP32 1.22 -> 0.71 ms, 301 of 192 in FP64
 // 0.21 -> 0.11, 16 of 96 0.075 -> 0.040.
 template <typename T>
 __global__ void __launch_bounds__(256) lu_solve_kernel(int n, const T* __restrict__ LU,

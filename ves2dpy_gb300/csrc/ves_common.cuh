@@ -54,6 +54,52 @@ __device__ __forceinline__ float mufu_lg2(float x) {
   return r;
 }
 
+// 1 / x, correctly rounded, for kRcpMin <= x <= kRcpMax: the hardware's
+// approximation (within an ulp) and one residual step in FMA (P. Markstein,
+// IBM J. Res. Dev. 34(1), 1990).  The general division has a branch of its own
+// for each call, so several of them do not overlap.
+constexpr float kRcpMin = 1e-30f, kRcpMax = 1e30f;
+__device__ __forceinline__ float rcp_normal(float x) {
+  const float r = mufu_rcp(x);
+  return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+// FP64 -> FP32 (to nearest even) and FP32 -> FP64 by integer operations, for
+// every value with the result of the conversion.  The conversion instructions
+// run on the FP64 pipe (2 lanes per clock and SM, a warp's instruction counts
+// even when a predicate turns it off), integer operations at 32 times that.
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned hi = (unsigned)(b >> 32), e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
+  if (e - 897u <= 253u) {  // normal; the carry of 2^128 - ulp is infinity
+    const unsigned long long t = b + 0x0fffffffull + ((b >> 29) & 1);
+    return __uint_as_float(((unsigned)(t >> 29) - 0xC0000000u) | sign);
+  }
+  if (e > 1150u) return __uint_as_float(e == 0x7ffu && (b << 12) != 0 ? 0x7fffffffu : sign | 0x7f800000u);
+  const int sh = e > 871u ? 926 - (int)e : 55;  // subnormal: units of 2^-149
+  const unsigned long long m = (b & 0xfffffffffffffull) | (1ull << 52), q = m >> sh, rem = m - (q << sh);
+  const unsigned long long half = 1ull << (sh - 1);
+  return __uint_as_float(sign | ((unsigned)q + (rem > half || (rem == half && (q & 1)) ? 1u : 0u)));
+}
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), a = b & 0x7fffffffu, e = a >> 23;
+  unsigned hi = (a >> 3) + 0x38000000u, lo = b << 29;
+  if (e - 1u > 253u) {
+    if (e == 255u) {  // infinite or NaN
+      hi += 0x38000000u;
+    } else if (a == 0u) {
+      hi = lo = 0u;
+    } else {  // subnormal
+      const int s = __clz((int)a) - 8;
+      const unsigned m = (a << s) & 0x7fffffu;
+      hi = ((unsigned)(897 - s) << 20) | (m >> 3);
+      lo = m << 29;
+    }
+  }
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)lo);
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
 static inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 // Host helper: map a CUDA error to a status code, recording the message.

@@ -99,9 +99,15 @@ __global__ void __launch_bounds__(256) dl_rows_kernel(int Nup, const double* __r
         v22 = K * (dy * dy);
       }
       const long long o = (long long)a * Nup + b;
-      D11[o] = (T)v11;
-      D12[o] = (T)v12;
-      D22[o] = (T)v22;
+      if constexpr (sizeof(T) == 4) {
+        D11[o] = narrow(v11);
+        D12[o] = narrow(v12);
+        D22[o] = narrow(v22);
+      } else {
+        D11[o] = v11;
+        D12[o] = v12;
+        D22[o] = v22;
+      }
     }
   }
 }
@@ -584,16 +590,6 @@ struct __align__(16) DLPair {
 // vesicles of N = 64, ns = 512, with contrast: 1.15 ms -> 0.33 ms per launch,
 // the same bits (FP64 shared out 0.69, branch-free reciprocal 0.41, four close
 // points at a time instead of eight, which leaves room for a fourth CTA, 0.33).
-// 1 / x, correctly rounded, for kRcpMin <= x <= kRcpMax: the hardware's
-// approximation (within an ulp) and one residual step in FMA (P. Markstein,
-// IBM J. Res. Dev. 34(1), 1990).  The general division has a branch of its own
-// for each call, so several of them do not overlap.
-constexpr float kRcpMin = 1e-30f, kRcpMax = 1e30f;
-__device__ __forceinline__ float rcp_normal(float x) {
-  const float r = mufu_rcp(x);
-  return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
-
 constexpr int kNear = 4;    // close points of a pair summed together
 constexpr int kDLRow = 33;  // doubles per row of their terms: rows start on different banks
 
@@ -732,8 +728,8 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 4 : 16 / WARPS) dl_mp_eva
         // t4 = R conj(h4 / omega^2)
         const float i2r = iwr * iwr - iwi * iwi, i2i = 2.f * iwr * iwi;   // 1/omega^2
         const float t4r = Sq.R * (h4.x * i2r - h4.y * i2i), t4i = -Sq.R * (h4.x * i2i + h4.y * i2r);
-        vx = 0.25 * (double)(t1r + t2r + t3r - t4r);
-        vy = 0.25 * (double)(t1i + t2i + t3i - t4i);
+        vx = widen(0.25f * (t1r + t2r + t3r - t4r));
+        vy = widen(0.25f * (t1i + t2i + t3i - t4i));
       } else if (pr.code < 0) {
         // direct rule over the upsampled points, FP32, coordinates relative to
         // the source centre; records staged 32 at a time
@@ -799,8 +795,8 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 4 : 16 / WARPS) dl_mp_eva
         }
         const bool close = !excl && !(dmin >= Sq.thr2);
         if (!excl && !close) {
-          vx = (double)bx;
-          vy = (double)by;
+          vx = widen(bx);
+          vy = widen(by);
         }
         // Points within 12 spacings: the full density in FP64.  A term takes ~20
         // FP64 instructions, the pipe 16 cycles for each however many lanes
