@@ -246,156 +246,340 @@ void launch_bgemv_f64(int nv, int m, int n, const double* A, const double* x, lo
 // Blocked right-looking LU with partial pivoting, one CTA per matrix
 // (the factorisation torch.linalg.lu_factor performs, tstep_biem.py:350).
 // piv[j] = row exchanged with row j at step j (LAPACK ipiv, 0-based).
+//
+// Panels of 32 columns.  A thread keeps ROWS whole rows of the panel in
+// registers, so a column costs two barriers: one for the largest entry (the
+// first on ties), one for the pivot row and the row it replaces, which pass
+// through shared memory.  Eight columns are unrolled (32 make 200 KB of
+// instructions, and fetching them was the bound), then they move to shared
+// memory, where the panel lies transposed (Lt) for what follows.  The panel's row exchanges are worked out as one
+// permutation: every other column is read, permuted and, right of the panel,
+// solved against the unit triangle by one thread, and the trailing matrix is
+// updated in 32 x 32 tiles per warp, 8 x 4 entries per thread.  An entry takes
+// its multiply-adds in ascending order of the column eliminated, whatever the
+// tiles, so the factors do not depend on them.
+// FP64 is bound by its pipe (1000 matrices of 384: 19 G multiply-adds, 33 ms;
+// 46.9 -> 39.3 ms; 8192 of 96: 4.1 ms, 9.1 -> 7.0), FP32 by the latency of a
+// column (1024 of 384: 13.8 -> 3.5 ms).  The first form passed a panel through
+// shared memory at a stride of 32 for every column, swapped rows in global
+// memory with a barrier each, and divided 64-bit indices for every entry.
 constexpr int LU_NB = 32;
 
+// distance of the transposed panel's rows: 16-byte aligned, off a multiple of 16
+__host__ __device__ inline int lu_pitch(int n) {
+  const int np = (n + 3) / 4 * 4;
+  return np % 16 ? np : np + 4;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) lu_factor_kernel(int n, T* __restrict__ A, int* __restrict__ piv,
-                                                        VesDeviceStatus* st) {
+__device__ __forceinline__ void lu_ld4(const T* p, T* v) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+  } else {
+    const double2 t = reinterpret_cast<const double2*>(p)[0], u = reinterpret_cast<const double2*>(p)[1];
+    v[0] = t.x, v[1] = t.y, v[2] = u.x, v[3] = u.y;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void lu_st4(T* p, const T* v) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+    reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+    reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+  }
+}
+
+// |x| as an integer of the same order, -1 for a NaN: comparing FP64 values
+// would take the FP64 pipe
+__device__ __forceinline__ int lu_key(float x) {
+  const int b = __float_as_int(x) & 0x7fffffff;
+  return b > 0x7f800000 ? -1 : b;
+}
+__device__ __forceinline__ long long lu_key(double x) {
+  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+  return b > 0x7ff0000000000000LL ? -1 : b;
+}
+
+template <typename T, int ROWS, int NT, int CTAS>
+__global__ void __launch_bounds__(NT, CTAS) lu_factor_kernel(int n, T* __restrict__ A, int* __restrict__ piv,
+                                                             VesDeviceStatus* st) {
+  constexpr int NB = LU_NB, NW = NT / 32;
+  using Key = decltype(lu_key(T(0)));
   extern __shared__ __align__(16) unsigned char lu_sh[];
-  T* sh = (T*)lu_sh;
-  const int k = blockIdx.x;
+  const int np = lu_pitch(n);
+  T* Lt = (T*)lu_sh;        // [NB][np] the panel, transposed
+  T* U12 = Lt + NB * np;    // [NB][np] the panel's rows of the other columns
+  __shared__ __align__(16) T prow[NB], jrow[NB];
+  __shared__ Key wv[NW];
+  __shared__ T pinv;
+  __shared__ int wi[NW], lpiv[NB], top[NB], orow[NB], osrc[NB], ocnt;
+  const int k = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   T* a = A + (long long)k * n * n;
   int* pv = piv + (long long)k * n;
-  T* panel = sh;                 // [n][LU_NB]
-  T* U12 = sh + n * LU_NB;       // [LU_NB][n]
-  __shared__ double red_v[256];
-  __shared__ int red_i[256];
-  __shared__ int s_piv;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const bool vec = n % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
 
-  for (int p0 = 0; p0 < n; p0 += LU_NB) {
-    const int nb = min(LU_NB, n - p0);
-    const int rows = n - p0;
-    for (int idx = tid; idx < rows * nb; idx += nt) {
-      const int i = idx / nb, j = idx % nb;
-      panel[i * LU_NB + j] = a[(long long)(p0 + i) * n + p0 + j];
-    }
+  for (int p0 = 0; p0 < n; p0 += NB) {
+    const int nb = min(NB, n - p0), rows = n - p0;
+    for (int i = warp; i < rows; i += NW)
+      if (lane < nb) Lt[lane * np + i] = a[(long long)(p0 + i) * n + p0 + lane];
     __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-      // pivot: first index of max |panel[i][j]|, i >= j
-      double best = -1.0;
-      int bi = n;
-      for (int i = j + tid; i < rows; i += nt) {
-        const double v = fabs((double)panel[i * LU_NB + j]);
-        if (v > best) {
-          best = v;
-          bi = i;
-        }
-      }
-      red_v[tid] = best;
-      red_i[tid] = bi;
-      __syncthreads();
-      for (int w = nt / 2; w > 0; w >>= 1) {
-        if (tid < w) {
-          const double v2 = red_v[tid + w];
-          const int i2 = red_i[tid + w];
-          if (v2 > red_v[tid] || (v2 == red_v[tid] && i2 < red_i[tid])) {
-            red_v[tid] = v2;
-            red_i[tid] = i2;
+    T row[ROWS][NB];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = tid + r * NT;
+#pragma unroll
+      for (int j = 0; j < NB; ++j) row[r][j] = (i < rows && j < nb) ? Lt[j * np + i] : T(0);
+    }
+    // eight columns per pass: the registers hold columns j0 .. j0 + 31 (those
+    // past the panel are zero)
+#pragma unroll 1
+    for (int j0 = 0; j0 < nb; j0 += 8) {
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        const int j = j0 + jj;
+        if (j >= nb) break;
+        // pivot: first index of max |a_ij|, i >= j (a NaN is never the largest)
+        Key best = -1;
+        int bi = j;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const int i = tid + r * NT;
+          const Key v = lu_key(row[r][jj]);
+          if (i >= j && i < rows && v > best) {
+            best = v;
+            bi = i;
           }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+          const Key v2 = __shfl_xor_sync(0xffffffffu, best, o);
+          const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (v2 > best || (v2 == best && i2 < bi)) {
+            best = v2;
+            bi = i2;
+          }
+        }
+        if (lane == 0) {
+          wv[warp] = best;
+          wi[warp] = bi;
         }
         __syncthreads();
-      }
-      if (tid == 0) {
-        s_piv = red_i[0];
-        pv[p0 + j] = p0 + red_i[0];
-        if (red_v[0] == 0.0) ves_set_error(st, VES_ERR_SINGULAR, 1, (long long)k * n + p0 + j);
-      }
-      __syncthreads();
-      const int ip = s_piv;
-      if (ip != j) {
-        for (int jj = tid; jj < nb; jj += nt) {
-          const T t = panel[j * LU_NB + jj];
-          panel[j * LU_NB + jj] = panel[ip * LU_NB + jj];
-          panel[ip * LU_NB + jj] = t;
-        }
-      }
-      __syncthreads();
-      const T d = panel[j * LU_NB + j];
-      const T rcp = (d != T(0)) ? T(1) / d : T(0);
-      for (int i = j + 1 + tid; i < rows; i += nt) panel[i * LU_NB + j] *= rcp;
-      __syncthreads();
-      const int rem = nb - j - 1;
-      if (rem > 0) {
-        for (int idx = tid; idx < (rows - j - 1) * rem; idx += nt) {
-          const int i = j + 1 + idx / rem, jj = j + 1 + idx % rem;
-          panel[i * LU_NB + jj] = fma(-panel[i * LU_NB + j], panel[j * LU_NB + jj], panel[i * LU_NB + jj]);
-        }
-      }
-      __syncthreads();
-    }
-    // write the panel back
-    for (int idx = tid; idx < rows * nb; idx += nt) {
-      const int i = idx / nb, j = idx % nb;
-      a[(long long)(p0 + i) * n + p0 + j] = panel[i * LU_NB + j];
-    }
-    // apply this panel's row exchanges to the columns left and right of it
-    for (int j = 0; j < nb; ++j) {
-      const int r1 = p0 + j, r2 = pv[p0 + j];
-      if (r2 != r1) {
-        for (int c = tid; c < n; c += nt) {
-          if (c >= p0 && c < p0 + nb) continue;
-          const T t = a[(long long)r1 * n + c];
-          a[(long long)r1 * n + c] = a[(long long)r2 * n + c];
-          a[(long long)r2 * n + c] = t;
-        }
-      }
-      __syncthreads();
-    }
-    const int ncol = n - p0 - nb;
-    if (ncol > 0) {
-      // U12 = L11^{-1} A12 (unit lower triangular), one thread per column
-      for (int c = tid; c < ncol; c += nt) {
-        T col[LU_NB];
+        best = wv[0];
+        int ip = wi[0];
 #pragma unroll
-        for (int j = 0; j < LU_NB; ++j)
-          if (j < nb) col[j] = a[(long long)(p0 + j) * n + p0 + nb + c];
-#pragma unroll
-        for (int j = 0; j < LU_NB; ++j) {
-          if (j >= nb) break;
-          const T v = col[j];
-          for (int i = j + 1; i < nb; ++i) col[i] = fma(-panel[i * LU_NB + j], v, col[i]);
-        }
-#pragma unroll
-        for (int j = 0; j < LU_NB; ++j)
-          if (j < nb) {
-            U12[j * n + c] = col[j];
-            a[(long long)(p0 + j) * n + p0 + nb + c] = col[j];
+        for (int w = 1; w < NW; ++w) {
+          const Key v2 = wv[w];
+          const int i2 = wi[w];
+          if (v2 > best || (v2 == best && i2 < ip)) {
+            best = v2;
+            ip = i2;
           }
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const int i = tid + r * NT;
+          if (i == ip) {
+#pragma unroll
+            for (int q = 0; q < NB; q += 4) lu_st4(prow + q, &row[r][q]);
+            pinv = (row[r][jj] != T(0)) ? T(1) / row[r][jj] : T(0);
+          }
+          if (i == j && ip != j) {
+#pragma unroll
+            for (int q = 0; q < NB; q += 4) lu_st4(jrow + q, &row[r][q]);
+          }
+        }
+        if (tid == 0) {
+          lpiv[j] = ip;
+          pv[p0 + j] = p0 + ip;
+          if (best == 0) ves_set_error(st, VES_ERR_SINGULAR, 1, (long long)k * n + p0 + j);
+        }
+        __syncthreads();
+        if (ip != j && tid < j0) {  // the columns already in shared memory
+          const T t = Lt[tid * np + ip];
+          Lt[tid * np + ip] = Lt[tid * np + j];
+          Lt[tid * np + j] = t;
+        }
+        const T rcp = pinv;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const int i = tid + r * NT;
+          if (ip != j && (i == ip || i == j)) {
+            const T* from = i == ip ? jrow : prow;
+#pragma unroll
+            for (int q = 0; q < NB; q += 4) lu_ld4(from + q, &row[r][q]);
+          }
+          if (i > j && i < rows) {
+            const T l = row[r][jj] * rcp;
+            row[r][jj] = l;
+#pragma unroll
+            for (int g = 0; g < NB; g += 8) {
+              if (g > 0 && j0 + g >= nb) break;
+#pragma unroll
+              for (int q = g; q < g + 8; q += 4) {
+                T u[4];
+                lu_ld4(prow + q, u);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  if (q + e > jj) row[r][q + e] = fma(-l, u[e], row[r][q + e]);
+              }
+            }
+          }
+        }
       }
-      __syncthreads();
-      // A22 -= L21 * U12
-      const int m2 = rows - nb;
-      for (long long idx = tid; idx < (long long)m2 * ncol; idx += nt) {
-        const int i = (int)(idx / ncol), c = (int)(idx % ncol);
-        T s = a[(long long)(p0 + nb + i) * n + p0 + nb + c];
-        const T* l = panel + (nb + i) * LU_NB;
-#pragma unroll 8
-        for (int j = 0; j < nb; ++j) s = fma(-l[j], U12[j * n + c], s);
-        a[(long long)(p0 + nb + i) * n + p0 + nb + c] = s;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int i = tid + r * NT;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (i < rows && j0 + q < nb) Lt[(j0 + q) * np + i] = row[r][q];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) row[r][q] = q + 8 < NB ? row[r][q + 8] : T(0);
+      }
+    }
+    __syncthreads();
+    // the nb exchanges as one permutation: top[j] = row that ends at place j,
+    // orow / osrc = rows below the panel's that change and what they receive
+    // (always one of the panel's own rows: place j takes a lower row only at
+    // step j, after which no exchange moves it down)
+    if (warp == 0) {
+      int t = lane, orw = -1, osr = -1, cnt = 0;
+      for (int j = 0; j < nb; ++j) {
+        const int r2 = lpiv[j];
+        const int tj = __shfl_sync(0xffffffffu, t, j);
+        if (r2 < nb) {
+          const int t2 = __shfl_sync(0xffffffffu, t, r2);
+          if (lane == r2) t = tj;
+          if (lane == j) t = t2;
+        } else {
+          const unsigned m = __ballot_sync(0xffffffffu, orw == r2);
+          const int e = m ? __ffs(m) - 1 : cnt;
+          if (!m && lane == cnt) orw = osr = r2;
+          if (!m) ++cnt;
+          const int oe = __shfl_sync(0xffffffffu, osr, e);
+          if (lane == j) t = oe;
+          if (lane == e) osr = tj;
+        }
+      }
+      top[lane] = t;
+      orow[lane] = orw;
+      osrc[lane] = osr;
+      if (lane == 0) ocnt = cnt;
+    }
+    __syncthreads();
+    for (int i = warp; i < rows; i += NW)
+      if (lane < nb) a[(long long)(p0 + i) * n + p0 + lane] = Lt[lane * np + i];
+    // the other columns, one thread each
+    for (int c = tid; c < n; c += NT) {
+      if (c >= p0 && c < p0 + nb) continue;
+      T col[NB];
+      T* ac = a + (long long)p0 * n + c;
+#pragma unroll
+      for (int j = 0; j < NB; ++j) col[j] = j < nb ? ac[(long long)j * n] : T(0);
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        if (j < nb) U12[j * np + c] = col[j];
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        if (j < nb) col[j] = top[j] < nb ? U12[top[j] * np + c] : ac[(long long)top[j] * n];
+      for (int e = 0; e < ocnt; ++e) ac[(long long)orow[e] * n] = U12[osrc[e] * np + c];
+      if (c > p0) {  // L11^{-1} A12; nb == NB
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          const T v = col[j];
+#pragma unroll
+          for (int q = j / 4 * 4; q < NB; q += 4) {
+            T l[4];
+            lu_ld4(Lt + j * np + q, l);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (q + e > j) col[q + e] = fma(-l[e], v, col[q + e]);
+          }
+          U12[j * np + c] = v;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        if (j < nb) ac[(long long)j * n] = col[j];
+    }
+    __syncthreads();
+    // A22 -= L21 U12; the tiles' last rows and columns may lie past the matrix:
+    // their operands are whatever follows in shared memory, and are not stored
+    const int m2 = rows - nb, nr = (m2 + 31) / 32;
+    const int ty = lane >> 3, tx = lane & 7;
+    for (int u = warp; u < nr * nr; u += NW) {
+      const int i0 = u / nr * 32 + 8 * ty, c0 = u % nr * 32 + 4 * tx;  // in A22
+      T* at = a + (long long)(p0 + nb + i0) * n + p0 + nb + c0;
+      const int mr = min(8, m2 - i0), mc = min(4, m2 - c0);
+      T acc[8][4];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        if (r < mr && vec && mc > 0) {
+          lu_ld4(at + (long long)r * n, acc[r]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[r][e] = (r < mr && e < mc) ? at[(long long)r * n + e] : T(0);
+        }
+      }
+      const T* lp = Lt + nb + i0;
+      const T* up = U12 + p0 + nb + c0;
+#pragma unroll 4
+      for (int j = 0; j < NB; ++j) {
+        T l[8], v[4];
+        lu_ld4(lp + j * np, l);
+        lu_ld4(lp + j * np + 4, l + 4);
+        lu_ld4(up + j * np, v);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[r][e] = fma(-l[r], v[e], acc[r][e]);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        if (r < mr && vec && mc > 0) {
+          lu_st4(at + (long long)r * n, acc[r]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (r < mr && e < mc) at[(long long)r * n + e] = acc[r][e];
+        }
       }
     }
     __syncthreads();
   }
 }
 
-template <typename T>
-static int lu_factor_t(ves_ctx* c, int nv, int n, T* A, int* piv, cudaStream_t s) {
-  if (nv <= 0) return VES_OK;
-  const size_t sh = (size_t)(n * LU_NB + LU_NB * n) * sizeof(T);
-  if (sh > 220 * 1024) {
-    ves_record_error(VES_ERR_SHAPE, "lu_factor: n=%d too large", n);
-    return VES_ERR_SHAPE;
-  }
+template <typename T, int ROWS, int NT, int CTAS>
+static int lu_factor_start(ves_ctx* c, int nv, int n, T* A, int* piv, cudaStream_t s) {
+  const size_t sh = ((size_t)2 * LU_NB * lu_pitch(n) + 32) * sizeof(T);  // the last tiles read up to 31 past the end
   if (sh > 32 * 1024) {  // dynamic + static shared memory must fit the opt-in limit
     int rc = ves_cuda_status(
-        cudaFuncSetAttribute(lu_factor_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
+        cudaFuncSetAttribute(lu_factor_kernel<T, ROWS, NT, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
         "lu_factor smem attribute");
     if (rc) return rc;
   }
   ves_count_launch();
-  lu_factor_kernel<T><<<nv, 256, sh, s>>>(n, A, piv, c->status);
+  lu_factor_kernel<T, ROWS, NT, CTAS><<<nv, NT, sh, s>>>(n, A, piv, c->status);
   return ves_launch_check("lu_factor");
+}
+
+template <typename T>
+static int lu_factor_t(ves_ctx* c, int nv, int n, T* A, int* piv, cudaStream_t s) {
+  if (nv <= 0) return VES_OK;
+  if ((size_t)2 * LU_NB * n * sizeof(T) > 220 * 1024) {
+    ves_record_error(VES_ERR_SHAPE, "lu_factor: n=%d too large", n);
+    return VES_ERR_SHAPE;
+  }
+  // a thread per panel row, or two or four rows per thread where a CTA has
+  // fewer threads; FP64 stops at n = 440
+  if (n <= 128) return lu_factor_start<T, 1, 128, 4>(c, nv, n, A, piv, s);
+  if (n <= 256) return lu_factor_start<T, 1, 256, 2>(c, nv, n, A, piv, s);
+  if constexpr (sizeof(T) == 8) {
+    return lu_factor_start<T, 2, 256, 1>(c, nv, n, A, piv, s);
+  } else {
+    if (n <= 512) return lu_factor_start<T, 2, 256, 2>(c, nv, n, A, piv, s);
+    return lu_factor_start<T, 4, 256, 1>(c, nv, n, A, piv, s);
+  }
 }
 
 int launch_lu_factor(ves_ctx* c, int nv, int n, double* A, int* piv, cudaStream_t s) {
