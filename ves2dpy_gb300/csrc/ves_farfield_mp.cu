@@ -305,7 +305,10 @@ __device__ __forceinline__ void horner(float2& xr, float2& xi, float2& yr, float
 // run as packed FP32x2 fmas, two series to a register pair, which halves the
 // instructions per term.  Close pairs run the direct rule on records staged
 // 32 at a time by the warp itself, so no warp waits for another's close pairs
-// inside a stage.  Five CTAs of four warps per SM (102 registers): with 80
+// inside a stage, and a stage's buffer is refilled by the warp that leaves it
+// last, so that none waits for another's between stages either (S == 1; with a
+// barrier per stage a fifth of the warps' time: 8192 x N=32 13.3 -> 12.9 ms,
+// 2048 x N=96 4.04 -> 3.66, 1024 x N=128 2.05 -> 2.00).  Five CTAs of four warps per SM (102 registers): with 80
 // registers the direct rule's loads and MUFU results are not overlapped, with
 // 128 the series wait.  One sum, before (one column per CTA, every thread
 // working out every pair, all 25 orders staged) and now: 8192 x N=32 32.6 ->
@@ -326,7 +329,7 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_k
   __shared__ MPPair pairs[WARPS][kStage];
   __shared__ float4 drec[WARPS][32];
   __shared__ float2 part[S > 1 ? 2 : 1][S > 1 ? kUnits : 1][S > 1 ? kStage : 1][32];
-  __shared__ int turn[2][kUnits];
+  __shared__ int turn[2][kUnits], done[2];
   __shared__ uint64_t bar[2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = warp / S, sub = warp % S;
@@ -356,12 +359,15 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_k
     tc_fence_async_smem();
   }
   if (threadIdx.x < 2 * kUnits) turn[threadIdx.x / kUnits][threadIdx.x % kUnits] = 0;
+  if (threadIdx.x < 2) done[threadIdx.x] = 0;
   __syncthreads();
   float2 tot = make_float2(0.f, 0.f), cmp = make_float2(0.f, 0.f);
   unsigned terms = 0, ndirect = 0;
   int kst = 0;  // stages so far: stage buffers and barrier phases alternate
   bool failed = false;
-  for (int q = 0; q < p.ng && !failed; ++q) {
+  for (int q = 0; q < p.ng; ++q) {
+    // every warp is through with the last set's stages, or one has given up
+    if (q > 0 && __syncthreads_or(failed ? 1 : 0)) break;
     const MPSet& set = p.set[q];
     const int nstages = (set.nsrc + kStage - 1) / kStage;
     auto fetch = [&](int st, int buf) {  // thread 0
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_k
     for (int st = 0; st < nstages; ++st, ++kst) {
       const int buf = kst & 1, s0 = st * kStage, n = min(kStage, set.nsrc - s0);
       if (!tc_mbar_wait(&bar[buf], (kst >> 1) & 1, p.st, 30)) failed = true;
+      __syncwarp();  // S == 1: the previous stage's pairs have been read
       if (lane < n) {
         const MPSrc Sq = ssrc[buf][lane];
         const int s = s0 + lane;
@@ -495,23 +502,43 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_k
         else
           two_sum(tot, cmp, v);  // points past the column's end add too; they are not stored
       }
-      // nobody reads this stage any more (and every contribution is in)
-      failed = __syncthreads_or(failed ? 1 : 0) != 0;
-      if (S > 1) {
+      if constexpr (S == 1) {
+        // the warp that finishes a stage last fetches the next one into its
+        // place; nobody waits for the others
+        failed = __any_sync(0xffffffffu, failed);
+        if (failed) {  // the copies in flight land before the CTA ends
+          tc_mbar_wait(&bar[buf], (kst >> 1) & 1, nullptr, 0);
+          if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((kst + 1) >> 1) & 1, nullptr, 0);
+          break;
+        }
+        if (lane == 0) {
+          __threadfence_block();
+          if (atomicAdd(&done[buf], 1) == WARPS - 1) {
+            __threadfence_block();
+            done[buf] = 0;
+            if (st + 2 < nstages) {
+              tc_fence_async_smem();
+              fetch(st + 2, buf);
+            }
+          }
+        }
+      } else {
+        // nobody reads this stage any more and every contribution is in
+        failed = __syncthreads_or(failed ? 1 : 0) != 0;
         if (threadIdx.x < kUnits) turn[buf][threadIdx.x] = 0;
         if (sub == 0)
           for (int qs = 0; qs < n; ++qs) two_sum(tot, cmp, part[buf][unit][qs][lane]);
-      }
-      if (failed) {  // the copies in flight land before the CTA ends
-        if (threadIdx.x == 0) {
-          tc_mbar_wait(&bar[buf], (kst >> 1) & 1, nullptr, 0);
-          if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((kst + 1) >> 1) & 1, nullptr, 0);
+        if (failed) {  // the copies in flight land before the CTA ends
+          if (threadIdx.x == 0) {
+            tc_mbar_wait(&bar[buf], (kst >> 1) & 1, nullptr, 0);
+            if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((kst + 1) >> 1) & 1, nullptr, 0);
+          }
+          break;
         }
-        break;
-      }
-      if (threadIdx.x == 0 && st + 2 < nstages) {
-        tc_fence_async_smem();
-        fetch(st + 2, buf);
+        if (threadIdx.x == 0 && st + 2 < nstages) {
+          tc_fence_async_smem();
+          fetch(st + 2, buf);
+        }
       }
     }
   }
