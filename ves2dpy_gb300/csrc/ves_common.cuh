@@ -100,6 +100,23 @@ __device__ __forceinline__ double widen(float x) {
 }
 __device__ __forceinline__ double widen(double x) { return x; }
 
+// Row j of a circulant matrix (first column d) times two sequences, the matrix
+// read once: sa = sum_l d[(j - l) mod n] a[l], sb with b.
+__device__ __forceinline__ void circ2(const double* __restrict__ d, const double* __restrict__ a,
+                                      const double* __restrict__ b, int n, int j, double& sa, double& sb) {
+  double s = 0.0, t = 0.0;
+  for (int l = 0; l <= j; ++l) {
+    s = fma(d[j - l], a[l], s);
+    t = fma(d[j - l], b[l], t);
+  }
+  for (int l = j + 1; l < n; ++l) {
+    s = fma(d[j - l + n], a[l], s);
+    t = fma(d[j - l + n], b[l], t);
+  }
+  sa = s;
+  sb = t;
+}
+
 static inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 // Host helper: map a CUDA error to a status code, recording the message.

@@ -252,11 +252,15 @@ __device__ void eig2_lapack(double a, double b, double c, double d, double* w0, 
   v[3] = v2y;
 }
 
-__device__ void phys_center(int N, const double* d, const double* x, const double* y, double* red, double& cx,
-                            double& cy) {
+// dxb, dyb: the curve's derivative, left there for the caller
+__device__ void phys_center(int N, const double* d, const double* x, const double* y, double* dxb, double* dyb,
+                            double* red, double& cx, double& cy) {
   double a = 0, sx = 0, sy = 0;
   for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double dx = circ(d, x, N, j), dy = circ(d, y, N, j);
+    double dx, dy;
+    circ2(d, x, y, N, j, dx, dy);
+    dxb[j] = dx;
+    dyb[j] = dy;
     a += x[j] * dy - y[j] * dx;
     sx += x[j] * x[j] * dy;
     sy += y[j] * y[j] * dx;
@@ -266,7 +270,11 @@ __device__ void phys_center(int N, const double* d, const double* x, const doubl
   cy = -bsum(sy, red) / A;
 }
 
-__global__ void standardize_kernel(int N, const double* __restrict__ d1, const double* __restrict__ X,
+// One CTA per vesicle, latency-bound at few vesicles, bound by the FP64 pipe
+// (three derivatives, N^2 multiply-adds per coordinate each) at many.  The polar
+// angles are taken by all threads: one thread took all N for most of the
+// kernel's time.  N = 128: 61 vesicles 273 -> 67 us, 4096 vesicles 2.98 -> 1.29 ms.
+__global__ void __launch_bounds__(128) standardize_kernel(int N, const double* __restrict__ d1, const double* __restrict__ X,
                                    double* __restrict__ Xs, double* __restrict__ scaling, double* __restrict__ rotate,
                                    double* __restrict__ rot_center, double* __restrict__ trans,
                                    int* __restrict__ sort_idx) {
@@ -276,8 +284,10 @@ __global__ void standardize_kernel(int N, const double* __restrict__ d1, const d
   double* y = x + N;
   double* xr = y + N;
   double* yr = xr + N;
-  double* red = yr + N;  // [blockDim]
-  __shared__ int s_start;
+  double* dxb = yr + N;
+  double* dyb = dxb + N;
+  double* red = dyb + N;  // [blockDim]
+  __shared__ int s_start, s_idx[128];
   const int k = blockIdx.x;
   const double* Xk = X + (long long)k * 2 * N;
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
@@ -287,7 +297,7 @@ __global__ void standardize_kernel(int N, const double* __restrict__ d1, const d
   }
   __syncthreads();
   double cx, cy;
-  phys_center(N, d, x, y, red, cx, cy);
+  phys_center(N, d, x, y, dxb, dyb, red, cx, cy);
   // principal axes about the centre (curve_batch_compile.py:279-376)
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     xr[i] = x[i] - cx;
@@ -296,7 +306,8 @@ __global__ void standardize_kernel(int N, const double* __restrict__ d1, const d
   __syncthreads();
   double j11 = 0, j12 = 0, j21 = 0, j22 = 0;
   for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double dx = circ(d, xr, N, j), dy = circ(d, yr, N, j);
+    double dx, dy;
+    circ2(d, xr, yr, N, j, dx, dy);
     const double jac = sqrt(dx * dx + dy * dy);
     const double nx = dy / jac, ny = -dx / jac;
     const double xc = xr[j], yc = yr[j];
@@ -324,28 +335,48 @@ __global__ void standardize_kernel(int N, const double* __restrict__ d1, const d
   }
   __syncthreads();
   double ccx, ccy;
-  phys_center(N, d, xr, yr, red, ccx, ccy);
+  phys_center(N, d, xr, yr, dxb, dyb, red, ccx, ccy);
   const double tx = -ccx, ty = -ccy;
   double ls = 0.0;
   for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double dx = circ(d, xr, N, j), dy = circ(d, yr, N, j);
-    ls += sqrt(dx * dx + dy * dy);
+    ls += sqrt(dxb[j] * dxb[j] + dyb[j] * dyb[j]);
   }
   const double length = bsum(ls, red) * 2.0 * VES_PI / N;
   const double sc = 1.0 / length;
-  // first point of the sort order: smallest non-negative polar angle
-  if (threadIdx.x == 0) {
-    double best = 0;
-    int bi = -1;
-    for (int j = 0; j < N; ++j) {
-      double th = atan2(yr[j] + ty, xr[j] + tx);
-      if (th < 0) th = 100.0;
-      if (bi < 0 || th < best) {
-        best = th;
-        bi = j;
+  // first point of the sort order: smallest non-negative polar angle, the
+  // first such point on ties (a NaN only if it is the first point's)
+  double best = 0;
+  int bi = -1;
+  for (int j = threadIdx.x; j < N; j += blockDim.x) {
+    double th = atan2(yr[j] + ty, xr[j] + tx);
+    if (th < 0) th = 100.0;
+    if (j == 0 && th != th) th = -1.0;
+    if (th == th && (bi < 0 || th < best)) {
+      best = th;
+      bi = j;
+    }
+  }
+  red[threadIdx.x] = best;
+  s_idx[threadIdx.x] = bi;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    bi = -1;
+    for (int t = threadIdx.x; t < blockDim.x; t += 32) {
+      const int i2 = s_idx[t];
+      if (i2 >= 0 && (bi < 0 || red[t] < best || (red[t] == best && i2 < bi))) {
+        best = red[t];
+        bi = i2;
       }
     }
-    s_start = bi;
+    for (int o = 16; o > 0; o >>= 1) {
+      const double b2 = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (i2 >= 0 && (bi < 0 || b2 < best || (b2 == best && i2 < bi))) {
+        best = b2;
+        bi = i2;
+      }
+    }
+    if (threadIdx.x == 0) s_start = bi;
   }
   __syncthreads();
   const int start = s_start;
@@ -789,7 +820,7 @@ int standardize_run(ves_ctx* c, int nv, const double* X, double* Xs, double* sca
   }
   const int threads = 128;
   ves_count_launch();
-  standardize_kernel<<<nv, threads, (size_t)(5 * N + threads) * sizeof(double), s>>>(N, c->d1N, R, Xs, scaling,
+  standardize_kernel<<<nv, threads, (size_t)(7 * N + threads) * sizeof(double), s>>>(N, c->d1N, R, Xs, scaling,
                                                                                       rotate, rot_center, trans,
                                                                                       sort_idx);
   return ves_launch_check("standardize");

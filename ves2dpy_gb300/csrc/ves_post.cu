@@ -60,7 +60,7 @@ int pow2_threads(int n) {
 constexpr int kSpreadChunk = 64;
 
 __global__ void jac_dev_kernel(int N, const double* __restrict__ d1, const double* __restrict__ X,
-                               double* __restrict__ dev) {
+                               double* __restrict__ dev, double* __restrict__ jsum) {
   extern __shared__ double sh[];
   double* d = sh;
   double* x = d + N;
@@ -77,11 +77,13 @@ __global__ void jac_dev_kernel(int N, const double* __restrict__ d1, const doubl
   __syncthreads();
   double js = 0.0;
   for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double dx = circ(d, x, N, j), dy = circ(d, y, N, j);
+    double dx, dy;
+    circ2(d, x, y, N, j, dx, dy);
     jac[j] = sqrt(dx * dx + dy * dy);
     js += jac[j];
   }
-  const double mean = bsum(js, red) / N;
+  const double total = bsum(js, red), mean = total / N;
+  if (threadIdx.x == 0) jsum[k] = total;
   for (int j = threadIdx.x; j < N; j += blockDim.x) dev[(long long)k * N + j] = fabs(jac[j] - mean);
 }
 
@@ -110,17 +112,18 @@ __global__ void spread_kernel(int nchunk, int N, const double* __restrict__ part
   if (threadIdx.x == 0) *spread = anynan ? __longlong_as_double(0x7ff8000000000000LL) : r;
 }
 
-// one redistributeArcLength pass; flags[k] = 1 if vesicle k was left as is
-__global__ void redistribute_kernel(int N, const double* __restrict__ d1, const double* __restrict__ cos6,
+// one redistributeArcLength pass; flags[k] = 1 if vesicle k was left as is.
+// Bound by the FP64 pipe (transforms of 6N points, N series of N terms) at many
+// vesicles, by latency at few, so the length is the one jac_dev_kernel summed, a
+// weight is divided once and the transforms have twice the threads of the series.
+// N = 128: 61 vesicles 113 -> 85 us, 4096 vesicles 2.28 -> 1.97 ms.
+__global__ void redistribute_kernel(int N, const double* __restrict__ jsum_p, const double* __restrict__ cos6,
                                     const double* __restrict__ sin6, const double* __restrict__ spread_p,
                                     const double* __restrict__ X, double* __restrict__ Xout,
-                                    int* __restrict__ flags) {
+                                    int* __restrict__ flags, int parts) {
   extern __shared__ double sh[];
   const int M = 6 * N;  // upsampled grid of the arc-length parameter search
-  double* d = sh;
-  double* x = d + N;
-  double* y = x + N;
-  double* are = y + N;     // [M] spectrum work arrays
+  double* are = sh;        // [M] spectrum work arrays
   double* aim = are + M;   // [M]
   double* tre = aim + M;   // [M] FFT scratch
   double* tim = tre + M;   // [M]
@@ -132,19 +135,7 @@ __global__ void redistribute_kernel(int N, const double* __restrict__ d1, const 
   const int k = blockIdx.x;
   const double* Xk = X + (long long)k * 2 * N;
   double* Ok = Xout + (long long)k * 2 * N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    d[i] = d1[i];
-    x[i] = Xk[i];
-    y[i] = Xk[N + i];
-  }
-  __syncthreads();
-  // jacobian on the N grid: its spread decides, its sum is the length
-  double js = 0.0;
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const double dx = circ(d, x, N, j), dy = circ(d, y, N, j);
-    js += sqrt(dx * dx + dy * dy);
-  }
-  const double jsum = bsum(js, red);
+  const double jsum = jsum_p[k];
   const double mean = jsum / N;
   if (!(*spread_p > 1e-5 * mean)) {
     for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) Ok[i] = Xk[i];
@@ -155,8 +146,8 @@ __global__ void redistribute_kernel(int N, const double* __restrict__ d1, const 
   // zh = fft(x + i y)/N, modes 0..N/2-1, -N/2..-1 (length-N FFT, twiddles
   // from the 6N table); also the coefficients of the final evaluation
   for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    zr[j] = x[j];
-    zi[j] = y[j];
+    zr[j] = Xk[j];
+    zi[j] = Xk[N + j];
   }
   ves_fft(zr, zi, tre, tim, N, cos6, sin6, -1, 6);
   for (int m = threadIdx.x; m < N; m += blockDim.x) {
@@ -197,14 +188,18 @@ __global__ void redistribute_kernel(int N, const double* __restrict__ d1, const 
   const double C0 = are[0];
   // al(t_u) = int_0^{t_u} arc = (C_0/M) t_u + sum_{k=1}^{M/2-1} 2/(k M) [C_k sin(k t_u) - S_k (cos(k t_u) - 1)]
   //         = (C_0/M) t_u + sum_k 2/(k M) S_k + Im sum_k (2/(k M)) X_k e^{i k t_u}
-  double cpart = 0.0;
-  for (int kk = 1 + threadIdx.x; kk < M / 2; kk += blockDim.x) cpart += 2.0 / ((double)kk * M) * (-aim[kk]);
+  __syncthreads();  // all have read are[0]
+  double cpart = 0.0;  // the first `parts` threads sum, in this order whatever the CTA's size
+  for (int kk = threadIdx.x; kk < M; kk += blockDim.x)
+    if (kk == 0 || kk >= M / 2) are[kk] = aim[kk] = 0.0;
+  if (threadIdx.x < parts)
+    for (int kk = 1 + threadIdx.x; kk < M / 2; kk += parts) {
+      const double f = 2.0 / ((double)kk * M);
+      cpart = fma(f, -aim[kk], cpart);
+      are[kk] *= f;
+      aim[kk] *= f;
+    }
   const double K0 = bsum(cpart, red);
-  for (int kk = threadIdx.x; kk < M; kk += blockDim.x) {
-    const double f = (kk >= 1 && kk < M / 2) ? 2.0 / ((double)kk * M) : 0.0;
-    are[kk] *= f;
-    aim[kk] *= f;
-  }
   ves_fft(are, aim, tre, tim, M, cos6, sin6, +1);
   for (int u = threadIdx.x; u < M; u += blockDim.x) al[u] = C0 / M * (2.0 * VES_PI * u / M) + K0 + aim[u];
   __syncthreads();
@@ -504,6 +499,7 @@ int post_redistribute(ves_ctx* c, int nv, const double* X, double* Xout, int* fl
   double* dev = ws.take<double>((size_t)nv * N);
   double* partial = ws.take<double>((size_t)nchunk * N);
   double* spread = ws.take<double>(1);
+  double* jsum = ws.take<double>(nv);
   if (ws.sizing) return VES_OK;
   if (!ws.ok()) {
     ves_record_error(VES_ERR_WORKSPACE, "redistribute: workspace too small (%zu needed)", ws.off);
@@ -516,10 +512,11 @@ int post_redistribute(ves_ctx* c, int nv, const double* X, double* Xout, int* fl
   }
   const int threads = pow2_threads(N);
   ves_count_launch(3);
-  jac_dev_kernel<<<nv, threads, (size_t)(4 * N + threads) * sizeof(double), s>>>(N, c->d1N, X, dev);
+  jac_dev_kernel<<<nv, threads, (size_t)(4 * N + threads) * sizeof(double), s>>>(N, c->d1N, X, dev, jsum);
   dev_rowsum_kernel<<<nchunk, 128, 0, s>>>(nv, N, dev, partial);
   spread_kernel<<<1, 256, 0, s>>>(nchunk, N, partial, spread);
-  const size_t sh = (size_t)(6 * N + 5 * M + threads) * sizeof(double);
+  const int wide = threads < 256 ? 2 * threads : threads;  // the transforms have 6N points
+  const size_t sh = (size_t)(3 * N + 5 * M + wide) * sizeof(double);
   if (sh > 32 * 1024) {
     int rc = ves_cuda_status(cudaFuncSetAttribute(redistribute_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)sh),
@@ -527,7 +524,7 @@ int post_redistribute(ves_ctx* c, int nv, const double* X, double* Xout, int* fl
     if (rc) return rc;
   }
   ves_count_launch();
-  redistribute_kernel<<<nv, threads, sh, s>>>(N, c->d1N, c->cos6, c->sin6, spread, X, Xout, flags);
+  redistribute_kernel<<<nv, wide, sh, s>>>(N, jsum, c->cos6, c->sin6, spread, X, Xout, flags, threads);
   return ves_launch_check("redistribute");
 }
 
