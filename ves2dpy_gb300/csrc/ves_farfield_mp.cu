@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(256) mp_prep_kernel(int ns, const double* __re
   for (int q = 0; q < kPer; ++q) A[q] = B[q] = E[q] = make_float2(0.f, 0.f);
   const double iR = 1.0 / R;
   for (int c0 = 0; c0 < ns; c0 += 256) {
-    // each point scaled once (FP64 is the slow pipe: 80 of 262 us at 1024 x
-    // N=128 went on every warp scaling every point) and read by every warp
+    // each point scaled once (FP64 is the slow pipe) and read by every warp:
+    // 262 -> 122 us at 1024 x N=128
     __syncthreads();
     if (c0 + t < ns) {
       const int j = c0 + t;
