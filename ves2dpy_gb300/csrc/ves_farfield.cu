@@ -546,6 +546,8 @@ struct FFPlan {
   size_t smem;
 };
 
+constexpr long long kFFFill = 152 * 2;  // resident CTAs of the FP32 rule
+
 template <typename Real>
 FFPlan ff_plan(int nsrc, int ns, long long total_pts) {
   FFPlan pl;
@@ -562,6 +564,15 @@ FFPlan ff_plan(int nsrc, int ns, long long total_pts) {
   if (nsplit > max_split) nsplit = max_split;
   if (nsplit < 1) nsplit = 1;
   int per = (nsrc + nsplit - 1) / nsplit;
+  if (sizeof(Real) == 4 && (long long)pl.tgt_blocks * nsplit < kFFFill) {
+    // Too few CTAs with two whole stages per split: stages and splits of as few
+    // vesicles as fill the chip once, down to one.  One sum with its
+    // preparation: 16 x N=32 387 -> 83 us, 40 x N=16 344 -> 82, 12 x N=128 381 ->
+    // 229, 100 x N=32 389 -> 131; from one filled chip on (61 x N=128) the plan
+    // and its sum are what they were.
+    per = (int)std::max(1LL, ((long long)nsrc * pl.tgt_blocks + kFFFill - 1) / kFFFill);
+    pl.sv_per_stage = std::min(pl.sv_per_stage, per);
+  }
   per = ((per + pl.sv_per_stage - 1) / pl.sv_per_stage) * pl.sv_per_stage;
   pl.src_per_split = per > 0 ? per : 1;
   pl.nsplit = (nsrc + pl.src_per_split - 1) / pl.src_per_split;
