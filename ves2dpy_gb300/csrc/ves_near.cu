@@ -501,31 +501,89 @@ __global__ void __launch_bounds__(128) matlab_zone_kernel(int Nt, int Ns, int ma
   for (int i = threadIdx.x; i < wN; i += blockDim.x) em[i] = bits[i];
 }
 
-// MATLAB correction, one warp per entry.  DL: the layer potential at the
-// Lagrange points is the double layer (kernelDirect = exactStokesDL,
-// tstep_biem.py:236,501), with normals (ty, -tx) of the upsampled source and
-// den already scaled by (1 - visc); otherwise the single layer.
-// Targets Xt and LP with Nt points per vesicle; sources with Ns points (vself)
-// and Nup upsampled points (Xup, tang_up, den).
-// One MATLAB-scheme correction problem: targets of a point set with Nt
-// points per vesicle against the sources (Ns points, Nup upsampled) of
-// another set or of itself, with the near entries of its lists.
+// MATLAB correction.  DL: the layer potential at the Lagrange points is the
+// double layer (kernelDirect = exactStokesDL, tstep_biem.py:236,501), with
+// normals (ty, -tx) of the upsampled source and den already scaled by
+// (1 - visc); otherwise the single layer.
+// One correction problem: targets of a point set (Xt and LP, Nt points per
+// vesicle) against the sources (vself with Ns points; Xup, tang_up and den
+// with Nup upsampled points) of another set or of itself, with the near
+// entries of its lists.
 struct MatlabPair {
   int Nt, Ns, Nup;
   double h;
   const double *Xt, *Xup, *tang_up, *den, *vself, *lag;
   const int* n_entries;
-  int max_entries;
+  int max_entries, maxc;
   const int *ent_tsj, *ent_icp;
   const double* ent_geo;
+  const int* cand_count;
+  const uint32_t* excl_mask;
   double *LP, *near_only;
 };
 
-// Near entry e of one correction problem, one warp (lane = its lane).
+// Several correction problems (every pair of point sets of a suspension with
+// several point counts) in one launch: problem k owns the warps
+// [warp0[k], warp0[k+1]), one per near-entry slot.
+constexpr int kMatlabPairs = 16;
+struct MatlabPairs {
+  int np;
+  long long warp0[kMatlabPairs + 1];
+  MatlabPair pair[kMatlabPairs];
+};
+
+// Problem, source vesicle and list place of an entry, in the order in which
+// the entries of one target point are added.
+typedef unsigned long long MatlabKey;
+static_assert(kMatlabPairs <= 16, "four bits of a key");
+constexpr MatlabKey kNoEntry = ~0ull;
+__device__ __forceinline__ MatlabKey matlab_key(int k, int s, int e) {
+  return ((MatlabKey)k << 60) | ((MatlabKey)(unsigned)s << 32) | (unsigned)e;
+}
+
+// true if point j of target vesicle t lies near more than one source vesicle
+// of the problems that add to LP (the warp's lanes share the slots)
+__device__ __forceinline__ bool matlab_shared(const MatlabPairs& P, const double* LP, int t, int j, int lane) {
+  int n = 0;
+  for (int k = 0; k < P.np; ++k) {
+    const MatlabPair& a = P.pair[k];
+    if (a.LP != LP || !a.cand_count || !a.excl_mask) continue;
+    const int cc = min(a.cand_count[t], a.maxc), nw = (a.Nt + 31) / 32;
+    const uint32_t* m = a.excl_mask + (long long)t * a.maxc * nw + (j >> 5);
+    for (int s0 = 0; s0 < cc; s0 += 32) {
+      const bool bit = s0 + lane < cc && ((m[(long long)(s0 + lane) * nw] >> (j & 31)) & 1u);
+      n += __popc(__ballot_sync(0xffffffffu, bit));
+    }
+  }
+  return n > 1;
+}
+
+// the first entry of point (t, j) at or after key `from` (kNoEntry: none)
+__device__ __forceinline__ MatlabKey matlab_next(const MatlabPairs& P, const double* LP, int t, int j, MatlabKey from,
+                                                 int lane) {
+  MatlabKey best = kNoEntry;
+  for (int k = 0; k < P.np; ++k) {
+    const MatlabPair& a = P.pair[k];
+    if (a.LP != LP) continue;
+    const int ne = min(*a.n_entries, a.max_entries);
+#pragma unroll 4
+    for (int e = lane; e < ne; e += 32) {
+      if (a.ent_tsj[3 * e] != t || a.ent_tsj[3 * e + 2] != j) continue;
+      const MatlabKey key = matlab_key(k, a.ent_tsj[3 * e + 1], e);
+      if (key >= from && key < best) best = key;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const MatlabKey b = __shfl_xor_sync(0xffffffffu, best, o);
+    if (b < best) best = b;
+  }
+  return best;
+}
+
+// Near entry e of problem a (target t, source s, point j), one warp: its value
+// is added to LP by lane 0.
 template <bool DL>
-__device__ __forceinline__ void matlab_correct_entry(const MatlabPair& a, int e, int lane) {
-  const int ne = min(*a.n_entries, a.max_entries);
-  if (e >= ne) return;
+__device__ __forceinline__ void matlab_add_entry(const MatlabPair& a, int e, int lane) {
   const int t = a.ent_tsj[3 * e], s = a.ent_tsj[3 * e + 1], j = a.ent_tsj[3 * e + 2];
   const int icp = a.ent_icp[e];
   const double dist = a.ent_geo[4 * e], nxp = a.ent_geo[4 * e + 1], nyp = a.ent_geo[4 * e + 2], th = a.ent_geo[4 * e + 3];
@@ -601,36 +659,36 @@ __device__ __forceinline__ void matlab_correct_entry(const MatlabPair& a, int e,
   }
 }
 
+// One warp per near entry.  A point near one source takes one addition.  The
+// entries of a point near several sources (of one set or of several) are all
+// added by the warp of the first of them, in ascending order of (problem,
+// source), so that the sum does not depend on the order of the lists or of the
+// warps; such points are few, and finding their entries is a search of the
+// lists.  FP64 arithmetic (six layer potentials over Nup points per entry)
+// bounds the kernel.
 template <bool DL>
-__global__ void matlab_correct_kernel(int Nt, int Ns, int Nup, double h, const double* __restrict__ Xt,
-                                      const double* __restrict__ Xup, const double* __restrict__ tang_up,
-                                      const double* __restrict__ den,
-                                      const double* __restrict__ vself, const double* __restrict__ lag,
-                                      const int* __restrict__ n_entries, int max_entries,
-                                      const int* __restrict__ ent_tsj, const int* __restrict__ ent_icp,
-                                      const double* __restrict__ ent_geo, double* __restrict__ LP,
-                                      double* __restrict__ near_only) {
-  const MatlabPair a{Nt, Ns, Nup, h, Xt, Xup, tang_up, den, vself, lag, n_entries, max_entries,
-                     ent_tsj, ent_icp, ent_geo, LP, near_only};
-  matlab_correct_entry<DL>(a, (blockIdx.x * blockDim.x + threadIdx.x) / 32, threadIdx.x % 32);
-}
-
-// Several correction problems (every pair of point sets of a suspension with
-// several point counts) in one launch: problem k owns the warps
-// [warp0[k], warp0[k+1]), one per near-entry slot.
-constexpr int kMatlabPairs = 16;
-struct MatlabPairs {
-  int np;
-  long long warp0[kMatlabPairs + 1];
-  MatlabPair pair[kMatlabPairs];
-};
-
-__global__ void matlab_correct_pairs_kernel(MatlabPairs P) {
+__global__ void matlab_correct_kernel(const __grid_constant__ MatlabPairs P) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int lane = threadIdx.x % 32;
   if (w >= P.warp0[P.np]) return;
   int k = 0;
   while (k + 1 < P.np && w >= P.warp0[k + 1]) ++k;
-  matlab_correct_entry<false>(P.pair[k], (int)(w - P.warp0[k]), threadIdx.x % 32);
+  int e = (int)(w - P.warp0[k]);
+  const double* LP = P.pair[k].LP;
+  if (e >= min(*P.pair[k].n_entries, P.pair[k].max_entries)) return;
+  const int* tsj = P.pair[k].ent_tsj + 3 * (long long)e;
+  const int t = tsj[0], j = tsj[2];
+  const bool shared = matlab_shared(P, LP, t, j, lane);
+  MatlabKey key = matlab_key(k, tsj[1], e);
+  if (shared && matlab_next(P, LP, t, j, 0, lane) != key) return;
+  for (;;) {
+    matlab_add_entry<DL>(P.pair[k], e, lane);
+    if (!shared) return;
+    key = matlab_next(P, LP, t, j, key + 1, lane);
+    if (key == kNoEntry) return;
+    k = (int)(key >> 60);
+    e = (int)(unsigned)key;
+  }
 }
 
 __global__ void min_reduce_kernel(int n, const double* __restrict__ a, double* __restrict__ out) {
@@ -730,6 +788,49 @@ int find_candidates(ves_ctx* c, int nt, int ns, bool same_set, const double* tbo
     return VES_ERR_NEARLIST_OVERFLOW;
   }
   return VES_OK;
+}
+
+// One MATLAB correction problem of a launch: targets Xt of context ct, sources
+// of context cs, lists nl.
+MatlabPair matlab_pair(const ves_ctx* ct, const ves_ctx* cs, const double* Xt, const double* Xup_s,
+                       const double* tang_up, const double* den_s, const double* vself_s, const ves_near_lists* nl,
+                       double h, double* LP, double* near_only) {
+  MatlabPair a;
+  a.Nt = ct->N;
+  a.Ns = cs->N;
+  a.Nup = cs->Nup;
+  a.h = h;
+  a.Xt = Xt;
+  a.Xup = Xup_s;
+  a.tang_up = tang_up;
+  a.den = den_s;
+  a.vself = vself_s;
+  a.lag = ct->lag;
+  a.n_entries = nl->n_entries;
+  a.max_entries = nl->max_entries;
+  a.maxc = nl->maxc;
+  a.ent_tsj = nl->ent_tsj;
+  a.ent_icp = nl->ent_icp;
+  a.ent_geo = nl->ent_geo;
+  a.cand_count = nl->cand_count;
+  a.excl_mask = nl->excl_mask;
+  a.LP = LP;
+  a.near_only = near_only;
+  return a;
+}
+
+template <bool DL>
+void launch_matlab_correct(int np, const MatlabPair* pairs, cudaStream_t s) {
+  MatlabPairs P;
+  memset(&P, 0, sizeof(P));
+  P.np = np;
+  for (int k = 0; k < np; ++k) {
+    P.pair[k] = pairs[k];
+    P.warp0[k + 1] = P.warp0[k] + pairs[k].max_entries;
+  }
+  if (P.warp0[np] <= 0) return;
+  ves_count_launch();
+  matlab_correct_kernel<DL><<<(unsigned)ceil_div(P.warp0[np] * 32, 256), 256, 0, s>>>(P);
 }
 
 }  // namespace
@@ -858,12 +959,8 @@ int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const doubl
     hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
                                                                     nl->cand_src, nl->hh_mask, vself, LP, near_only);
   } else if (scheme == VES_NEAR_MATLAB) {
-    const long long warps = nl->max_entries;
-    ves_count_launch();
-    matlab_correct_kernel<false><<<ceil_div(warps * 32, 256), 256, 0, s>>>(N, N, Nup, h, X, Xup, nullptr, den, vself,
-                                                                           c->lag,
-                                                                    nl->n_entries, nl->max_entries, nl->ent_tsj,
-                                                                    nl->ent_icp, nl->ent_geo, LP, near_only);
+    const MatlabPair a = matlab_pair(c, c, X, Xup, nullptr, den, vself, nl, h, LP, near_only);
+    launch_matlab_correct<false>(1, &a, s);
   }
   return ves_launch_check("near_sing_int");
 }
@@ -912,12 +1009,8 @@ int near_zone_matlab_cross(ves_ctx* ct, ves_ctx* cs, int nvt, const double* Xt, 
 // velocities vself_s; the near entries of nl; added to LP.
 int near_correct_matlab(ves_ctx* ct, ves_ctx* cs, const double* Xt, const double* Xup_s, const double* den_s,
                         const double* vself_s, const ves_near_lists* nl, double h, double* LP, cudaStream_t s) {
-  const long long warps = nl->max_entries;
-  if (warps <= 0) return VES_OK;
-  ves_count_launch();
-  matlab_correct_kernel<false><<<ceil_div(warps * 32, 256), 256, 0, s>>>(
-      ct->N, cs->N, cs->Nup, h, Xt, Xup_s, nullptr, den_s, vself_s, ct->lag, nl->n_entries, nl->max_entries,
-      nl->ent_tsj, nl->ent_icp, nl->ent_geo, LP, nullptr);
+  const MatlabPair a = matlab_pair(ct, cs, Xt, Xup_s, nullptr, den_s, vself_s, nl, h, LP, nullptr);
+  launch_matlab_correct<false>(1, &a, s);
   return ves_launch_check("near_correct_matlab");
 }
 
@@ -932,42 +1025,17 @@ int near_correct_matlab_pairs(int np, ves_ctx* const* ct, ves_ctx* const* cs, co
     ves_record_error(VES_ERR_ARG, "near_correct_matlab_pairs: 1 to %d problems", kMatlabPairs);
     return VES_ERR_ARG;
   }
-  MatlabPairs P;
-  memset(&P, 0, sizeof(P));
-  P.np = np;
-  P.warp0[0] = 0;
-  for (int k = 0; k < np; ++k) {
-    MatlabPair& a = P.pair[k];
-    a.Nt = ct[k]->N;
-    a.Ns = cs[k]->N;
-    a.Nup = cs[k]->Nup;
-    a.h = h[k];
-    a.Xt = Xt[k];
-    a.Xup = Xup_s[k];
-    a.tang_up = nullptr;
-    a.den = den_s[k];
-    a.vself = vself_s[k];
-    a.lag = ct[k]->lag;
-    a.n_entries = nl[k]->n_entries;
-    a.max_entries = nl[k]->max_entries;
-    a.ent_tsj = nl[k]->ent_tsj;
-    a.ent_icp = nl[k]->ent_icp;
-    a.ent_geo = nl[k]->ent_geo;
-    a.LP = LP[k];
-    a.near_only = nullptr;
-    P.warp0[k + 1] = P.warp0[k] + nl[k]->max_entries;
-  }
-  const long long warps = P.warp0[np];
-  if (warps <= 0) return VES_OK;
-  ves_count_launch();
-  matlab_correct_pairs_kernel<<<(unsigned)ceil_div(warps * 32, 256), 256, 0, s>>>(P);
+  MatlabPair pairs[kMatlabPairs];
+  for (int k = 0; k < np; ++k)
+    pairs[k] = matlab_pair(ct[k], cs[k], Xt[k], Xup_s[k], nullptr, den_s[k], vself_s[k], nl[k], h[k], LP[k], nullptr);
+  launch_matlab_correct<false>(np, pairs, s);
   return ves_launch_check("near_correct_matlab_pairs");
 }
 
 int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision, int nvt, const double* Xt, int nvs,
                             const double* Xup_s, const double* den_s, const double* vself_s,
                             const ves_near_lists* nl, double h, double* LP, WsCarver& ws, cudaStream_t s) {
-  const int Nt = ct->N, Ns = cs->N, Nups = cs->Nup;
+  const int Nt = ct->N, Nups = cs->Nup;
   double* tmp = ws.take<double>((size_t)nvt * 2 * Nt);
   const ves_near_lists* excl = (scheme == VES_NEAR_MATLAB) ? nl : nullptr;
   if (ws.sizing) {
@@ -989,11 +1057,8 @@ int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision,
   ves_count_launch();
   add_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, tmp, LP);
   if (scheme == VES_NEAR_MATLAB) {
-    const long long warps = nl->max_entries;
-    ves_count_launch();
-    matlab_correct_kernel<false><<<ceil_div(warps * 32, 256), 256, 0, s>>>(
-        Nt, Ns, Nups, h, Xt, Xup_s, nullptr, den_s, vself_s, ct->lag, nl->n_entries, nl->max_entries, nl->ent_tsj,
-        nl->ent_icp, nl->ent_geo, LP, nullptr);
+    const MatlabPair a = matlab_pair(ct, cs, Xt, Xup_s, nullptr, den_s, vself_s, nl, h, LP, nullptr);
+    launch_matlab_correct<false>(1, &a, s);
   }
   return ves_launch_check("near_sing_int_cross");
 }
@@ -1048,11 +1113,8 @@ int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const do
     hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
                                                                     nl->cand_src, nl->hh_mask, vself, LP, near_only);
   } else if (scheme == VES_NEAR_MATLAB) {
-    const long long warps = nl->max_entries;
-    ves_count_launch();
-    matlab_correct_kernel<true><<<ceil_div(warps * 32, 256), 256, 0, s>>>(
-        N, N, Nup, h, X, Xup, tang_up, den, vself, c->lag, nl->n_entries, nl->max_entries, nl->ent_tsj, nl->ent_icp,
-        nl->ent_geo, LP, near_only);
+    const MatlabPair a = matlab_pair(c, c, X, Xup, tang_up, den, vself, nl, h, LP, near_only);
+    launch_matlab_correct<true>(1, &a, s);
   }
   return ves_launch_check("near_sing_int_dl");
 }
