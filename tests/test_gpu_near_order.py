@@ -94,3 +94,33 @@ def test_step_of_two_point_sets_repeats():
         out = [a.clone() for a in list(Xn) + list(sig)]
         ref = ref or out
         assert all(torch.equal(a, b) for a, b in zip(out, ref)), k
+
+
+def hedgehog(N, thresh, maxc=32, nrow=5):
+    from ves2dpy_gb300 import Poten
+    from ves2dpy_gb300.biem_support import NearZone
+    from ves2dpy_gb300.capsules import capsules
+    from ves2dpy_gb300.layout import to_vm
+    X = T(circles(*packed_circles(nrow, nrow, 0.05), N))
+    near = NearZone.build_py(to_vm(X), N, thresh=thresh, maxc=maxc)
+    f = torch.randn(X.shape, dtype=torch.float64, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3))
+    op = Poten(N)
+    ves = capsules(X, None, None, 1.0, 1.0)
+
+    def correction():
+        """The far field with the correction, and the correction alone, of self velocities f."""
+        return op.nearSingInt_hh(ves, f, lambda F: F, near, precision="fp64")
+
+    return X, near, f, correction
+
+
+def test_hedgehog_stays_in_its_lists():
+    """A candidate count above the lists' capacity is read as the capacity."""
+    _, near, _, correction = hedgehog(16, 0.2)
+    need = int(near.cand_count.max().item())
+    _, near, _, correction = hedgehog(16, 0.2, maxc=need)
+    assert near.maxc == need
+    LP, only = correction()
+    near.cand_count[near.cand_count == need] = need + 1000
+    LP2, only2 = correction()
+    assert torch.equal(LP, LP2) and torch.equal(only, only2) and float(only.abs().max()) > 0

@@ -342,8 +342,8 @@ __global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, i
   extern __shared__ double xk[];  // [2][N] coarse points of t (k1 of every pair)
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int nc = cand_count[t];
-  if (nc == 0) return;
+  const int nc = min(cand_count[t], maxc);
+  if (nc <= 0) return;
   for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) xk[i] = X[(long long)t * 2 * N + i];
   __syncthreads();
   const int wU = (Nup + 31) / 32;
