@@ -124,3 +124,35 @@ def test_hedgehog_stays_in_its_lists():
     near.cand_count[near.cand_count == need] = need + 1000
     LP2, only2 = correction()
     assert torch.equal(LP, LP2) and torch.equal(only, only2) and float(only.abs().max()) > 0
+
+
+@pytest.mark.parametrize("N, thresh, most", [(16, 0.7, 2), (16, 2.0, 7), (32, 1.2, 3)])
+def test_hedgehog_adds_in_ascending_order(N, thresh, most):
+    """The correction alone, bit for bit, against additions in ascending order
+    of the vesicle whose self velocity is added; hedgehog points of up to `most`
+    vesicles."""
+    X, near, f, correction = hedgehog(N, thresh)
+    nv, Nup = X.shape[1], near.Nup
+    Xh, fh = X.cpu().numpy(), f.cpu().numpy()
+    up = torch.fft.fft(torch.complex(X[:N], X[N:]), dim=0).cpu().numpy()
+    pad = np.zeros((Nup, nv), dtype=complex)
+    pad[:N // 2], pad[Nup - N // 2:] = up[:N // 2], up[N // 2:]
+    z = np.fft.ifft(pad, axis=0) * (Nup / N)
+    ref, times = np.zeros((2 * N, nv)), np.zeros((N, nv), dtype=int)
+    for id1, t in zip(*near.hh()):  # ascending t
+        k2, J = divmod(int(id1), N)
+        if k2 >= nv or k2 == t:
+            continue
+        d2 = (Xh[:N, t] - z[J, k2].real) ** 2 + (Xh[N:, t] - z[J, k2].imag) ** 2
+        p = (int(np.argmin(d2)) - 3) % N
+        two = np.sort(d2)[:2]
+        assert two[1] - two[0] > 1e-9  # no tie decides
+        ref[J, k2] += fh[p, t]
+        ref[N + J, k2] += fh[N + p, t]
+        times[J, k2] += 1
+    assert times.max() == most
+    LP, only = correction()
+    assert np.array_equal(only.cpu().numpy(), ref)
+    for _ in range(20):
+        LP2, only2 = correction()
+        assert torch.equal(LP, LP2) and torch.equal(only, only2)

@@ -173,10 +173,15 @@ int near_zone_py(ves_ctx* c, int nv, const double* X, const double* Xup, double 
                  const ves_near_lists* nl, WsCarver& ws, cudaStream_t s);
 int near_zone_matlab(ves_ctx* c, int nv, const double* X, double h, const ves_near_lists* nl,
                      WsCarver& ws, cudaStream_t s);
+// Which hedgehog points of the lists of near_zone_py several vesicles add to:
+// hits [3][nv][N], read by the py_hh correction.  Depends on the lists alone, so
+// a step makes them once.
+int hedgehog_hits(const ves_ctx* c, int nv, const ves_near_lists* nl, int* hits, cudaStream_t s);
+// hits: hedgehog_hits of nl (scheme VES_NEAR_PY_HH), or null: made in the workspace
 int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const double* X,
                       const double* sa_up, const double* Xup, const double* f, const double* vself,
                       const ves_near_lists* nl, double h, double* LP, double* near_only, WsCarver& ws,
-                      cudaStream_t s);
+                      cudaStream_t s, const int* hits = nullptr);
 // between two vesicle sets (targets: ct, Xt; sources: cs, Xs / Xup_s, den_s, vself_s)
 int near_zone_matlab_cross(ves_ctx* ct, ves_ctx* cs, int nvt, const double* Xt, int nvs, const double* Xs, double h,
                            const ves_near_lists* nl, WsCarver& ws, cudaStream_t s);
@@ -205,7 +210,7 @@ int farfield_dl_run(ves_ctx* c, int precision, int nsrc, int ns, const double* X
 int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* Xup,
                          const double* tang_up, const double* sa_up, const double* visc, const double* f,
                          const double* vself, const ves_near_lists* nl, double h, double* LP, double* near_only,
-                         WsCarver& ws, cudaStream_t s);
+                         WsCarver& ws, cudaStream_t s, const int* hits = nullptr);
 
 // RBF near-field fits (nearSingInt_rbf): adds the fits of the near pairs to LP
 int rbf_near_correct(ves_ctx* c, int nv, const double* X, const double* f, const double* vself,

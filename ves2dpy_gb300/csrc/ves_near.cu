@@ -326,17 +326,80 @@ __global__ void __launch_bounds__(256) py_masks_kernel(int N, int Nup, int maxc,
   for (int i = threadIdx.x; i < wU; i += blockDim.x) hm[i] = hbits[i];
 }
 
-// py_hh correction: one CTA per vesicle t.  Latency-bound: a hedgehog point is
-// a search of the N coarse points (FP64 distances), and the points of a close
-// pair sit side by side, that is in one or two words of the mask.  So the
-// warps take the set bits in turn and the lanes share one point's search (a
-// lane per word ran all of a word's searches one after the other: 374 us a
-// call at 301 vesicles of N = 64, 30 us like this).
+// py_hh correction.  Bit u of a pair (t, s) of the lists is the hedgehog point
+// of upsampled point u of s: read as (k2, J) with s Nup + u = k2 N + J it adds
+// the self velocity of t at the coarse point of t three before the closest one
+// to upsampled point J of k2.
+__device__ __forceinline__ bool hh_point(int nv, int N, int Nup, int t, int s, int u, int& k2, int& J) {
+  const int q = u / N;  // Nup is a multiple of N
+  k2 = s * (Nup / N) + q;
+  J = u - q * N;
+  return k2 < nv && k2 != t;
+}
+
+// What the pairs (t, s) with one hedgehog point have in common: how many
+// vesicles t there are (less one) and the first and last of them.  hits: three
+// arrays [nv][N], every byte 0xff before the first launch.
+__global__ void __launch_bounds__(128) hh_count_kernel(int nv, int N, int Nup, int maxc,
+                                                       const int* __restrict__ cand_count,
+                                                       const int* __restrict__ cand_src,
+                                                       const uint32_t* __restrict__ hh_mask, int* __restrict__ hits) {
+  const int t = blockIdx.x, wU = (Nup + 31) / 32;
+  const int nc = min(cand_count[t], maxc);
+  const size_t n = (size_t)nv * N;
+  for (int i = threadIdx.x; i < nc * wU; i += blockDim.x) {
+    const int slot = i / wU, w = i - slot * wU;
+    uint32_t bits = hh_mask[((long long)t * maxc + slot) * wU + w];
+    if (bits == 0u) continue;
+    const int s = cand_src[(long long)t * maxc + slot];
+    for (; bits; bits &= bits - 1) {
+      int k2, J;
+      if (!hh_point(nv, N, Nup, t, s, w * 32 + __ffs(bits) - 1, k2, J)) continue;
+      const size_t p = (size_t)k2 * N + J;
+      atomicAdd(&hits[p], 1);
+      atomicMin(reinterpret_cast<unsigned*>(hits) + n + p, (unsigned)t);
+      atomicMax(&hits[2 * n + p], t);
+    }
+  }
+}
+
+// the first vesicle from t0 on, up to t1 and without k2, that has hedgehog point u of s
+__device__ __forceinline__ int hh_next(int Nup, int maxc, const int* __restrict__ cand_count,
+                                       const int* __restrict__ cand_src, const uint32_t* __restrict__ hh_mask, int t0,
+                                       int t1, int k2, int s, int u, int lane) {
+  const int wU = (Nup + 31) / 32;
+  for (int b = t0; b <= t1; b += 32) {
+    const int t = b + lane;
+    bool bit = false;
+    if (t <= t1 && t != k2) {
+      const int* row = cand_src + (long long)t * maxc;
+      const int nc = min(cand_count[t], maxc);
+      int lo = 0, hi = nc;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (row[mid] < s) lo = mid + 1; else hi = mid;
+      }
+      bit = lo < nc && row[lo] == s && ((hh_mask[((long long)t * maxc + lo) * wU + (u >> 5)] >> (u & 31)) & 1u);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, bit);
+    if (m) return b + __ffs(m) - 1;
+  }
+  return t1 + 1;
+}
+
+// One CTA per vesicle t.  Latency-bound: a hedgehog point is a search of the N
+// coarse points (FP64 distances), and the points of a close pair sit side by
+// side, that is in one or two words of the mask.  So the warps take the set
+// bits in turn and the lanes share one point's search (30 us a call at 301
+// vesicles of N = 64).  A point that several vesicles add to is taken by the
+// warp of the first of them, which adds the others' values after its own in
+// ascending order: the sum does not depend on which CTA is first.
 __global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, int maxc, const double* __restrict__ X,
                                                        const double* __restrict__ Xup,
                                                        const int* __restrict__ cand_count,
                                                        const int* __restrict__ cand_src,
                                                        const uint32_t* __restrict__ hh_mask,
+                                                       const int* __restrict__ hits,
                                                        const double* __restrict__ vself, double* __restrict__ LP,
                                                        double* __restrict__ near_only) {
   extern __shared__ double xk[];  // [2][N] coarse points of t (k1 of every pair)
@@ -347,6 +410,35 @@ __global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, i
   for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) xk[i] = X[(long long)t * 2 * N + i];
   __syncthreads();
   const int wU = (Nup + 31) / 32;
+  const size_t n = (size_t)nv * N;
+  // the value of vesicle t1 (coarse points x) at upsampled point J of k2
+  auto add = [&](int t1, const double* x, int k2, int J, double px, double py) {
+    double best = 1e300;
+    int icp = 0x7fffffff;  // closest coarse point (first minimum)
+    for (int i = lane; i < N; i += 32) {
+      const double dx = x[i] - px, dy = x[N + i] - py;
+      const double d2 = dx * dx + dy * dy;
+      if (d2 < best) {
+        best = d2;
+        icp = i;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double d2 = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, icp, o);
+      if (d2 < best || (d2 == best && i2 < icp)) {
+        best = d2;
+        icp = i2;
+      }
+    }
+    if (icp == 0x7fffffff) icp = 0;  // no finite distance
+    const int pn0 = ((icp - 3) % N + N) % N;
+    if (lane < 2) {  // one component each
+      const double v = vself[(long long)t1 * 2 * N + lane * N + pn0];
+      atomicAdd(&LP[(long long)k2 * 2 * N + lane * N + J], v);
+      if (near_only) atomicAdd(&near_only[(long long)k2 * 2 * N + lane * N + J], v);
+    }
+  };
   int turn = 0;  // set bits so far: each belongs to one warp
   for (int slot = 0; slot < nc; ++slot) {
     const int s = cand_src[(long long)t * maxc + slot];
@@ -363,35 +455,17 @@ __global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, i
           bits &= bits - 1;
           if (turn++ % nw != warp) continue;
           const int u = (w0 + wl) * 32 + b;
-          const long long id1 = (long long)s * Nup + u;
-          const int k2 = (int)(id1 / N), J = (int)(id1 % N);
-          if (k2 >= nv || k2 == t) continue;
-          // closest coarse point of k1 to upsampled point J of vesicle k2 (first minimum)
+          int k2, J;
+          if (!hh_point(nv, N, Nup, t, s, u, k2, J)) continue;
+          const size_t p = (size_t)k2 * N + J;
+          const int more = hits[p], first = hits[n + p], last = hits[2 * n + p];
           const double px = Xup[(long long)k2 * 2 * Nup + J], py = Xup[(long long)k2 * 2 * Nup + Nup + J];
-          double best = 1e300;
-          int icp = 0x7fffffff;
-          for (int i = lane; i < N; i += 32) {
-            const double dx = xk[i] - px, dy = xk[N + i] - py;
-            const double d2 = dx * dx + dy * dy;
-            if (d2 < best) {
-              best = d2;
-              icp = i;
-            }
-          }
-          for (int o = 16; o > 0; o >>= 1) {
-            const double d2 = __shfl_xor_sync(0xffffffffu, best, o);
-            const int i2 = __shfl_xor_sync(0xffffffffu, icp, o);
-            if (d2 < best || (d2 == best && i2 < icp)) {
-              best = d2;
-              icp = i2;
-            }
-          }
-          if (icp == 0x7fffffff) icp = 0;  // no finite distance
-          const int pn0 = ((icp - 3) % N + N) % N;
-          if (lane < 2) {  // one component each
-            const double v = vself[(long long)t * 2 * N + lane * N + pn0];
-            atomicAdd(&LP[(long long)k2 * 2 * N + lane * N + J], v);
-            if (near_only) atomicAdd(&near_only[(long long)k2 * 2 * N + lane * N + J], v);
+          if (first != t) continue;
+          add(t, xk, k2, J, px, py);
+          int t1 = t;
+          for (int left = more; left > 0 && t1 < last; --left) {
+            t1 = left == 1 ? last : hh_next(Nup, maxc, cand_count, cand_src, hh_mask, t1 + 1, last, k2, s, u, lane);
+            add(t1, X + (long long)t1 * 2 * N, k2, J, px, py);
           }
         }
       }
@@ -833,7 +907,33 @@ void launch_matlab_correct(int np, const MatlabPair* pairs, cudaStream_t s) {
   matlab_correct_kernel<DL><<<(unsigned)ceil_div(P.warp0[np] * 32, 256), 256, 0, s>>>(P);
 }
 
+// The py_hh correction.  hits: hedgehog_hits of the lists, or null: made in
+// scratch (3 nv N ints).
+int launch_hedgehog(const ves_ctx* c, int nv, const double* X, const double* Xup, const double* vself,
+                    const ves_near_lists* nl, const int* hits, int* scratch, double* LP, double* near_only,
+                    cudaStream_t s) {
+  if (!hits) {
+    const int rc = hedgehog_hits(c, nv, nl, scratch, s);
+    if (rc) return rc;
+    hits = scratch;
+  }
+  ves_count_launch();
+  hh_apply_kernel<<<nv, 128, (size_t)2 * c->N * sizeof(double), s>>>(nv, c->N, c->Nup, nl->maxc, X, Xup,
+                                                                     nl->cand_count, nl->cand_src, nl->hh_mask, hits,
+                                                                     vself, LP, near_only);
+  return VES_OK;
+}
+
 }  // namespace
+
+int hedgehog_hits(const ves_ctx* c, int nv, const ves_near_lists* nl, int* hits, cudaStream_t s) {
+  if (nv <= 0) return VES_OK;
+  const int rc = ves_cuda_status(cudaMemsetAsync(hits, 0xff, (size_t)3 * nv * c->N * sizeof(int), s), "hedgehog hits");
+  if (rc) return rc;
+  ves_count_launch();
+  hh_count_kernel<<<nv, 128, 0, s>>>(nv, c->N, c->Nup, nl->maxc, nl->cand_count, nl->cand_src, nl->hh_mask, hits);
+  return ves_launch_check("hedgehog_hits");
+}
 
 int near_zone_py(ves_ctx* c, int nv, const double* X, const double* Xup_in, double thresh,
                  const ves_near_lists* nl, WsCarver& ws, cudaStream_t s) {
@@ -914,7 +1014,7 @@ int near_zone_matlab(ves_ctx* c, int nv, const double* X, double h, const ves_ne
 
 int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* sa_up,
                       const double* Xup, const double* f, const double* vself, const ves_near_lists* nl,
-                      double h, double* LP, double* near_only, WsCarver& ws, cudaStream_t s) {
+                      double h, double* LP, double* near_only, WsCarver& ws, cudaStream_t s, const int* hits) {
   const int N = c->N, Nup = c->Nup;
   double* fup = ws.take<double>((size_t)nv * 2 * Nup);
   double* den = ws.take<double>((size_t)nv * 2 * Nup);
@@ -955,9 +1055,7 @@ int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const doubl
     // nearSingInt_rbf: the far field above plus the fits of the near pairs
     if ((rc = rbf_near_correct(c, nv, X, f, vself, nl, LP, ws, s))) return rc;
   } else if (scheme == VES_NEAR_PY_HH) {
-    ves_count_launch();
-    hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
-                                                                    nl->cand_src, nl->hh_mask, vself, LP, near_only);
+    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, hits, (int*)fup, LP, near_only, s))) return rc;
   } else if (scheme == VES_NEAR_MATLAB) {
     const MatlabPair a = matlab_pair(c, c, X, Xup, nullptr, den, vself, nl, h, LP, near_only);
     launch_matlab_correct<false>(1, &a, s);
@@ -1072,7 +1170,7 @@ int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision,
 int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* Xup,
                          const double* tang_up, const double* sa_up, const double* visc, const double* f,
                          const double* vself, const ves_near_lists* nl, double h, double* LP, double* near_only,
-                         WsCarver& ws, cudaStream_t s) {
+                         WsCarver& ws, cudaStream_t s, const int* hits) {
   const int N = c->N, Nup = c->Nup;
   double* fup = ws.take<double>((size_t)nv * 2 * Nup);
   double* den = ws.take<double>((size_t)nv * 2 * Nup);
@@ -1109,9 +1207,7 @@ int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const do
                            s);
   if (rc) return rc;
   if (scheme == VES_NEAR_PY_HH) {
-    ves_count_launch();
-    hh_apply_kernel<<<nv, 128, (size_t)2 * N * sizeof(double), s>>>(nv, N, Nup, nl->maxc, X, Xup, nl->cand_count,
-                                                                    nl->cand_src, nl->hh_mask, vself, LP, near_only);
+    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, hits, (int*)fup, LP, near_only, s))) return rc;
   } else if (scheme == VES_NEAR_MATLAB) {
     const MatlabPair a = matlab_pair(c, c, X, Xup, tang_up, den, vself, nl, h, LP, near_only);
     launch_matlab_correct<true>(1, &a, s);

@@ -262,6 +262,7 @@ struct StepState {
   const double* visc;
   double *alpha, *D, *tang_up, *Xm, *DX, *vdl, *Fdl;
   ves_near_lists nl;
+  int* hits;  // hedgehog_hits of nl (py lists)
   double h;
   // matvec temporaries
   double *f, *Gf, *LP;
@@ -280,7 +281,7 @@ int matvec(StepState& S, const double* v, double* out) {
   launch_bgemv_f64(nv, 2 * N, 2 * N, S.G, S.f, 2LL * N, S.Gf, 2LL * N, S.s);
   WsCarver sub(S.scratch, S.scratch_bytes);
   int rc = near_sing_int_run(c, S.prm->near_scheme, S.prm->farfield_precision, nv, S.X, S.sa_up, S.Xup, S.f, S.Gf,
-                             &S.nl, S.h, S.LP, nullptr, sub, S.s);
+                             &S.nl, S.h, S.LP, nullptr, sub, S.s, S.hits);
   if (rc) return rc;
   if (S.visc) {
     // D Xm and the double layer of Xm (tstep_biem.py:489, 497-501)
@@ -293,7 +294,7 @@ int matvec(StepState& S, const double* v, double* out) {
     WsCarver sub2(S.scratch, S.scratch_bytes);
     if ((rc = near_sing_int_dl_run(c, S.dl_scheme, S.prm->farfield_precision, nv, S.X, S.Xup, S.tang_up, S.sa_up,
                                    S.visc, S.Xm, S.vdl, &S.nl,
-                                   S.h, S.Fdl, nullptr, sub2, S.s)))
+                                   S.h, S.Fdl, nullptr, sub2, S.s, S.hits)))
       return rc;
   }
   ves_count_launch();
@@ -710,6 +711,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   B.ydev = ws.take<double>(restart + 2);
   double* vinf = ws.take<double>((size_t)nv * 2 * N);
   double* rhs2 = ws.take<double>((size_t)nv * N);
+  S.hits = S.dl_scheme == VES_NEAR_PY_HH ? ws.take<int>((size_t)3 * nv * N) : nullptr;
   // one scratch region shared by the sub-stages
   size_t scratch = 0;
   {
@@ -817,6 +819,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   } else if (prm->near_scheme == VES_NEAR_PY_HH || prm->near_scheme == VES_NEAR_PY_RBF) {
     WsCarver sub(S.scratch, S.scratch_bytes);
     if ((rc = near_zone_py(c, nv, X, S.Xup, 0.0, &S.nl, sub, s))) goto done;
+    if ((prm->near_scheme == VES_NEAR_PY_HH || vc) && (rc = hedgehog_hits(c, nv, &S.nl, S.hits, s))) goto done;
   }
   // right-hand side [X + dt*vinf; surfaceDiv(X)], with the double layer of X
   // (Fdlp + D X, tstep_biem.py:231-244) and the repulsion when present
@@ -829,7 +832,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
     WsCarver sub(S.scratch, S.scratch_bytes);
     if ((rc = near_sing_int_dl_run(c, S.dl_scheme, prm->farfield_precision, nv, X, S.Xup, S.tang_up, S.sa_up, S.visc,
                                    X, S.vdl, &S.nl, S.h,
-                                   S.Fdl, nullptr, sub, s)))
+                                   S.Fdl, nullptr, sub, s, S.hits)))
       goto done;
   }
   if (prm->repulsion && nv > 1) {
