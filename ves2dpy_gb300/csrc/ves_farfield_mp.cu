@@ -511,6 +511,7 @@ __global__ void __launch_bounds__(WARPS * 32, S == 1 ? 5 : 16 / WARPS) mp_eval_k
           if (st + 1 < nstages) tc_mbar_wait(&bar[buf ^ 1], ((kst + 1) >> 1) & 1, nullptr, 0);
           break;
         }
+        __syncwarp();  // every lane's reads of the stage, ordered before lane 0's signal
         if (lane == 0) {
           __threadfence_block();
           if (atomicAdd(&done[buf], 1) == WARPS - 1) {
