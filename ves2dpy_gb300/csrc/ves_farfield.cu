@@ -548,8 +548,9 @@ struct FFPlan {
 
 constexpr long long kFFFill = 152 * 2;  // resident CTAs of the FP32 rule
 
+// room: bytes for the partial sums
 template <typename Real>
-FFPlan ff_plan(int nsrc, int ns, long long total_pts) {
+FFPlan ff_plan(int nsrc, int ns, long long total_pts, size_t room = ~(size_t)0) {
   FFPlan pl;
   const size_t rec = sizeof(typename FFT<Real>::Rec);
   const size_t stage_budget = sizeof(Real) == 4 ? 24 * 1024 : 48 * 1024;
@@ -569,9 +570,15 @@ FFPlan ff_plan(int nsrc, int ns, long long total_pts) {
     // vesicles as fill the chip once, down to one.  One sum with its
     // preparation: 16 x N=32 387 -> 83 us, 40 x N=16 344 -> 82, 12 x N=128 381 ->
     // 229, 100 x N=32 389 -> 131; from one filled chip on (61 x N=128) the plan
-    // and its sum are what they were.
-    per = (int)std::max(1LL, ((long long)nsrc * pl.tgt_blocks + kFFFill - 1) / kFFFill);
-    pl.sv_per_stage = std::min(pl.sv_per_stage, per);
+    // and its sum are what they were.  More splits take more scratch: where a
+    // caller's buffer does not hold it, the plan of whole stages stays.
+    const int few = (int)std::max(1LL, ((long long)nsrc * pl.tgt_blocks + kFFFill - 1) / kFFFill);
+    const int stage = std::min(pl.sv_per_stage, few), split = (few + stage - 1) / stage * stage;
+    const long long splits = ((long long)nsrc + split - 1) / split;
+    if ((size_t)splits * total_pts * 2 * sizeof(double) <= room) {
+      per = few;
+      pl.sv_per_stage = stage;
+    }
   }
   per = ((per + pl.sv_per_stage - 1) / pl.sv_per_stage) * pl.sv_per_stage;
   pl.src_per_split = per > 0 ? per : 1;
@@ -588,7 +595,6 @@ int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double*
   typedef typename FFT<Real>::Rec Rec;
   typedef typename FFT<Real>::Pair Pair;
   const long long total_pts = (long long)nt * ntp;
-  const FFPlan pl = ff_plan<Real>(nsrc, ns, total_pts);
   Rec* rec = ws.take<Rec>((size_t)nsrc * ns);
   Pair* shi = ws.take<Pair>(nsrc);
   Pair* slo = ws.take<Pair>(nsrc);
@@ -596,6 +602,7 @@ int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double*
   Pair* tloc = ws.take<Pair>((size_t)total_pts);
   Pair* thi = ws.take<Pair>(nt);
   Pair* tlo = ws.take<Pair>(nt);
+  const FFPlan pl = ff_plan<Real>(nsrc, ns, total_pts, ws.left());
   double* partial = ws.take<double>((size_t)pl.nsplit * total_pts * 2);
   if (ws.sizing) return VES_OK;
   if (!ws.ok()) {

@@ -84,6 +84,11 @@ struct WsCarver {
     return p;
   }
   bool ok() const { return sizing || off <= cap; }
+  // bytes that the next take can have (all there are when sizing)
+  size_t left() const {
+    const size_t o = (off + 255) & ~(size_t)255;
+    return sizing ? ~(size_t)0 : (cap > o ? cap - o : 0);
+  }
 };
 
 // launchers (implemented in the .cu files) ------------------------------------
