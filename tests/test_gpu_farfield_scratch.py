@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
 
 
-@pytest.mark.parametrize("precision", ["fp32c"])
+@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
 @pytest.mark.parametrize("nsrc,ns,most,ntp", [(16, 192, 640, 32), (40, 64, 40, 16), (33, 96, 130, 48)])
 def test_smaller_calls_fit_the_largest_call_s_buffer(nsrc, ns, most, ntp, precision):
     from ves2dpy_gb300 import _native as nat

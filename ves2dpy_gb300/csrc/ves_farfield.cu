@@ -664,24 +664,21 @@ struct FF64Plan {
 
 // Pieces of at least 16 points (below that the per-piece centre terms, one
 // log and one divide, are over a tenth of the work), as many splits as give
-// 16 CTAs of 4 warps per SM (two rounds of resident CTAs).  The partial sums
-// fit in what the staged plan of whole vesicles took, or in 32 MiB with the
-// records: a caller's fixed scratch holds every size that it held.
-FF64Plan ff64_plan(int nsrc, int ns, long long total_pts) {
+// 16 CTAs of 4 warps per SM (two rounds of resident CTAs), as far as their
+// partial sums fit in ``room`` bytes.  A buffer that holds one split serves.
+FF64Plan ff64_plan(int nsrc, int ns, long long total_pts, size_t room) {
   FF64Plan pl;
   const long long tb = (total_pts + FF64_THREADS - 1) / FF64_THREADS;
   pl.tgt_blocks = (int)tb;
-  long long want = tb > 0 ? (152LL * 16 + tb - 1) / tb : 1;
-  const long long held = ff_plan<double>(nsrc, ns, total_pts).nsplit;
-  const long long base = (long long)nsrc * ns * (long long)sizeof(Rec64), room = (32LL << 20) - base;
-  const long long fit = total_pts > 0 && room > 0 ? room / (total_pts * 16) : 0;
-  want = std::max(1LL, std::min(want, std::max(held, fit)));
+  const long long want = tb > 0 ? (152LL * 16 + tb - 1) / tb : 1;
+  const long long per = std::max(1LL, total_pts) * 2 * (long long)sizeof(double);
+  const long long splits = (long long)std::max<size_t>(1, std::min((size_t)want, room / (size_t)per));
   const long long most = std::max(1, ns / 16);
-  pl.nchunk = (int)std::max(1LL, std::min(most, nsrc > 0 ? (want + nsrc - 1) / nsrc : 1));
+  pl.nchunk = (int)std::max(1LL, std::min(most, nsrc > 0 ? (splits + nsrc - 1) / nsrc : 1));
   pl.chunk = (ns + pl.nchunk - 1) / pl.nchunk;
   pl.nchunk = (ns + pl.chunk - 1) / pl.chunk;
   const long long units = (long long)nsrc * pl.nchunk;
-  pl.per_split = (int)std::max(1LL, (units + want - 1) / want);
+  pl.per_split = (int)std::max(1LL, (units + splits - 1) / splits);
   pl.nsplit = (int)std::max(1LL, (units + pl.per_split - 1) / pl.per_split);
   return pl;
 }
@@ -690,7 +687,6 @@ int ff64_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const doubl
              const double* Xtar, const int* self_idx, const ves_near_lists* nl, double* out, WsCarver& ws,
              cudaStream_t s) {
   const long long total_pts = (long long)nt * ntp;
-  const FF64Plan pl = ff64_plan(nsrc, ns, total_pts);
   Rec64* rec = ws.take<Rec64>((size_t)nsrc * ns);
   double2* shi = ws.take<double2>(nsrc);
   double2* slo = ws.take<double2>(nsrc);
@@ -698,6 +694,7 @@ int ff64_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const doubl
   double2* tloc = ws.take<double2>((size_t)total_pts);
   double2* thi = ws.take<double2>(nt);
   double2* tlo = ws.take<double2>(nt);
+  const FF64Plan pl = ff64_plan(nsrc, ns, total_pts, ws.left());
   double* partial = ws.take<double>((size_t)pl.nsplit * total_pts * 2);
   if (ws.sizing) return VES_OK;
   if (!ws.ok()) {
