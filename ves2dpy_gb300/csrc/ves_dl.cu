@@ -969,10 +969,6 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
   return dl_mp_start<8, 8>(a, units, s);
 }
 
-int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const double* tang, const double* den,
-                       const double* sa, const double* visc, int nt, int ntp, const double* Xtar,
-                       const int* self_idx, const ves_near_lists* nl, double* out, WsCarver& ws, cudaStream_t s);
-
 int farfield_dl_run(ves_ctx* c, int precision, int nsrc, int ns, const double* Xsrc, const double* tang,
                     const double* den, const double* sa, const double* visc, int nt, int ntp, const double* Xtar,
                     const int* self_idx, const ves_near_lists* nl, double* out, WsCarver& ws, cudaStream_t s) {

@@ -31,9 +31,6 @@
 
 namespace {
 
-#ifndef VES_FF_PAIRED_RCP
-#define VES_FF_PAIRED_RCP 0
-#endif
 #ifndef VES_FF_MINB
 #define VES_FF_MINB 2  // resident CTAs per SM requested from the register allocator
 #endif
@@ -47,14 +44,13 @@ struct __align__(32) Rec64 {
   double x, y, z, w;  // local x, local y, den x, den y (float4 field names)
 };
 
+// records and pairs of the two rules
 template <typename Real>
 struct FFT;
 template <>
 struct FFT<float> {
   typedef float4 Rec;  // x, y (local), denx, deny
   typedef float2 Pair;
-  static __device__ __forceinline__ float rcp(float x) { return mufu_rcp(x); }
-  static __device__ __forceinline__ float lg2(float x) { return mufu_lg2(x); }
   static __device__ __forceinline__ Rec rec(float x, float y, float a, float b) { return make_float4(x, y, a, b); }
   static __device__ __forceinline__ Pair pair(float a, float b) { return make_float2(a, b); }
 };
@@ -106,17 +102,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned phase,
   return false;
 }
 
-template <typename Real>
 struct FFArgs {
   int nsrc, ns, nt, ntp;
   long long total_pts;
-  const typename FFT<Real>::Rec* src;
-  const typename FFT<Real>::Pair* src_hi;   // centre, high part
-  const typename FFT<Real>::Pair* src_lo;   // centre, low part (0 in FP64)
-  const typename FFT<Real>::Pair* src_dsum; // sum of den over the vesicle
-  const typename FFT<Real>::Pair* tgt_local;
-  const typename FFT<Real>::Pair* tgt_hi;
-  const typename FFT<Real>::Pair* tgt_lo;
+  const float4* src;
+  const float2* src_hi;   // centre, high part
+  const float2* src_lo;   // centre, low part
+  const float2* src_dsum; // sum of den over the vesicle
+  const float2* tgt_local;
+  const float2* tgt_hi;
+  const float2* tgt_lo;
   const int* self_idx;
   const int* cand_count;
   const int* cand_src;
@@ -186,15 +181,12 @@ __global__ void __launch_bounds__(256) ff_prep_kernel(int n, const double* __res
 }
 
 // --------------------------------------------------------------------------
-template <typename Real>
-__global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFArgs<Real> p) {
-  typedef typename FFT<Real>::Rec Rec;
-  typedef typename FFT<Real>::Pair Pair;
+__global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFArgs p) {
   extern __shared__ __align__(128) unsigned char ff_smem[];
   __shared__ __align__(8) uint64_t bars[2];
   const int stage_elems = p.sv_per_stage * p.ns;
-  Rec* buf0 = reinterpret_cast<Rec*>(ff_smem);
-  Rec* buf1 = buf0 + stage_elems;
+  float4* buf0 = reinterpret_cast<float4*>(ff_smem);
+  float4* buf1 = buf0 + stage_elems;
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int split = blockIdx.y;
@@ -205,8 +197,8 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
   long long pt[FF_TPL];
   int col[FF_TPL], pidx[FF_TPL], self[FF_TPL], cur[FF_TPL], cend[FF_TPL];
   bool valid[FF_TPL];
-  Pair tl[FF_TPL], thi[FF_TPL], tlo[FF_TPL];
-  Real tot_x[FF_TPL], tot_y[FF_TPL], cmp_x[FF_TPL], cmp_y[FF_TPL];
+  float2 tl[FF_TPL], thi[FF_TPL], tlo[FF_TPL];
+  float tot_x[FF_TPL], tot_y[FF_TPL], cmp_x[FF_TPL], cmp_y[FF_TPL];
 #pragma unroll
   for (int q = 0; q < FF_TPL; ++q) {
     pt[q] = ((long long)blockIdx.x * FF_WARPS + warp) * FF_PTS_PER_WARP + q * 32 + lane;
@@ -220,7 +212,7 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
     tlo[q] = p.tgt_lo[col[q]];
     cur[q] = 0;
     cend[q] = p.cand_count ? min(p.cand_count[col[q]], p.maxc) : 0;
-    tot_x[q] = tot_y[q] = cmp_x[q] = cmp_y[q] = Real(0);
+    tot_x[q] = tot_y[q] = cmp_x[q] = cmp_y[q] = 0.f;
   }
 
   const int nstages = (s_end > s_begin) ? (s_end - s_begin + p.sv_per_stage - 1) / p.sv_per_stage : 0;
@@ -234,7 +226,7 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
     for (int st = 0; st < 2 && st < nstages; ++st) {
       const int v0 = s_begin + st * p.sv_per_stage;
       const int nvs = min(p.sv_per_stage, s_end - v0);
-      const unsigned bytes = (unsigned)((size_t)nvs * p.ns * sizeof(Rec));
+      const unsigned bytes = (unsigned)((size_t)nvs * p.ns * sizeof(float4));
       mbar_arrive_expect_tx(&bars[st], bytes);
       bulk_g2s(st ? buf1 : buf0, p.src + (long long)v0 * p.ns, bytes, &bars[st]);
     }
@@ -244,70 +236,38 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
   for (int st = 0; st < nstages; ++st) {
     const unsigned phase = (st >> 1) & 1;
     if (!mbar_wait_bounded(&bars[st & 1], phase, p.st, 10)) break;
-    const Rec* S = (st & 1) ? buf1 : buf0;
+    const float4* S = (st & 1) ? buf1 : buf0;
     const int v0 = s_begin + st * p.sv_per_stage;
     const int nvs = min(p.sv_per_stage, s_end - v0);
     for (int v = 0; v < nvs; ++v) {
       const int s = v0 + v;
-      const Pair shi = p.src_hi[s], slo = p.src_lo[s], dsum = p.src_dsum[s];
-      Real tx[FF_TPL], ty[FF_TPL], irc2[FF_TPL];
-      Real acx[FF_TPL], acy[FF_TPL], alx[FF_TPL], aly[FF_TPL];
+      const float2 shi = p.src_hi[s], slo = p.src_lo[s], dsum = p.src_dsum[s];
+      float tx[FF_TPL], ty[FF_TPL], irc2[FF_TPL];
+      float acx[FF_TPL], acy[FF_TPL], alx[FF_TPL], aly[FF_TPL];
 #pragma unroll
       for (int q = 0; q < FF_TPL; ++q) {
-        const Real ox = (thi[q].x - shi.x) + (tlo[q].x - slo.x);
-        const Real oy = (thi[q].y - shi.y) + (tlo[q].y - slo.y);
+        const float ox = (thi[q].x - shi.x) + (tlo[q].x - slo.x);
+        const float oy = (thi[q].y - shi.y) + (tlo[q].y - slo.y);
         tx[q] = tl[q].x + ox;
         ty[q] = tl[q].y + oy;
-        irc2[q] = FFT<Real>::rcp(tx[q] * tx[q] + ty[q] * ty[q]);
-        acx[q] = acy[q] = alx[q] = aly[q] = Real(0);
+        irc2[q] = mufu_rcp(tx[q] * tx[q] + ty[q] * ty[q]);
+        acx[q] = acy[q] = alx[q] = aly[q] = 0.f;
       }
-      const Rec* Sv = S + v * p.ns;
-      if (sizeof(Real) == 4 && VES_FF_PAIRED_RCP) {
-        // One MUFU reciprocal per two target slots: 1/a = b * rcp(a*b).  The
-        // 1e-20 inside the FMA keeps a*b normal when a slot coincides with a
-        // source (its own vesicle, whose result is discarded) and is below one
-        // ulp of every separated pair's |r|^2.
+      const float4* Sv = S + v * p.ns;
 #pragma unroll 2
-        for (int j = 0; j < p.ns; ++j) {
-          const Rec r = Sv[j];
+      for (int j = 0; j < p.ns; ++j) {
+        const float4 r = Sv[j];
 #pragma unroll
-          for (int q = 0; q < FF_TPL; q += 2) {
-            const Real dx0 = tx[q] - r.x, dy0 = ty[q] - r.y;
-            const Real dx1 = tx[q + 1] - r.x, dy1 = ty[q + 1] - r.y;
-            const Real r20 = fma(dx0, dx0, fma(dy0, dy0, Real(1e-20)));
-            const Real r21 = fma(dx1, dx1, fma(dy1, dy1, Real(1e-20)));
-            const Real ip = FFT<Real>::rcp(r20 * r21);
-            const Real inv0 = r21 * ip, inv1 = r20 * ip;
-            const Real lg0 = FFT<Real>::lg2(r20 * irc2[q]);
-            const Real lg1 = FFT<Real>::lg2(r21 * irc2[q + 1]);
-            const Real cc0 = fma(dx0, r.z, dy0 * r.w) * inv0;
-            const Real cc1 = fma(dx1, r.z, dy1 * r.w) * inv1;
-            acx[q] = fma(cc0, dx0, acx[q]);
-            acy[q] = fma(cc0, dy0, acy[q]);
-            alx[q] = fma(lg0, r.z, alx[q]);
-            aly[q] = fma(lg0, r.w, aly[q]);
-            acx[q + 1] = fma(cc1, dx1, acx[q + 1]);
-            acy[q + 1] = fma(cc1, dy1, acy[q + 1]);
-            alx[q + 1] = fma(lg1, r.z, alx[q + 1]);
-            aly[q + 1] = fma(lg1, r.w, aly[q + 1]);
-          }
-        }
-      } else {
-#pragma unroll 2
-        for (int j = 0; j < p.ns; ++j) {
-          const Rec r = Sv[j];
-#pragma unroll
-          for (int q = 0; q < FF_TPL; ++q) {
-            const Real dx = tx[q] - r.x, dy = ty[q] - r.y;
-            const Real r2 = fma(dx, dx, dy * dy);
-            const Real inv = FFT<Real>::rcp(r2);
-            const Real lg = FFT<Real>::lg2(r2 * irc2[q]);
-            const Real cc = fma(dx, r.z, dy * r.w) * inv;
-            acx[q] = fma(cc, dx, acx[q]);
-            acy[q] = fma(cc, dy, acy[q]);
-            alx[q] = fma(lg, r.z, alx[q]);
-            aly[q] = fma(lg, r.w, aly[q]);
-          }
+        for (int q = 0; q < FF_TPL; ++q) {
+          const float dx = tx[q] - r.x, dy = ty[q] - r.y;
+          const float r2 = fma(dx, dx, dy * dy);
+          const float inv = mufu_rcp(r2);
+          const float lg = mufu_lg2(r2 * irc2[q]);
+          const float cc = fma(dx, r.z, dy * r.w) * inv;
+          acx[q] = fma(cc, dx, acx[q]);
+          acy[q] = fma(cc, dy, acy[q]);
+          alx[q] = fma(lg, r.z, alx[q]);
+          aly[q] = fma(lg, r.w, aly[q]);
         }
       }
 #pragma unroll
@@ -323,11 +283,11 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
           }
         }
         if (valid[q] && s != self[q] && !excl) {
-          const Real lgc = FFT<Real>::lg2(tx[q] * tx[q] + ty[q] * ty[q]);
-          const Real px = acx[q] - Real(FF_HALF_LN2) * fma(lgc, dsum.x, alx[q]);
-          const Real py = acy[q] - Real(FF_HALF_LN2) * fma(lgc, dsum.y, aly[q]);
+          const float lgc = mufu_lg2(tx[q] * tx[q] + ty[q] * ty[q]);
+          const float px = acx[q] - (float)FF_HALF_LN2 * fma(lgc, dsum.x, alx[q]);
+          const float py = acy[q] - (float)FF_HALF_LN2 * fma(lgc, dsum.y, aly[q]);
           // Kahan-Babuska (Neumaier) compensated accumulation
-          Real t = tot_x[q] + px;
+          float t = tot_x[q] + px;
           cmp_x[q] += (fabs(tot_x[q]) >= fabs(px)) ? (tot_x[q] - t) + px : (px - t) + tot_x[q];
           tot_x[q] = t;
           t = tot_y[q] + py;
@@ -341,7 +301,7 @@ __global__ void __launch_bounds__(FF_WARPS * 32, VES_FF_MINB) ff_main_kernel(FFA
       const int sn = issued;
       const int v0n = s_begin + sn * p.sv_per_stage;
       const int nvn = min(p.sv_per_stage, s_end - v0n);
-      const unsigned bytes = (unsigned)((size_t)nvn * p.ns * sizeof(Rec));
+      const unsigned bytes = (unsigned)((size_t)nvn * p.ns * sizeof(float4));
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_arrive_expect_tx(&bars[sn & 1], bytes);
       bulk_g2s((sn & 1) ? buf1 : buf0, p.src + (long long)v0n * p.ns, bytes, &bars[sn & 1]);
@@ -549,23 +509,22 @@ struct FFPlan {
 constexpr long long kFFFill = 152 * 2;  // resident CTAs of the FP32 rule
 
 // room: bytes for the partial sums
-template <typename Real>
-FFPlan ff_plan(int nsrc, int ns, long long total_pts, size_t room = ~(size_t)0) {
+FFPlan ff_plan(int nsrc, int ns, long long total_pts, size_t room) {
   FFPlan pl;
-  const size_t rec = sizeof(typename FFT<Real>::Rec);
-  const size_t stage_budget = sizeof(Real) == 4 ? 24 * 1024 : 48 * 1024;
+  const size_t rec = sizeof(float4);
+  const size_t stage_budget = 24 * 1024;
   pl.sv_per_stage = (int)(stage_budget / (rec * (size_t)ns));
   if (pl.sv_per_stage < 1) pl.sv_per_stage = 1;
   if (pl.sv_per_stage > nsrc) pl.sv_per_stage = nsrc > 0 ? nsrc : 1;
   pl.tgt_blocks = (int)((total_pts + FF_PTS_PER_CTA - 1) / FF_PTS_PER_CTA);
   // aim for >= 8 waves of 152 SMs x 2 CTAs, but keep >= 2 stages per split
   const long long want = 152LL * 2 * 8;
-  int nsplit = (int)((want + pl.tgt_blocks - 1) / pl.tgt_blocks);
+  int nsplit = pl.tgt_blocks > 0 ? (int)((want + pl.tgt_blocks - 1) / pl.tgt_blocks) : 1;
   const int max_split = (nsrc + 2 * pl.sv_per_stage - 1) / (2 * pl.sv_per_stage);
   if (nsplit > max_split) nsplit = max_split;
   if (nsplit < 1) nsplit = 1;
   int per = (nsrc + nsplit - 1) / nsplit;
-  if (sizeof(Real) == 4 && (long long)pl.tgt_blocks * nsplit < kFFFill) {
+  if ((long long)pl.tgt_blocks * nsplit < kFFFill) {
     // Too few CTAs with two whole stages per split: stages and splits of as few
     // vesicles as fill the chip once, down to one.  One sum with its
     // preparation: 16 x N=32 387 -> 83 us, 40 x N=16 344 -> 82, 12 x N=128 381 ->
@@ -588,21 +547,18 @@ FFPlan ff_plan(int nsrc, int ns, long long total_pts, size_t room = ~(size_t)0) 
   return pl;
 }
 
-template <typename Real>
 int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double* den, int nt, int ntp,
            const double* Xtar, const int* self_idx, const ves_near_lists* nl, double* out, WsCarver& ws,
            cudaStream_t s) {
-  typedef typename FFT<Real>::Rec Rec;
-  typedef typename FFT<Real>::Pair Pair;
   const long long total_pts = (long long)nt * ntp;
-  Rec* rec = ws.take<Rec>((size_t)nsrc * ns);
-  Pair* shi = ws.take<Pair>(nsrc);
-  Pair* slo = ws.take<Pair>(nsrc);
-  Pair* dsum = ws.take<Pair>(nsrc);
-  Pair* tloc = ws.take<Pair>((size_t)total_pts);
-  Pair* thi = ws.take<Pair>(nt);
-  Pair* tlo = ws.take<Pair>(nt);
-  const FFPlan pl = ff_plan<Real>(nsrc, ns, total_pts, ws.left());
+  float4* rec = ws.take<float4>((size_t)nsrc * ns);
+  float2* shi = ws.take<float2>(nsrc);
+  float2* slo = ws.take<float2>(nsrc);
+  float2* dsum = ws.take<float2>(nsrc);
+  float2* tloc = ws.take<float2>((size_t)total_pts);
+  float2* thi = ws.take<float2>(nt);
+  float2* tlo = ws.take<float2>(nt);
+  const FFPlan pl = ff_plan(nsrc, ns, total_pts, ws.left());
   double* partial = ws.take<double>((size_t)pl.nsplit * total_pts * 2);
   if (ws.sizing) return VES_OK;
   if (!ws.ok()) {
@@ -616,10 +572,10 @@ int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double*
     return VES_ERR_SHAPE;
   }
   ves_count_launch();
-  ff_prep_kernel<Real><<<nsrc, 256, 0, s>>>(ns, Xsrc, den, rec, nullptr, shi, slo, dsum);
+  ff_prep_kernel<float><<<nsrc, 256, 0, s>>>(ns, Xsrc, den, rec, nullptr, shi, slo, dsum);
   ves_count_launch();
-  ff_prep_kernel<Real><<<nt, 256, 0, s>>>(ntp, Xtar, nullptr, nullptr, tloc, thi, tlo, nullptr);
-  FFArgs<Real> a;
+  ff_prep_kernel<float><<<nt, 256, 0, s>>>(ntp, Xtar, nullptr, nullptr, tloc, thi, tlo, nullptr);
+  FFArgs a;
   a.nsrc = nsrc;
   a.ns = ns;
   a.nt = nt;
@@ -644,14 +600,14 @@ int ff_run(const FFEnv& env, int nsrc, int ns, const double* Xsrc, const double*
   a.partial = partial;
   a.st = env.status;
   if (pl.smem > 32 * 1024) {  // dynamic + static shared memory must fit the opt-in limit
-    cudaError_t e = cudaFuncSetAttribute(ff_main_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(ff_main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)pl.smem);
     if (e != cudaSuccess) return ves_cuda_status(e, "farfield smem attribute");
   }
   dim3 grid(pl.tgt_blocks, pl.nsplit);
   ves_count_launch();
   if (env.timing) ves_ff_timing_begin(env.timing, s);
-  ff_main_kernel<Real><<<grid, FF_WARPS * 32, pl.smem, s>>>(a);
+  ff_main_kernel<<<grid, FF_WARPS * 32, pl.smem, s>>>(a);
   if (env.timing) ves_ff_timing_end(env.timing, s, (double)total_pts * ns * (double)nsrc);
   ves_count_launch();
   ff_reduce_kernel<<<ceil_div(total_pts, 256), 256, 0, s>>>(total_pts, ntp, pl.nsplit, partial, out);
@@ -748,7 +704,7 @@ int farfield_run_env(const FFEnv& env, int precision, int nsrc, int ns, const do
   if (precision == VES_PREC_FP64)
     return ff64_run(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
   if (precision == VES_PREC_FP32C)
-    return ff_run<float>(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
+    return ff_run(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
   if (precision == VES_PREC_FP32M)
     return farfield_mp_run(env, nsrc, ns, Xsrc, den, nt, ntp, Xtar, self_idx, nl, out, ws, s);
   ves_record_error(VES_ERR_ARG, "farfield: bad precision %d", precision);

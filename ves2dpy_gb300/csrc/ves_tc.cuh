@@ -140,21 +140,6 @@ __device__ __forceinline__ bool tc_elect() {
   return r != 0;
 }
 
-// 8 consecutive FP32 columns of this thread's TMEM lane (lane = 32*(warp%4) +
-// laneid), with the wait for the load in the same statement so that no use of
-// the registers can be scheduled before the data has arrived.
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-      "tcgen05.wait::ld.sync.aligned;\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Store 32 consecutive FP32 columns of this thread's lane; complete with
 // tc_wait_st before the columns are used by an MMA.
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const float* v) {
