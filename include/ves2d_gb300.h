@@ -509,7 +509,8 @@ VES_API size_t ves_isolated_step_workspace(ves_ctx* ctx, int nv, int sl_precisio
  * order conv1_1.{weight,bias}, conv1_2, conv2_1, conv2_2, deconv1, deconv2,
  * mix, then bn1..bn4.{weight, bias, running_mean, running_var} (the state-dict
  * names of the reference modules); batch norm is trained as its
- * evaluation-mode affine map (running statistics fixed). */
+ * evaluation-mode affine map (running statistics fixed).  length: a multiple of
+ * 4, 12 or more (the convolutions pad rows of length / 2 points by 6). */
 typedef struct ves_trainer ves_trainer;
 VES_API int ves_trainer_create(int precision, int length, int nblocks, const ves_net_block* blocks,
                                const float* const* params, int max_batch, ves_trainer** out);

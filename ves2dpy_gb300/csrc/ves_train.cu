@@ -479,9 +479,10 @@ __global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(int B, int spc, in
   for (int b = b0; b < b1; ++b) {
     __syncthreads();
     for (int i = threadIdx.x; i < cin * row; i += blockDim.x) {
-      int q = HALO ? i % row - pad : i % row;
+      const int at = i % row;
+      int q = HALO ? at - pad : at;
       q = q < 0 ? q + L : (q >= L ? q - L : q);
-      sx[i] = x[((long long)b * cin + i / row) * L + q];
+      if (!HALO || at < row - 1) sx[i] = x[((long long)b * cin + i / row) * L + q];  // the last place only spaces rows
     }
     for (int i = threadIdx.x; i < cout * Lo; i += blockDim.x) sg[i] = dZ[((long long)b * ztot + zoff) * Lo + i];
     __syncthreads();
@@ -971,6 +972,13 @@ extern "C" int ves_trainer_create(int precision, int L, int nblocks, const ves_n
     return VES_ERR_ARG;
   }
   *out = nullptr;
+  if (L < 12) {
+    // circular padding of 6 (the dilated convolutions) around rows of L and of
+    // L / 2 points: a row shorter than the padding would wrap more than once
+    ves_record_error(VES_ERR_SHAPE, "trainer_create: rows of %d points are shorter than the circular padding allows (12)",
+                     L);
+    return VES_ERR_SHAPE;
+  }
   for (int i = 0; i < nblocks; ++i) {
     const ves_net_block& b = blocks[i];
     if (b.cin <= 0 || b.c1 <= 0 || b.c2 <= 0 || b.cmix <= 0 || b.npass < 0 || b.npass > b.cin ||
