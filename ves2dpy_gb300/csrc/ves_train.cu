@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kThreads) conv_fwd_kernel(int B, int spg, int 
                                                             const Real* __restrict__ W, const Real* __restrict__ bias,
                                                             const Real* __restrict__ x, int ctot, int coff,
                                                             Real* __restrict__ out) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;            // [kOT][cin][7]
   Real* sx = sw + kOT * cin * 7;      // [cin][L]
   const int o0 = blockIdx.x * kOT, no = min(kOT, cout - o0);
@@ -123,12 +123,13 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads) deconv_fwd_kernel(int B, int spg, int d, int Lin, const Real* __restrict__ W,
                                                               const Real* __restrict__ bias, const Real* __restrict__ x,
                                                               Real* __restrict__ out) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;          // [d][kOT][10]
   Real* sx = sw + d * kOT * 10;     // [d][Lin + 4], input i at i + 2
   const int o0 = blockIdx.x * kOT, no = min(kOT, d - o0);
   const int Lp = Lin + 4, Lo = 2 * Lin;
   const int nmb = (Lin + kR - 1) / kR;
+  static_assert(kOT * 10 * sizeof(float) % 16 == 0, "rows of inputs follow the weights on 16 bytes");
   const bool vec = Lin % 4 == 0;  // rows start on 16 bytes and end with their last block
   for (int c = threadIdx.x / 32; c < d; c += kThreads / 32)  // a warp per row of weights
     for (int r = threadIdx.x % 32; r < no * 10; r += 32) sw[c * kOT * 10 + r] = W[((long long)c * d + o0) * 10 + r];
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(kThreads) mix_fwd_kernel(int B, int spg, int d
                                                            int residual, const Real* __restrict__ W,
                                                            const Real* __restrict__ bias, const Real* __restrict__ D,
                                                            const Real* __restrict__ x0, Real* __restrict__ out) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;        // [kOT][d][3]
   Real* sd = sw + kOT * d * 3;    // [d][L]
   const int o0 = blockIdx.x * kOT, no = min(kOT, cmix - o0);
@@ -286,7 +287,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads) mix_bwd_data_kernel(int B, int spg, int d, int L, int cmix, int cout,
                                                                 const Real* __restrict__ W,
                                                                 const Real* __restrict__ dout, Real* __restrict__ dD) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;        // [cmix][kOT][3]
   Real* sg = sw + cmix * kOT * 3; // [cmix][L]
   const int c0 = blockIdx.x * kOT, nc = min(kOT, d - c0);
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(kThreads) deconv_bwd_data_kernel(int B, int sp
                                                                    const Real* __restrict__ W,
                                                                    const Real* __restrict__ dZ,
                                                                    Real* __restrict__ dIn) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;          // [kOT][d][10]
   Real* sg = sw + kOT * d * 10;     // [2][d][Lin + 4]: parity, channel, m + 2
   const int c0 = blockIdx.x * kOT, nc = min(kOT, d - c0);
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(kThreads) conv_bwd_data_kernel(int B, int spg,
                                                                  int pad, const Real* __restrict__ W, int ztot, int zoff,
                                                                  const Real* __restrict__ dZ, int accumulate,
                                                                  Real* __restrict__ dIn) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sw = (Real*)smraw;          // [cout][kOT][7]
   Real* sg = sw + cout * kOT * 7;   // [cout][L/2]
   const int c0 = blockIdx.x * kOT, nc = min(kOT, cin - c0);
@@ -465,7 +466,7 @@ template <typename Real, int DIL, bool HALO>
 __global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(int B, int spc, int cin, int L, int cout, int pad,
                                                               const Real* __restrict__ x, int ztot, int zoff,
                                                               const Real* __restrict__ dZ, Real* __restrict__ dW) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int Lo = L / 2, row = HALO ? wgrad_row(L, DIL) : L;
   Real* sx = (Real*)smraw;    // [cin][row], input q at q + pad (circular)
   Real* sg = sx + cin * row;  // [cout][L/2]
@@ -503,7 +504,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kWT * kWT) deconv_wgrad_kernel(int B, int spc, int d, int Lin,
                                                                  const Real* __restrict__ x,
                                                                  const Real* __restrict__ dZ, Real* __restrict__ dW) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int Lo = 2 * Lin, Lg = Lo + 10;
   Real* sx = (Real*)smraw;          // [kWT][Lin]
   Real* sg = sx + kWT * Lin;        // [kWT][Lo + 10], dZ j at j + 4
@@ -556,7 +557,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads) mix_wgrad_kernel(int B, int spc, int d, int L, int cmix, int cout,
                                                              const Real* __restrict__ D, const Real* __restrict__ dout,
                                                              Real* __restrict__ dW) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   Real* sx = (Real*)smraw;  // [d][L]
   Real* sg = sx + d * L;    // [cmix][L]
   const int ncoef = cmix * d * 3;
