@@ -224,13 +224,15 @@ VES_API int ves_dl_density(int nv, int ns, const double* f, const double* sa, co
  * precision VES_PREC_FP64: direct FP64 sum (ntp <= 1024, no workspace);
  * VES_PREC_FP32M (or FP32C): multipole series of each source vesicle for the
  * separated pairs, direct FP64 for the others (ntp <= 128; needs the source
- * jacobian sa[nsrc][ns] and contrasts visc[nsrc] of the density, and the
- * workspace of ves_farfield_dl_workspace). */
+ * jacobian sa[nsrc][ns] and contrasts visc[nsrc] of the density, ns <= 8533,
+ * and the workspace of ves_farfield_dl_workspace_ns; that of
+ * ves_farfield_dl_workspace holds every ns, at 200 KB per source). */
 VES_API int ves_farfield_dl(ves_ctx* ctx, int precision, int nsrc, int ns, const double* Xsrc, const double* tang,
                             const double* den, const double* sa, const double* visc, int nt, int ntp,
                             const double* Xtar, const int* self_idx, const ves_near_lists* nl, double* out,
                             void* ws, size_t ws_bytes, void* stream);
 VES_API size_t ves_farfield_dl_workspace(int precision, int nsrc, int nt, int ntp);
+VES_API size_t ves_farfield_dl_workspace_ns(int precision, int nsrc, int ns, int nt, int ntp);
 /* nearSingInt with kernelDirect = exactStokesDL (tstep_biem.py:236,501;
  * poten_py.m:495-692): double-layer far field over the Nup-upsampled sources
  * (Xup, tang_up, sa_up of the upsampled curve) with the near pairs removed,

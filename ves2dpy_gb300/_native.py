@@ -222,6 +222,7 @@ SIGNATURES = {
     "ves_farfield_dl": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _I, _P, _P, ctypes.POINTER(NearLists), _P,
                              _P, _SZ, _P]),
     "ves_farfield_dl_workspace": (_SZ, [_I, _I, _I, _I]),
+    "ves_farfield_dl_workspace_ns": (_SZ, [_I, _I, _I, _I, _I]),
     "ves_near_sing_int_dl": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, ctypes.POINTER(NearLists), _D, _P,
                                   _P, _P, _SZ, _P]),
     "ves_near_sing_int_dl_workspace": (_SZ, [_P, _I]),

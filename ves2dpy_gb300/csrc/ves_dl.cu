@@ -334,7 +334,8 @@ namespace {
 constexpr int kDLPMax = 24;          // highest expansion order
 constexpr float kDLRhoMax = 0.35f;   // expansion used for rho_pair <= this
 constexpr float kDLEps = 1e-10f;     // truncation bound relative to sum |c|, sum |e|
-constexpr int kDLStage = 12;         // source vesicles per shared-memory stage (48 KB with eight warps)
+constexpr int kDLStage = 12;         // source vesicles per shared-memory stage
+constexpr int kDLMaxPoints = 8533;   // points per source: what a workspace sized without their count holds (200 KB each)
 
 struct __align__(16) DLSrc {
   float2 chi, clo;  // centre, high and low FP32 parts
@@ -540,7 +541,7 @@ struct DLMPArgs {
   int nsrc, ns, nt, ntp;
   const float4* recA;  // [nsrc][ns] local x, y, normal x, y
   const float2* recB;  // [nsrc][ns] mean-free density
-  const double* Xsrc;  // the FP64 sources (targets within 6 spacings)
+  const double* Xsrc;  // the FP64 sources (targets within 12 spacings)
   const double* tang;
   const double* den;
   const double* Xtar;
@@ -925,8 +926,7 @@ int farfield_dl_mp_run(ves_ctx* c, int nsrc, int ns, const double* Xsrc, const d
     ves_record_error(VES_ERR_ARG, "farfield_dl: the multipole path needs the source jacobian sa");
     return VES_ERR_ARG;
   }
-  const size_t dsmem = (size_t)ns * (sizeof(float4) + sizeof(float2));
-  if (dsmem > 200 * 1024) {
+  if (ns > kDLMaxPoints) {
     ves_record_error(VES_ERR_SHAPE, "farfield_dl: %d source points per vesicle exceed the multipole path", ns);
     return VES_ERR_SHAPE;
   }
@@ -1024,11 +1024,15 @@ extern "C" int ves_dl_density(int nv, int ns, const double* f, const double* sa,
   return ves_launch_check("dl_density");
 }
 
-extern "C" size_t ves_farfield_dl_workspace(int precision, int nsrc, int nt, int ntp) {
+extern "C" size_t ves_farfield_dl_workspace_ns(int precision, int nsrc, int ns, int nt, int ntp) {
   WsCarver w(nullptr, 0);
-  farfield_dl_run(nullptr, precision, nsrc, 1, nullptr, nullptr, nullptr, nullptr, nullptr, nt, ntp, nullptr, nullptr,
-                  nullptr, nullptr, w, 0);
+  farfield_dl_run(nullptr, precision, nsrc, ns > 0 ? ns : 1, nullptr, nullptr, nullptr, nullptr, nullptr, nt, ntp,
+                  nullptr, nullptr, nullptr, nullptr, w, 0);
   return w.off + 256;
+}
+
+extern "C" size_t ves_farfield_dl_workspace(int precision, int nsrc, int nt, int ntp) {
+  return ves_farfield_dl_workspace_ns(precision, nsrc, kDLMaxPoints, nt, ntp);
 }
 
 extern "C" int ves_farfield_dl(ves_ctx* c, int precision, int nsrc, int ns, const double* Xsrc, const double* tang,

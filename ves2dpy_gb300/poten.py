@@ -115,7 +115,7 @@ class Poten:
         Xt = to_vm(Xtar)
         out = torch.empty(ncol, 2 * ntp, dtype=torch.float64, device=dev)
         prec = nat.PREC[precision]
-        ws = self._ctx.workspace(lib.ves_farfield_dl_workspace(prec, len(K1), ncol, ntp))
+        ws = self._ctx.workspace(lib.ves_farfield_dl_workspace_ns(prec, len(K1), N, ncol, ntp))
         nat.check(lib.ves_farfield_dl(self._ctx.handle, prec, len(K1), N, Xs.data_ptr(), ts.data_ptr(), den.data_ptr(),
                                       sas.data_ptr(), visc.data_ptr(), ncol, ntp, Xt.data_ptr(), None, None,
                                       out.data_ptr(), ws.data_ptr(), ws.numel(), st), "exactStokesDL")
