@@ -590,11 +590,6 @@ int launch_lu_factor_f32(ves_ctx* c, int nv, int n, float* A, int* piv, cudaStre
   return lu_factor_t<float>(c, nv, n, A, piv, s);
 }
 
-// exponent between -895 and 896: no intermediate result of the correction is subnormal
-__device__ __forceinline__ bool mid_range(double z) {
-  return (((uint32_t)__double2hiint(z) >> 20) & 0x7ffu) - 128u < 1792u;
-}
-
 // x = LU^{-1} P b per vesicle, one CTA each.  Blocks of 32 rows: the
 // off-diagonal part is a GEMV, four rows to a warp, the 32x32 diagonal block
 // is solved by one warp.  Bound by the FP64 pipe (16 cycles per warp
@@ -688,10 +683,7 @@ __global__ void __launch_bounds__(256) lu_solve_kernel(int n, const T* __restric
       double v = (lane < nr) ? xs[r0 + lane] : 0.0;
       for (int j = nr - 1; j >= 0; --j) {
         const double vj = __shfl_sync(0xffffffffu, v, j), d = tile[j][j], y = rcp[j];
-        const double q0 = vj * y;
-        const double q = fma(fma(-d, q0, vj), y, q0);
-        // zero, and what would leave the correction's range, is divided
-        const double xj = mid_range(q) && mid_range(vj) && mid_range(y) ? q : vj / d;
+        const double xj = quotient(vj, d, y);
         if (lane == j) v = xj;
         if (lane < j) v = fma(-tile[lane][j], xj, v);
       }

@@ -54,9 +54,11 @@ __device__ __forceinline__ float mufu_lg2(float x) {
   return r;
 }
 
-// 1 / x, correctly rounded, for kRcpMin <= x <= kRcpMax: the hardware's
-// approximation (within an ulp) and one residual step in FMA (P. Markstein,
-// IBM J. Res. Dev. 34(1), 1990).  The general division has a branch of its own
+// 1 / x for kRcpMin <= x <= kRcpMax: the hardware's approximation (within an
+// ulp) and one residual step in FMA (P. Markstein, IBM J. Res. Dev. 34(1),
+// 1990).  The theorem leaves out the mantissa of all ones; the result was
+// compared with the division's over every mantissa and is the same
+// (tests/test_gpu_arith.py).  The general division has a branch of its own
 // for each call, so several of them do not overlap.
 constexpr float kRcpMin = 1e-30f, kRcpMax = 1e30f;
 __device__ __forceinline__ float rcp_normal(float x) {
@@ -99,6 +101,19 @@ __device__ __forceinline__ double widen(float x) {
   return __hiloint2double((int)((b & 0x80000000u) | hi), (int)lo);
 }
 __device__ __forceinline__ double widen(double x) { return x; }
+
+// a / d with y = 1 / d from the division: a product and Markstein's correction,
+// the rounding of the division (tests/test_gpu_arith.py).  What would leave the
+// correction's range (exponents between -895 and 896: no intermediate result is
+// subnormal), zero among it, is divided.
+__device__ __forceinline__ bool mid_range(double z) {
+  return (((uint32_t)__double2hiint(z) >> 20) & 0x7ffu) - 128u < 1792u;
+}
+__device__ __forceinline__ double quotient(double a, double d, double y) {
+  const double q0 = a * y;
+  const double q = fma(fma(-d, q0, a), y, q0);
+  return mid_range(q) && mid_range(a) && mid_range(y) ? q : a / d;
+}
 
 // Row j of a circulant matrix (first column d) times two sequences, the matrix
 // read once: sa = sum_l d[(j - l) mod n] a[l], sb with b.

@@ -347,38 +347,6 @@ __global__ void ff_reduce_kernel(long long total_pts, int ntp, int nsplit, const
 // relative error is 2.7-3.6e-16, as it was (2.7-4.9e-16).  Each piece is summed relative to its vesicle's centre as in
 // the FP32 kernel, the centre's log times the vesicle's density sum being
 // added with the first piece.
-//
-// 1 / x and ln x of a positive normal x = 2^k m, m in [sqrt(1/2), sqrt(2)):
-// with the table's y near 1 / m and r = m y - 1 (|r| < 2^-6.9, exact up to
-// rounding), ln x = k ln 2 - ln y + ln(1 + r) by the series to r^8, and 1 / m
-// = y (1 - r)(1 + r^2) corrected by one Newton step.  Both within 1.3 units in
-// the last place on 2e4 arguments against 50 digits.  Anything else (0,
-// subnormal, infinite, NaN) takes the library's functions.
-__device__ __forceinline__ void rcp_log(double x, const double2* __restrict__ tab, double& inv, double& lg) {
-  const uint32_t h = (uint32_t)__double2hiint(x);
-  if (h - 0x00100000u >= 0x7fe00000u) {
-    inv = 1.0 / x;
-    lg = log(x);
-    return;
-  }
-  const uint32_t hx = h + (0x3ff00000u - 0x3fe6a09eu);
-  const int k = (int)(hx >> 20) - 0x3ff;
-  const uint32_t hm = (hx & 0xfffffu) + 0x3fe6a09eu;
-  const double m = __hiloint2double((int)hm, __double2loint(x));
-  const double2 t = tab[(hm - 0x3fe6a09eu) >> 13];
-  const double r = fma(m, t.x, -1.0), r2 = r * r;
-  double y = fma(-r, t.x, t.x);
-  y = fma(y, r2, y);
-  y = fma(y, fma(-m, y, 1.0), y);
-  // y 2^-k by its exponent (1 / x is subnormal only where x is not below 2^1022)
-  inv = k < 1020 && k > -1020 ? __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y)) : 1.0 / x;
-  const double kd = __hiloint2double(0x43300000, (int)((uint32_t)k ^ 0x80000000u)) - 4503601774854144.0;  // k
-  double q = fma(r2, -0.125, fma(r, 1.0 / 7, -1.0 / 6));
-  q = fma(r2, q, fma(r, 0.2, -0.25));
-  q = fma(r2, q, fma(r, 1.0 / 3, -0.5));
-  lg = fma(kd, 0.69314718055994530942, t.y) + fma(r2, q, r);
-}
-
 struct FF64Args {
   int nsrc, ns, ntp;
   long long total_pts;
