@@ -84,10 +84,11 @@ struct WsCarver {
     return p;
   }
   bool ok() const { return sizing || off <= cap; }
-  // bytes that the next take can have (all there are when sizing)
+  // bytes that the next take can have; sizing without a capacity: any number
   size_t left() const {
     const size_t o = (off + 255) & ~(size_t)255;
-    return sizing ? ~(size_t)0 : (cap > o ? cap - o : 0);
+    if (sizing && cap == 0) return ~(size_t)0;
+    return cap > o ? cap - o : 0;
   }
 };
 

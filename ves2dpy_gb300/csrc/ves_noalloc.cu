@@ -71,7 +71,7 @@ extern "C" int ves_farfield_static_scratch(int precision, int nsrc, int ns, cons
   env.status = nullptr;
   env.N = ntp;
   env.timing = nullptr;
-  WsCarver sizing(nullptr, 0);
+  WsCarver sizing(nullptr, cap);
   farfield_run_env(env, precision, nsrc, ns, nullptr, nullptr, nt, ntp, nullptr, nullptr, nullptr, nullptr, sizing, s);
   if (sizing.off > cap) {
     ves_record_error(VES_ERR_WORKSPACE,
