@@ -126,7 +126,7 @@ def test_hedgehog_stays_in_its_lists():
     assert torch.equal(LP, LP2) and torch.equal(only, only2) and float(only.abs().max()) > 0
 
 
-@pytest.mark.parametrize("N, thresh, most", [(16, 0.7, 2), (16, 2.0, 7), (32, 1.2, 3)])
+@pytest.mark.parametrize("N, thresh, most", [(16, 0.7, 2), (16, 2.0, 7), (16, 3.0, 13), (32, 1.2, 3)])
 def test_hedgehog_adds_in_ascending_order(N, thresh, most):
     """The correction alone, bit for bit, against additions in ascending order
     of the vesicle whose self velocity is added; hedgehog points of up to `most`

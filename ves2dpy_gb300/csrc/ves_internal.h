@@ -179,9 +179,11 @@ int near_zone_py(ves_ctx* c, int nv, const double* X, const double* Xup, double 
                  const ves_near_lists* nl, WsCarver& ws, cudaStream_t s);
 int near_zone_matlab(ves_ctx* c, int nv, const double* X, double h, const ves_near_lists* nl,
                      WsCarver& ws, cudaStream_t s);
-// Which hedgehog points of the lists of near_zone_py several vesicles add to:
-// hits [3][nv][N], read by the py_hh correction.  Depends on the lists alone, so
-// a step makes them once.
+// Which vesicles add to each hedgehog point of the lists of near_zone_py: hits
+// [VES_HEDGEHOG_HITS][nv][N], read by the py_hh correction (their number, and up
+// to eight of them; no more than the density's scratch holds, 4 Nup / N ints a
+// point with Nup >= 3 N).  Depends on the lists alone, so a step makes it once.
+constexpr int VES_HEDGEHOG_HITS = 9;
 int hedgehog_hits(const ves_ctx* c, int nv, const ves_near_lists* nl, int* hits, cudaStream_t s);
 // hits: hedgehog_hits of nl (scheme VES_NEAR_PY_HH), or null: made in the workspace
 int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const double* X,

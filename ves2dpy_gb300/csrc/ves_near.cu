@@ -337,9 +337,9 @@ __device__ __forceinline__ bool hh_point(int nv, int N, int Nup, int t, int s, i
   return k2 < nv && k2 != t;
 }
 
-// What the pairs (t, s) with one hedgehog point have in common: how many
-// vesicles t there are (less one) and the first and last of them.  hits: three
-// arrays [nv][N], every byte 0xff before the first launch.
+// The vesicles t that add to a point: hits[0][nv][N] counts them (zero before the
+// launch), hits[1..kHits][nv][N] has up to kHits of them in any order.
+constexpr int kHits = VES_HEDGEHOG_HITS - 1;
 __global__ void __launch_bounds__(128) hh_count_kernel(int nv, int N, int Nup, int maxc,
                                                        const int* __restrict__ cand_count,
                                                        const int* __restrict__ cand_src,
@@ -356,22 +356,22 @@ __global__ void __launch_bounds__(128) hh_count_kernel(int nv, int N, int Nup, i
       int k2, J;
       if (!hh_point(nv, N, Nup, t, s, w * 32 + __ffs(bits) - 1, k2, J)) continue;
       const size_t p = (size_t)k2 * N + J;
-      atomicAdd(&hits[p], 1);
-      atomicMin(reinterpret_cast<unsigned*>(hits) + n + p, (unsigned)t);
-      atomicMax(&hits[2 * n + p], t);
+      const int at = atomicAdd(&hits[p], 1);
+      if (at < kHits) hits[(size_t)(1 + at) * n + p] = t;
     }
   }
 }
 
-// the first vesicle from t0 on, up to t1 and without k2, that has hedgehog point u of s
-__device__ __forceinline__ int hh_next(int Nup, int maxc, const int* __restrict__ cand_count,
+// The first vesicle from t0 on that adds to the point (u of s, J of k2), nv if
+// none: by the lists, for a point of more than kHits.
+__device__ __forceinline__ int hh_scan(int nv, int Nup, int maxc, const int* __restrict__ cand_count,
                                        const int* __restrict__ cand_src, const uint32_t* __restrict__ hh_mask, int t0,
-                                       int t1, int k2, int s, int u, int lane) {
+                                       int k2, int s, int u, int lane) {
   const int wU = (Nup + 31) / 32;
-  for (int b = t0; b <= t1; b += 32) {
+  for (int b = t0; b < nv; b += 32) {
     const int t = b + lane;
     bool bit = false;
-    if (t <= t1 && t != k2) {
+    if (t < nv && t != k2) {
       const int* row = cand_src + (long long)t * maxc;
       const int nc = min(cand_count[t], maxc);
       int lo = 0, hi = nc;
@@ -384,7 +384,7 @@ __device__ __forceinline__ int hh_next(int Nup, int maxc, const int* __restrict_
     const unsigned m = __ballot_sync(0xffffffffu, bit);
     if (m) return b + __ffs(m) - 1;
   }
-  return t1 + 1;
+  return nv;
 }
 
 // One CTA per vesicle t.  Latency-bound: a hedgehog point is a search of the N
@@ -458,15 +458,19 @@ __global__ void __launch_bounds__(128) hh_apply_kernel(int nv, int N, int Nup, i
           int k2, J;
           if (!hh_point(nv, N, Nup, t, s, u, k2, J)) continue;
           const size_t p = (size_t)k2 * N + J;
-          const int more = hits[p], first = hits[n + p], last = hits[2 * n + p];
+          const int m = hits[p];
           const double px = Xup[(long long)k2 * 2 * Nup + J], py = Xup[(long long)k2 * 2 * Nup + Nup + J];
-          if (first != t) continue;
-          add(t, xk, k2, J, px, py);
-          int t1 = t;
-          for (int left = more; left > 0 && t1 < last; --left) {
-            t1 = left == 1 ? last : hh_next(Nup, maxc, cand_count, cand_src, hh_mask, t1 + 1, last, k2, s, u, lane);
-            add(t1, X + (long long)t1 * 2 * N, k2, J, px, py);
+          if (m <= 1) {
+            add(t, xk, k2, J, px, py);
+            continue;
           }
+          const int own = m <= kHits && lane < m ? hits[(size_t)(1 + lane) * n + p] : nv;  // a vesicle per lane
+          auto next = [&](int t0) {  // the first of them from t0 on
+            return m <= kHits ? (int)__reduce_min_sync(0xffffffffu, (unsigned)(own >= t0 ? own : nv))
+                              : hh_scan(nv, Nup, maxc, cand_count, cand_src, hh_mask, t0, k2, s, u, lane);
+          };
+          if (next(0) != t) continue;
+          for (int t1 = t; t1 < nv; t1 = next(t1 + 1)) add(t1, X + (long long)t1 * 2 * N, k2, J, px, py);
         }
       }
     }
@@ -928,7 +932,7 @@ int launch_hedgehog(const ves_ctx* c, int nv, const double* X, const double* Xup
 
 int hedgehog_hits(const ves_ctx* c, int nv, const ves_near_lists* nl, int* hits, cudaStream_t s) {
   if (nv <= 0) return VES_OK;
-  const int rc = ves_cuda_status(cudaMemsetAsync(hits, 0xff, (size_t)3 * nv * c->N * sizeof(int), s), "hedgehog hits");
+  const int rc = ves_cuda_status(cudaMemsetAsync(hits, 0, (size_t)nv * c->N * sizeof(int), s), "hedgehog hits");
   if (rc) return rc;
   ves_count_launch();
   hh_count_kernel<<<nv, 128, 0, s>>>(nv, c->N, c->Nup, nl->maxc, nl->cand_count, nl->cand_src, nl->hh_mask, hits);

@@ -711,7 +711,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   B.ydev = ws.take<double>(restart + 2);
   double* vinf = ws.take<double>((size_t)nv * 2 * N);
   double* rhs2 = ws.take<double>((size_t)nv * N);
-  S.hits = S.dl_scheme == VES_NEAR_PY_HH ? ws.take<int>((size_t)3 * nv * N) : nullptr;
+  S.hits = S.dl_scheme == VES_NEAR_PY_HH ? ws.take<int>((size_t)VES_HEDGEHOG_HITS * nv * N) : nullptr;
   // one scratch region shared by the sub-stages
   size_t scratch = 0;
   {
