@@ -42,16 +42,17 @@ def shuffled(near, perm):
 
 
 @pytest.mark.parametrize("double", [False, True])
-@pytest.mark.parametrize("N", [16, 32])
-def test_entries_in_any_order(N, double):
+@pytest.mark.parametrize("N, room", [(16, 1024), (32, 1024), (32, 8192)])  # lists searched, lists with an index
+def test_entries_in_any_order(N, room, double):
     from ves2dpy_gb300 import Poten
     from ves2dpy_gb300.biem_support import NearZone
     from ves2dpy_gb300.capsules import capsules
     from ves2dpy_gb300.layout import to_vm
     X = T(circles(*packed_circles(6, 6, 0.05), N))
     ves = capsules(X, None, None, 1.0, 3.0 if double else 1.0)
-    near = NearZone.build_matlab(to_vm(X), N, h=0.9)
+    near = NearZone.build_matlab(to_vm(X), N, h=0.9, max_entries=room)
     n = int(near.n_entries[0].item())
+    assert (near.max_entries >= 4096) == (room >= 4096)
     tsj = near.ent_tsj[:3 * n].reshape(n, 3).cpu().numpy()
     _, of_point = np.unique(tsj[:, [0, 2]], axis=0, return_counts=True)
     assert (of_point == 2).sum() >= 20 and (of_point >= 3).sum() >= 3

@@ -185,22 +185,29 @@ int near_zone_matlab(ves_ctx* c, int nv, const double* X, double h, const ves_ne
 // point with Nup >= 3 N).  Depends on the lists alone, so a step makes it once.
 constexpr int VES_HEDGEHOG_HITS = 9;
 int hedgehog_hits(const ves_ctx* c, int nv, const ves_near_lists* nl, int* hits, cudaStream_t s);
-// hits: hedgehog_hits of nl (scheme VES_NEAR_PY_HH), or null: made in the workspace
+// Which entries of MATLAB-scheme lists belong to each target point, for np (<= 16)
+// problems corrected together: nvt[k] targets of context ct[k], which are target
+// set set[k] (problems of one set add to the same points), lists nl[k].  Depends
+// on the lists alone, so a step makes it once; matlab_index_ints gives its size.
+size_t matlab_index_ints(int np, const int* set, ves_ctx* const* ct, const int* nvt, const ves_near_lists* const* nl);
+int matlab_index(int np, const int* set, ves_ctx* const* ct, const int* nvt, const ves_near_lists* const* nl,
+                 int* index, cudaStream_t s);
+// index: hedgehog_hits (VES_NEAR_PY_HH) or matlab_index (VES_NEAR_MATLAB, one
+// problem) of nl, or null: made in the workspace
 int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const double* X,
                       const double* sa_up, const double* Xup, const double* f, const double* vself,
                       const ves_near_lists* nl, double h, double* LP, double* near_only, WsCarver& ws,
-                      cudaStream_t s, const int* hits = nullptr);
+                      cudaStream_t s, const int* index = nullptr);
 // between two vesicle sets (targets: ct, Xt; sources: cs, Xs / Xup_s, den_s, vself_s)
 int near_zone_matlab_cross(ves_ctx* ct, ves_ctx* cs, int nvt, const double* Xt, int nvs, const double* Xs, double h,
                            const ves_near_lists* nl, WsCarver& ws, cudaStream_t s);
-// the MATLAB near-singular correction alone, added to LP (the far field
-// computed elsewhere); ct == cs for a set against itself
-int near_correct_matlab(ves_ctx* ct, ves_ctx* cs, const double* Xt, const double* Xup_s, const double* den_s,
-                        const double* vself_s, const ves_near_lists* nl, double h, double* LP, cudaStream_t s);
-// several MATLAB corrections (np <= 16 pairs of point sets) in one launch
-int near_correct_matlab_pairs(int np, ves_ctx* const* ct, ves_ctx* const* cs, const double* const* Xt,
-                              const double* const* Xup_s, const double* const* den_s, const double* const* vself_s,
-                              const ves_near_lists* const* nl, const double* h, double* const* LP, cudaStream_t s);
+// MATLAB near-singular corrections alone (the far field computed elsewhere),
+// added to LP: np <= 16 pairs of point sets in one launch; index: their
+// matlab_index, or null
+int near_correct_matlab_pairs(int np, const int* set, ves_ctx* const* ct, ves_ctx* const* cs, const int* nvt,
+                              const double* const* Xt, const double* const* Xup_s, const double* const* den_s,
+                              const double* const* vself_s, const ves_near_lists* const* nl, const double* h, double* const* LP, const int* index,
+                              cudaStream_t s);
 int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision, int nvt, const double* Xt, int nvs,
                             const double* Xup_s, const double* den_s, const double* vself_s,
                             const ves_near_lists* nl, double h, double* LP, WsCarver& ws, cudaStream_t s);
@@ -218,7 +225,7 @@ int farfield_dl_run(ves_ctx* c, int precision, int nsrc, int ns, const double* X
 int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* Xup,
                          const double* tang_up, const double* sa_up, const double* visc, const double* f,
                          const double* vself, const ves_near_lists* nl, double h, double* LP, double* near_only,
-                         WsCarver& ws, cudaStream_t s, const int* hits = nullptr);
+                         WsCarver& ws, cudaStream_t s, const int* index = nullptr);
 
 // RBF near-field fits (nearSingInt_rbf): adds the fits of the near pairs to LP
 int rbf_near_correct(ves_ctx* c, int nv, const double* X, const double* f, const double* vself,

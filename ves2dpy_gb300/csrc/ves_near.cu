@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(128) matlab_zone_kernel(int Nt, int Ns, int ma
 // with Nup upsampled points) of another set or of itself, with the near
 // entries of its lists.
 struct MatlabPair {
-  int Nt, Ns, Nup;
+  int set;  // number of the target set: problems of one set add to the same LP
+  int nvt, Nt, Ns, Nup;
   double h;
   const double *Xt, *Xup, *tang_up, *den, *vself, *lag;
   const int* n_entries;
@@ -602,13 +603,35 @@ struct MatlabPair {
 
 // Several correction problems (every pair of point sets of a suspension with
 // several point counts) in one launch: problem k owns the warps
-// [warp0[k], warp0[k+1]), one per near-entry slot.
+// [warp0[k], warp0[k+1]), one per near-entry slot.  The index (or null) chains
+// the slots of each target point: head[k][t Nt + j] is one of them and next[w]
+// the one after slot w, -1 at the end; problems of one target set share their
+// chains.
 constexpr int kMatlabPairs = 16;
 struct MatlabPairs {
   int np;
   long long warp0[kMatlabPairs + 1];
   MatlabPair pair[kMatlabPairs];
+  int* next;
+  int* head[kMatlabPairs];
 };
+
+__device__ __forceinline__ int matlab_problem(const MatlabPairs& P, long long w) {
+  int k = 0;
+  while (k + 1 < P.np && w >= P.warp0[k + 1]) ++k;
+  return k;
+}
+
+// one thread per slot (heads are -1 before the launch)
+__global__ void __launch_bounds__(256) matlab_index_kernel(const __grid_constant__ MatlabPairs P) {
+  const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= P.warp0[P.np]) return;
+  const int k = matlab_problem(P, w), e = (int)(w - P.warp0[k]);
+  const MatlabPair& a = P.pair[k];
+  if (e >= min(*a.n_entries, a.max_entries)) return;
+  const long long at = (long long)a.ent_tsj[3 * (long long)e] * a.Nt + a.ent_tsj[3 * (long long)e + 2];
+  P.next[w] = atomicExch(&P.head[k][at], (int)w);
+}
 
 // Problem, source vesicle and list place of an entry, in the order in which
 // the entries of one target point are added.
@@ -620,12 +643,15 @@ __device__ __forceinline__ MatlabKey matlab_key(int k, int s, int e) {
 }
 
 // true if point j of target vesicle t lies near more than one source vesicle
-// of the problems that add to LP (the warp's lanes share the slots)
-__device__ __forceinline__ bool matlab_shared(const MatlabPairs& P, const double* LP, int t, int j, int lane) {
+// of the problems that add to problem k0's points: by its chain, or by the
+// lists' masks (the warp's lanes share the slots)
+__device__ __forceinline__ bool matlab_shared(const MatlabPairs& P, int k0, int t, int j, int lane) {
+  if (P.next) return P.next[P.head[k0][(long long)t * P.pair[k0].Nt + j]] >= 0;
+  const int set = P.pair[k0].set;
   int n = 0;
   for (int k = 0; k < P.np; ++k) {
     const MatlabPair& a = P.pair[k];
-    if (a.LP != LP || !a.cand_count || !a.excl_mask) continue;
+    if (a.set != set || !a.cand_count || !a.excl_mask) continue;
     const int cc = min(a.cand_count[t], a.maxc), nw = (a.Nt + 31) / 32;
     const uint32_t* m = a.excl_mask + (long long)t * a.maxc * nw + (j >> 5);
     for (int s0 = 0; s0 < cc; s0 += 32) {
@@ -636,13 +662,22 @@ __device__ __forceinline__ bool matlab_shared(const MatlabPairs& P, const double
   return n > 1;
 }
 
-// the first entry of point (t, j) at or after key `from` (kNoEntry: none)
-__device__ __forceinline__ MatlabKey matlab_next(const MatlabPairs& P, const double* LP, int t, int j, MatlabKey from,
-                                                 int lane) {
+// the first entry of point (t, j) of problem k's targets at or after key `from`
+// (kNoEntry: none): along the point's chain, or without one in all lists
+__device__ __forceinline__ MatlabKey matlab_next(const MatlabPairs& P, int k0, int t, int j, MatlabKey from, int lane) {
   MatlabKey best = kNoEntry;
+  if (P.next) {
+    for (int w = P.head[k0][(long long)t * P.pair[k0].Nt + j]; w >= 0; w = P.next[w]) {
+      const int k = matlab_problem(P, w), e = (int)(w - P.warp0[k]);
+      const MatlabKey key = matlab_key(k, P.pair[k].ent_tsj[3 * (long long)e + 1], e);
+      if (key >= from && key < best) best = key;
+    }
+    return best;
+  }
+  const int set = P.pair[k0].set;
   for (int k = 0; k < P.np; ++k) {
     const MatlabPair& a = P.pair[k];
-    if (a.LP != LP) continue;
+    if (a.set != set) continue;
     const int ne = min(*a.n_entries, a.max_entries);
 #pragma unroll 4
     for (int e = lane; e < ne; e += 32) {
@@ -741,28 +776,29 @@ __device__ __forceinline__ void matlab_add_entry(const MatlabPair& a, int e, int
 // entries of a point near several sources (of one set or of several) are all
 // added by the warp of the first of them, in ascending order of (problem,
 // source), so that the sum does not depend on the order of the lists or of the
-// warps; such points are few, and finding their entries is a search of the
-// lists.  FP64 arithmetic (six layer potentials over Nup points per entry)
-// bounds the kernel.
+// warps.  FP64 arithmetic (six layer potentials over Nup points per entry)
+// bounds the kernel.  CTAs of two warps: a warp with two or three entries holds
+// no others' places (with eight warps to a CTA 8192 x N=32, 50617 entries, 7.1
+// ms, with two 6.6), and few entries spread over the chip (1024 x N=128 1.06 ->
+// 0.52 ms).
+constexpr int kMatlabThreads = 64;
 template <bool DL>
-__global__ void matlab_correct_kernel(const __grid_constant__ MatlabPairs P) {
+__global__ void __launch_bounds__(kMatlabThreads) matlab_correct_kernel(const __grid_constant__ MatlabPairs P) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   if (w >= P.warp0[P.np]) return;
-  int k = 0;
-  while (k + 1 < P.np && w >= P.warp0[k + 1]) ++k;
-  int e = (int)(w - P.warp0[k]);
-  const double* LP = P.pair[k].LP;
-  if (e >= min(*P.pair[k].n_entries, P.pair[k].max_entries)) return;
-  const int* tsj = P.pair[k].ent_tsj + 3 * (long long)e;
+  const int k0 = matlab_problem(P, w);
+  int k = k0, e = (int)(w - P.warp0[k0]);
+  if (e >= min(*P.pair[k0].n_entries, P.pair[k0].max_entries)) return;
+  const int* tsj = P.pair[k0].ent_tsj + 3 * (long long)e;
   const int t = tsj[0], j = tsj[2];
-  const bool shared = matlab_shared(P, LP, t, j, lane);
-  MatlabKey key = matlab_key(k, tsj[1], e);
-  if (shared && matlab_next(P, LP, t, j, 0, lane) != key) return;
+  const bool shared = matlab_shared(P, k0, t, j, lane);
+  MatlabKey key = matlab_key(k0, tsj[1], e);
+  if (shared && matlab_next(P, k0, t, j, 0, lane) != key) return;
   for (;;) {
     matlab_add_entry<DL>(P.pair[k], e, lane);
     if (!shared) return;
-    key = matlab_next(P, LP, t, j, key + 1, lane);
+    key = matlab_next(P, k0, t, j, key + 1, lane);
     if (key == kNoEntry) return;
     k = (int)(key >> 60);
     e = (int)(unsigned)key;
@@ -868,12 +904,14 @@ int find_candidates(ves_ctx* c, int nt, int ns, bool same_set, const double* tbo
   return VES_OK;
 }
 
-// One MATLAB correction problem of a launch: targets Xt of context ct, sources
-// of context cs, lists nl.
-MatlabPair matlab_pair(const ves_ctx* ct, const ves_ctx* cs, const double* Xt, const double* Xup_s,
+// One MATLAB correction problem of a launch: nvt targets Xt of context ct (the
+// launch's target set `set`), sources of context cs, lists nl.
+MatlabPair matlab_pair(int set, const ves_ctx* ct, const ves_ctx* cs, int nvt, const double* Xt, const double* Xup_s,
                        const double* tang_up, const double* den_s, const double* vself_s, const ves_near_lists* nl,
                        double h, double* LP, double* near_only) {
   MatlabPair a;
+  a.set = set;
+  a.nvt = nvt;
   a.Nt = ct->N;
   a.Ns = cs->N;
   a.Nup = cs->Nup;
@@ -897,18 +935,64 @@ MatlabPair matlab_pair(const ves_ctx* ct, const ves_ctx* cs, const double* Xt, c
   return a;
 }
 
-template <bool DL>
-void launch_matlab_correct(int np, const MatlabPair* pairs, cudaStream_t s) {
-  MatlabPairs P;
+// The launch of np problems; index: its place, or null.  Returns the index's
+// size in ints: a chain link per slot, then heads for every set of points.
+size_t matlab_pairs(int np, const MatlabPair* pairs, int* index, MatlabPairs& P) {
   memset(&P, 0, sizeof(P));
   P.np = np;
   for (int k = 0; k < np; ++k) {
     P.pair[k] = pairs[k];
     P.warp0[k + 1] = P.warp0[k] + pairs[k].max_entries;
   }
+  size_t n = (size_t)P.warp0[np];
+  P.next = index;
+  for (int k = 0; k < np; ++k) {
+    int same = 0;
+    while (pairs[same].set != pairs[k].set) ++same;
+    if (same == k) {
+      P.head[k] = index ? index + n : nullptr;
+      n += (size_t)pairs[k].nvt * pairs[k].Nt;
+    } else {
+      P.head[k] = P.head[same];
+    }
+  }
+  return n;
+}
+
+int make_matlab_index(int np, const MatlabPair* pairs, int* index, cudaStream_t s) {
+  MatlabPairs P;
+  const size_t n = matlab_pairs(np, pairs, index, P);
+  const long long slots = P.warp0[np];
+  if (slots <= 0) return VES_OK;
+  const int rc = ves_cuda_status(cudaMemsetAsync(index + slots, 0xff, (n - slots) * sizeof(int), s), "near index");
+  if (rc) return rc;
+  ves_count_launch();
+  matlab_index_kernel<<<ceil_div(slots, 256), 256, 0, s>>>(P);
+  return ves_launch_check("near index");
+}
+
+template <bool DL>
+void launch_matlab_correct(int np, const MatlabPair* pairs, const int* index, cudaStream_t s) {
+  MatlabPairs P;
+  matlab_pairs(np, pairs, const_cast<int*>(index), P);
   if (P.warp0[np] <= 0) return;
   ves_count_launch();
-  matlab_correct_kernel<DL><<<(unsigned)ceil_div(P.warp0[np] * 32, 256), 256, 0, s>>>(P);
+  matlab_correct_kernel<DL><<<(unsigned)ceil_div(P.warp0[np] * 32, kMatlabThreads), kMatlabThreads, 0, s>>>(P);
+}
+
+// One problem whose caller has made no index: one in `scratch` (bytes of it),
+// where lists are long enough for searching them to cost more (from 4096
+// entries on, 128 reads of a warp) and the scratch holds it.
+template <bool DL>
+int launch_matlab_correct_one(const MatlabPair& a, const int* index, void* scratch, size_t bytes, cudaStream_t s) {
+  MatlabPairs P;
+  if (!index && a.max_entries >= 4096 && matlab_pairs(1, &a, nullptr, P) * sizeof(int) <= bytes) {
+    const int rc = make_matlab_index(1, &a, (int*)scratch, s);
+    if (rc) return rc;
+    index = (const int*)scratch;
+  }
+  launch_matlab_correct<DL>(1, &a, index, s);
+  return VES_OK;
 }
 
 // The py_hh correction.  hits: hedgehog_hits of the lists, or null: made in
@@ -1018,7 +1102,7 @@ int near_zone_matlab(ves_ctx* c, int nv, const double* X, double h, const ves_ne
 
 int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* sa_up,
                       const double* Xup, const double* f, const double* vself, const ves_near_lists* nl,
-                      double h, double* LP, double* near_only, WsCarver& ws, cudaStream_t s, const int* hits) {
+                      double h, double* LP, double* near_only, WsCarver& ws, cudaStream_t s, const int* index) {
   const int N = c->N, Nup = c->Nup;
   double* fup = ws.take<double>((size_t)nv * 2 * Nup);
   double* den = ws.take<double>((size_t)nv * 2 * Nup);
@@ -1059,10 +1143,10 @@ int near_sing_int_run(ves_ctx* c, int scheme, int precision, int nv, const doubl
     // nearSingInt_rbf: the far field above plus the fits of the near pairs
     if ((rc = rbf_near_correct(c, nv, X, f, vself, nl, LP, ws, s))) return rc;
   } else if (scheme == VES_NEAR_PY_HH) {
-    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, hits, (int*)fup, LP, near_only, s))) return rc;
+    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, index, (int*)fup, LP, near_only, s))) return rc;
   } else if (scheme == VES_NEAR_MATLAB) {
-    const MatlabPair a = matlab_pair(c, c, X, Xup, nullptr, den, vself, nl, h, LP, near_only);
-    launch_matlab_correct<false>(1, &a, s);
+    const MatlabPair a = matlab_pair(0, c, c, nv, X, Xup, nullptr, den, vself, nl, h, LP, near_only);
+    if ((rc = launch_matlab_correct_one<false>(a, index, fup, (size_t)nv * 2 * Nup * sizeof(double), s))) return rc;
   }
   return ves_launch_check("near_sing_int");
 }
@@ -1104,34 +1188,43 @@ int near_zone_matlab_cross(ves_ctx* ct, ves_ctx* cs, int nvt, const double* Xt, 
   return ves_launch_check("near_zone_cross");
 }
 
-// The MATLAB near-singular correction alone (nearSingInt with the far field
-// computed elsewhere, matlab/poten_py.m:495-692): targets Xt of context ct,
-// sources Xup_s of context cs (ct == cs for a set against itself, with the
-// self-vesicle entries of its own lists) with densities den_s and self
-// velocities vself_s; the near entries of nl; added to LP.
-int near_correct_matlab(ves_ctx* ct, ves_ctx* cs, const double* Xt, const double* Xup_s, const double* den_s,
-                        const double* vself_s, const ves_near_lists* nl, double h, double* LP, cudaStream_t s) {
-  const MatlabPair a = matlab_pair(ct, cs, Xt, Xup_s, nullptr, den_s, vself_s, nl, h, LP, nullptr);
-  launch_matlab_correct<false>(1, &a, s);
-  return ves_launch_check("near_correct_matlab");
-}
-
-// Several MATLAB corrections in one launch (np <= 16): problem k has targets
-// Xt[k] of context ct[k], sources Xup_s[k] of context cs[k] with densities
-// den_s[k] and self velocities vself_s[k], near entries nl[k], zone width
-// h[k], and adds to LP[k].
-int near_correct_matlab_pairs(int np, ves_ctx* const* ct, ves_ctx* const* cs, const double* const* Xt,
-                              const double* const* Xup_s, const double* const* den_s, const double* const* vself_s,
-                              const ves_near_lists* const* nl, const double* h, double* const* LP, cudaStream_t s) {
+// The MATLAB near-singular corrections alone (nearSingInt with the far field
+// computed elsewhere, matlab/poten_py.m:495-692), several in one launch (np <=
+// 16): problem k has nvt[k] targets Xt[k] of context ct[k] (target set set[k],
+// LP[k] the set's), sources Xup_s[k] of context cs[k] with densities den_s[k] and self velocities vself_s[k], near
+// entries nl[k], zone width h[k], and adds to LP[k].
+int near_correct_matlab_pairs(int np, const int* set, ves_ctx* const* ct, ves_ctx* const* cs, const int* nvt,
+                              const double* const* Xt, const double* const* Xup_s, const double* const* den_s,
+                              const double* const* vself_s, const ves_near_lists* const* nl, const double* h, double* const* LP, const int* index,
+                              cudaStream_t s) {
   if (np < 1 || np > kMatlabPairs) {
     ves_record_error(VES_ERR_ARG, "near_correct_matlab_pairs: 1 to %d problems", kMatlabPairs);
     return VES_ERR_ARG;
   }
   MatlabPair pairs[kMatlabPairs];
   for (int k = 0; k < np; ++k)
-    pairs[k] = matlab_pair(ct[k], cs[k], Xt[k], Xup_s[k], nullptr, den_s[k], vself_s[k], nl[k], h[k], LP[k], nullptr);
-  launch_matlab_correct<false>(np, pairs, s);
+    pairs[k] = matlab_pair(set[k], ct[k], cs[k], nvt[k], Xt[k], Xup_s[k], nullptr, den_s[k], vself_s[k], nl[k], h[k], LP[k],
+                           nullptr);
+  launch_matlab_correct<false>(np, pairs, index, s);
   return ves_launch_check("near_correct_matlab_pairs");
+}
+
+size_t matlab_index_ints(int np, const int* set, ves_ctx* const* ct, const int* nvt, const ves_near_lists* const* nl) {
+  MatlabPair pairs[kMatlabPairs];
+  MatlabPairs P;
+  for (int k = 0; k < np; ++k)
+    pairs[k] = matlab_pair(set[k], ct[k], ct[k], nvt[k], nullptr, nullptr, nullptr, nullptr, nullptr, nl[k], 0.0, nullptr,
+                           nullptr);
+  return matlab_pairs(np, pairs, nullptr, P);
+}
+
+int matlab_index(int np, const int* set, ves_ctx* const* ct, const int* nvt, const ves_near_lists* const* nl,
+                 int* index, cudaStream_t s) {
+  MatlabPair pairs[kMatlabPairs];
+  for (int k = 0; k < np; ++k)
+    pairs[k] = matlab_pair(set[k], ct[k], ct[k], nvt[k], nullptr, nullptr, nullptr, nullptr, nullptr, nl[k], 0.0, nullptr,
+                           nullptr);
+  return make_matlab_index(np, pairs, index, s);
 }
 
 int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision, int nvt, const double* Xt, int nvs,
@@ -1159,8 +1252,8 @@ int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision,
   ves_count_launch();
   add_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, tmp, LP);
   if (scheme == VES_NEAR_MATLAB) {
-    const MatlabPair a = matlab_pair(ct, cs, Xt, Xup_s, nullptr, den_s, vself_s, nl, h, LP, nullptr);
-    launch_matlab_correct<false>(1, &a, s);
+    const MatlabPair a = matlab_pair(0, ct, cs, nvt, Xt, Xup_s, nullptr, den_s, vself_s, nl, h, LP, nullptr);
+    if ((rc = launch_matlab_correct_one<false>(a, nullptr, tmp, (size_t)n * sizeof(double), s))) return rc;
   }
   return ves_launch_check("near_sing_int_cross");
 }
@@ -1174,7 +1267,7 @@ int near_sing_int_cross_add(ves_ctx* ct, ves_ctx* cs, int scheme, int precision,
 int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const double* X, const double* Xup,
                          const double* tang_up, const double* sa_up, const double* visc, const double* f,
                          const double* vself, const ves_near_lists* nl, double h, double* LP, double* near_only,
-                         WsCarver& ws, cudaStream_t s, const int* hits) {
+                         WsCarver& ws, cudaStream_t s, const int* index) {
   const int N = c->N, Nup = c->Nup;
   double* fup = ws.take<double>((size_t)nv * 2 * Nup);
   double* den = ws.take<double>((size_t)nv * 2 * Nup);
@@ -1211,10 +1304,10 @@ int near_sing_int_dl_run(ves_ctx* c, int scheme, int precision, int nv, const do
                            s);
   if (rc) return rc;
   if (scheme == VES_NEAR_PY_HH) {
-    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, hits, (int*)fup, LP, near_only, s))) return rc;
+    if ((rc = launch_hedgehog(c, nv, X, Xup, vself, nl, index, (int*)fup, LP, near_only, s))) return rc;
   } else if (scheme == VES_NEAR_MATLAB) {
-    const MatlabPair a = matlab_pair(c, c, X, Xup, tang_up, den, vself, nl, h, LP, near_only);
-    launch_matlab_correct<true>(1, &a, s);
+    const MatlabPair a = matlab_pair(0, c, c, nv, X, Xup, tang_up, den, vself, nl, h, LP, near_only);
+    if ((rc = launch_matlab_correct_one<true>(a, index, fup, (size_t)nv * 2 * Nup * sizeof(double), s))) return rc;
   }
   return ves_launch_check("near_sing_int_dl");
 }

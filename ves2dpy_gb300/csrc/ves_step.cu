@@ -262,7 +262,7 @@ struct StepState {
   const double* visc;
   double *alpha, *D, *tang_up, *Xm, *DX, *vdl, *Fdl;
   ves_near_lists nl;
-  int* hits;  // hedgehog_hits of nl (py lists)
+  int* index;  // hedgehog_hits or matlab_index of nl
   double h;
   // matvec temporaries
   double *f, *Gf, *LP;
@@ -281,7 +281,7 @@ int matvec(StepState& S, const double* v, double* out) {
   launch_bgemv_f64(nv, 2 * N, 2 * N, S.G, S.f, 2LL * N, S.Gf, 2LL * N, S.s);
   WsCarver sub(S.scratch, S.scratch_bytes);
   int rc = near_sing_int_run(c, S.prm->near_scheme, S.prm->farfield_precision, nv, S.X, S.sa_up, S.Xup, S.f, S.Gf,
-                             &S.nl, S.h, S.LP, nullptr, sub, S.s, S.hits);
+                             &S.nl, S.h, S.LP, nullptr, sub, S.s, S.index);
   if (rc) return rc;
   if (S.visc) {
     // D Xm and the double layer of Xm (tstep_biem.py:489, 497-501)
@@ -294,7 +294,7 @@ int matvec(StepState& S, const double* v, double* out) {
     WsCarver sub2(S.scratch, S.scratch_bytes);
     if ((rc = near_sing_int_dl_run(c, S.dl_scheme, S.prm->farfield_precision, nv, S.X, S.Xup, S.tang_up, S.sa_up,
                                    S.visc, S.Xm, S.vdl, &S.nl,
-                                   S.h, S.Fdl, nullptr, sub2, S.s, S.hits)))
+                                   S.h, S.Fdl, nullptr, sub2, S.s, S.index)))
       return rc;
   }
   ves_count_launch();
@@ -356,10 +356,29 @@ struct MixedState {
   double *fup[kMaxGroups], *den[kMaxGroups];
   ves_near_lists xl[kMaxGroups][kMaxGroups];  // [target group][source group]
   double h[kMaxGroups];
+  int* index;  // matlab_index of every pair of groups (merged far field)
   char* scratch;
   size_t scratch_bytes;
   int matvecs;
 };
+
+// The pairs of groups that a merged step corrects together: target group g,
+// source group q at place g ng + q.
+struct MixedPairs {
+  int np, set[kMaxGroups * kMaxGroups], nvt[kMaxGroups * kMaxGroups];
+  ves_ctx* ct[kMaxGroups * kMaxGroups];
+  const ves_near_lists* nl[kMaxGroups * kMaxGroups];
+};
+void mixed_pairs(MixedState& M, MixedPairs& P) {
+  P.np = 0;
+  for (int g = 0; g < M.ng; ++g)
+    for (int q = 0; q < M.ng; ++q, ++P.np) {
+      P.set[P.np] = g;
+      P.nvt[P.np] = M.g[g].nv;
+      P.ct[P.np] = M.g[g].c;
+      P.nl[P.np] = q == g ? &M.g[g].nl : &M.xl[g][q];
+    }
+}
 
 // The far field of every group from every group's upsampled sources (the
 // densities M.den of the current matvec), one launch (VES_PREC_FP32M), into
@@ -411,28 +430,27 @@ int matvec(MixedState& M, const double* v, double* out) {
     // the near corrections of every (target group, source group) pair in one
     if ((rc = mixed_farfield_merged(M))) return rc;
     if (prm->near_scheme == VES_NEAR_MATLAB) {
-      ves_ctx *ct[kMaxGroups * kMaxGroups], *cs[kMaxGroups * kMaxGroups];
+      MixedPairs P;
+      mixed_pairs(M, P);
+      ves_ctx* cs[kMaxGroups * kMaxGroups];
       const double *Xt[kMaxGroups * kMaxGroups], *Xs[kMaxGroups * kMaxGroups], *dn[kMaxGroups * kMaxGroups],
           *vs[kMaxGroups * kMaxGroups];
-      const ves_near_lists* nl[kMaxGroups * kMaxGroups];
       double hh[kMaxGroups * kMaxGroups];
       double* lp[kMaxGroups * kMaxGroups];
-      int np = 0;
-      for (int g = 0; g < M.ng; ++g)
-        for (int q = 0; q < M.ng; ++q, ++np) {
-          StepState& S = M.g[g];
+      for (int g = 0, k = 0; g < M.ng; ++g)
+        for (int q = 0; q < M.ng; ++q, ++k) {
           const StepState& Q = M.g[q];
-          ct[np] = S.c;
-          cs[np] = Q.c;
-          Xt[np] = S.X;
-          Xs[np] = Q.Xup;
-          dn[np] = M.den[q];
-          vs[np] = Q.Gf;
-          nl[np] = q == g ? &S.nl : &M.xl[g][q];
-          hh[np] = q == g ? S.h : M.h[q];
-          lp[np] = S.LP;
+          cs[k] = Q.c;
+          Xt[k] = M.g[g].X;
+          Xs[k] = Q.Xup;
+          dn[k] = M.den[q];
+          vs[k] = Q.Gf;
+          hh[k] = q == g ? M.g[g].h : M.h[q];
+          lp[k] = M.g[g].LP;
         }
-      if ((rc = near_correct_matlab_pairs(np, ct, cs, Xt, Xs, dn, vs, nl, hh, lp, M.s))) return rc;
+      if ((rc = near_correct_matlab_pairs(P.np, P.set, P.ct, cs, P.nvt, Xt, Xs, dn, vs, P.nl, hh, lp, M.index,
+                                          M.s)))
+        return rc;
     }
     for (int g = 0; g < M.ng; ++g) {
       StepState& S = M.g[g];
@@ -711,7 +729,11 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   B.ydev = ws.take<double>(restart + 2);
   double* vinf = ws.take<double>((size_t)nv * 2 * N);
   double* rhs2 = ws.take<double>((size_t)nv * N);
-  S.hits = S.dl_scheme == VES_NEAR_PY_HH ? ws.take<int>((size_t)VES_HEDGEHOG_HITS * nv * N) : nullptr;
+  const ves_near_lists* own = &S.nl;
+  const int own_set = 0;
+  S.index = nullptr;
+  if (S.dl_scheme == VES_NEAR_PY_HH) S.index = ws.take<int>((size_t)VES_HEDGEHOG_HITS * nv * N);
+  if (S.dl_scheme == VES_NEAR_MATLAB) S.index = ws.take<int>(matlab_index_ints(1, &own_set, &c, &nv, &own));
   // one scratch region shared by the sub-stages
   size_t scratch = 0;
   {
@@ -808,6 +830,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   if (prm->near_scheme == VES_NEAR_MATLAB) {
     WsCarver sub(S.scratch, S.scratch_bytes);
     if ((rc = near_zone_matlab(c, nv, X, 0.0, &S.nl, sub, s))) goto done;
+    if ((rc = matlab_index(1, &own_set, &c, &nv, &own, S.index, s))) goto done;
     // h = min length / N (capsules.py:46-47)
     double* len = (double*)S.scratch;
     launch_geom_prop(c, nv, X, nullptr, nullptr, len, s);
@@ -819,7 +842,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
   } else if (prm->near_scheme == VES_NEAR_PY_HH || prm->near_scheme == VES_NEAR_PY_RBF) {
     WsCarver sub(S.scratch, S.scratch_bytes);
     if ((rc = near_zone_py(c, nv, X, S.Xup, 0.0, &S.nl, sub, s))) goto done;
-    if ((prm->near_scheme == VES_NEAR_PY_HH || vc) && (rc = hedgehog_hits(c, nv, &S.nl, S.hits, s))) goto done;
+    if ((prm->near_scheme == VES_NEAR_PY_HH || vc) && (rc = hedgehog_hits(c, nv, &S.nl, S.index, s))) goto done;
   }
   // right-hand side [X + dt*vinf; surfaceDiv(X)], with the double layer of X
   // (Fdlp + D X, tstep_biem.py:231-244) and the repulsion when present
@@ -832,7 +855,7 @@ static int biem_step_impl(ves_ctx* c, const ves_step_params* prm, int nv, const 
     WsCarver sub(S.scratch, S.scratch_bytes);
     if ((rc = near_sing_int_dl_run(c, S.dl_scheme, prm->farfield_precision, nv, X, S.Xup, S.tang_up, S.sa_up, S.visc,
                                    X, S.vdl, &S.nl, S.h,
-                                   S.Fdl, nullptr, sub, s, S.hits)))
+                                   S.Fdl, nullptr, sub, s, S.index)))
       goto done;
   }
   if (prm->repulsion && nv > 1) {
@@ -1070,6 +1093,11 @@ static int biem_step_mixed_impl(int ng, ves_ctx* const* ctx, const ves_step_para
     M.scratch_bytes = 0;
     mixed_farfield_merged(M, true);
     scratch = std::max(scratch, M.scratch_bytes);
+    if (prm->near_scheme == VES_NEAR_MATLAB) {
+      MixedPairs P;
+      mixed_pairs(M, P);
+      M.index = ws.take<int>(matlab_index_ints(P.np, P.set, P.ct, P.nvt, P.nl));
+    }
   }
   M.scratch = ws.take<char>(scratch + 1024);
   M.scratch_bytes = scratch + 1024;
@@ -1131,6 +1159,11 @@ static int biem_step_mixed_impl(int ng, ves_ctx* const* ctx, const ves_step_para
                                          M.g[q].nv > 0 ? M.h[q] : 1.0, &M.xl[g][q], sub, s)))
           return rc;
       }
+    if (M.index) {
+      MixedPairs P;
+      mixed_pairs(M, P);
+      if ((rc = matlab_index(P.np, P.set, P.ct, P.nvt, P.nl, M.index, s))) return rc;
+    }
   }
   // right-hand side and initial guess, group by group; the preconditioner blocks
   for (int g = 0; g < ng; ++g) {
