@@ -480,10 +480,9 @@ __global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(int B, int spc, in
   for (int b = b0; b < b1; ++b) {
     __syncthreads();
     for (int i = threadIdx.x; i < cin * row; i += blockDim.x) {
-      const int at = i % row;
-      int q = HALO ? at - pad : at;
+      int q = HALO ? i % row - pad : i % row;
       q = q < 0 ? q + L : (q >= L ? q - L : q);
-      if (!HALO || at < row - 1) sx[i] = x[((long long)b * cin + i / row) * L + q];  // the last place only spaces rows
+      sx[i] = x[((long long)b * cin + i / row) * L + min(q, L - 1)];  // q = L: the last place, which only spaces rows
     }
     for (int i = threadIdx.x; i < cout * Lo; i += blockDim.x) sg[i] = dZ[((long long)b * ztot + zoff) * Lo + i];
     __syncthreads();
