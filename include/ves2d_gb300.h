@@ -194,7 +194,9 @@ VES_API int ves_density(int nv, int ns, const double* f, const double* sa, doubl
  * ves_near_zone_py) or VES_NEAR_MATLAB (lists of ves_near_zone_matlab),
  * VES_NEAR_NONE (nl ignored).  near_only (or NULL) receives the correction
  * alone (the reference's second return value; zero for VES_NEAR_PY_RBF, whose
- * reference returns LP only). */
+ * reference returns LP only).  Corrections of one point are added in ascending
+ * order of the source vesicle (MATLAB) or of the vesicle whose velocity is added
+ * (PY_HH), whatever the order of the entries. */
 VES_API int ves_near_sing_int(ves_ctx* ctx, int scheme, int precision, int nv, const double* X,
                       const double* sa_up, const double* Xup, const double* f,
                       const double* vself, const ves_near_lists* nl, double h, double* LP,

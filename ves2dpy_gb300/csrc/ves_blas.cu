@@ -252,17 +252,15 @@ void launch_bgemv_f64(int nv, int m, int n, const double* A, const double* x, lo
 // first on ties), one for the pivot row and the row it replaces, which pass
 // through shared memory.  Eight columns are unrolled (32 make 200 KB of
 // instructions, and fetching them was the bound), then they move to shared
-// memory, where the panel lies transposed (Lt) for what follows.  The panel's row exchanges are worked out as one
-// permutation: every other column is read, permuted and, right of the panel,
+// memory, where the panel lies transposed (Lt) for what follows.  The panel's
+// row exchanges are worked out as one permutation: every other column is read, permuted and, right of the panel,
 // solved against the unit triangle by one thread, and the trailing matrix is
 // updated in 32 x 32 tiles per warp, 8 x 4 entries per thread.  An entry takes
 // its multiply-adds in ascending order of the column eliminated, whatever the
 // tiles, so the factors do not depend on them.
 // FP64 is bound by its pipe (1000 matrices of 384: 19 G multiply-adds, 33 ms;
 // 46.9 -> 39.3 ms; 8192 of 96: 4.1 ms, 9.1 -> 7.0), FP32 by the latency of a
-// column (1024 of 384: 13.8 -> 3.5 ms).  The first form passed a panel through
-// shared memory at a stride of 32 for every column, swapped rows in global
-// memory with a barrier each, and divided 64-bit indices for every entry.
+// column (1024 of 384: 13.8 -> 3.5 ms).
 constexpr int LU_NB = 32;
 
 // distance of the transposed panel's rows: 16-byte aligned, off a multiple of 16

@@ -587,10 +587,9 @@ struct __align__(16) DLPair {
 // memory, where the unit's first warp adds them in source order, so the sum
 // does not depend on S.  What bounds it are the close pairs, a chain of ns
 // terms per point each: their FP32 divisions overlap eight at a time
-// (rcp_normal), and the points that need FP64 share a warp's lanes.  301
-// vesicles of N = 64, ns = 512, with contrast: 1.15 ms -> 0.33 ms per launch,
-// the same bits (FP64 shared out 0.69, branch-free reciprocal 0.41, four close
-// points at a time instead of eight, which leaves room for a fourth CTA, 0.33).
+// (rcp_normal), and the points that need FP64 share a warp's lanes, four of
+// them at a time, which leaves room for a fourth CTA.  301 vesicles of N = 64,
+// ns = 512, with contrast: 1.15 -> 0.33 ms per launch, the same bits.
 constexpr int kNear = 4;    // close points of a pair summed together
 constexpr int kDLRow = 33;  // doubles per row of their terms: rows start on different banks
 

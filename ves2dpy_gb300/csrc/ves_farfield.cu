@@ -337,14 +337,13 @@ __global__ void ff_reduce_kernel(long long total_pts, int ntp, int nsplit, const
 // FP64 direct rule.  Bound by the FP64 pipe (2 fma/clk/SM, 16 cycles per warp
 // instruction), so what counts is the instructions per pair: the reciprocal
 // and the logarithm share one table look-up and one reduced argument
-// (rcp_log), ~30 in all where 1 / x and log2 of the library brought it to ~72;
-// the operands need no staging.  One thread per target point, and the sources
-// are cut into pieces of a vesicle (``chunk`` points), ``per_split`` pieces per
-// CTA row, so that a small suspension spreads over the chip where whole source
-// vesicles staged two at a time left it to a single CTA.  One sum, 16 vesicles
-// of N = 32: 43 ms on one SM, 0.170 ms in pieces, 0.104 ms with the shared
-// look-up.  Against 113-bit sums (16 to 64 points, 10 to 40 vesicles) the
-// relative error is 2.7-3.6e-16, as it was (2.7-4.9e-16).  Each piece is summed relative to its vesicle's centre as in
+// (rcp_log), ~30 in all, ~72 with 1 / x and log2; the operands need no staging.
+// One thread per target point, and the sources are cut into pieces of a vesicle
+// (``chunk`` points), ``per_split`` pieces per CTA row, so that a small
+// suspension spreads over the chip.  One sum, 16 vesicles of N = 32: 43 ->
+// 0.104 ms.  Against 113-bit sums (16 to 64 points, 10 to 40 vesicles) the
+// relative error is 2.7-3.6e-16, with 1 / x and log2 2.7-4.9e-16.  Each piece
+// is summed relative to its vesicle's centre as in
 // the FP32 kernel, the centre's log times the vesicle's density sum being
 // added with the first piece.
 struct FF64Args {

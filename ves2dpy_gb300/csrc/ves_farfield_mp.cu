@@ -306,15 +306,11 @@ __device__ __forceinline__ void horner(float2& xr, float2& xi, float2& yr, float
 // instructions per term.  Close pairs run the direct rule on records staged
 // 32 at a time by the warp itself, so no warp waits for another's close pairs
 // inside a stage, and a stage's buffer is refilled by the warp that leaves it
-// last, so that none waits for another's between stages either (S == 1; with a
-// barrier per stage a fifth of the warps' time: 8192 x N=32 13.3 -> 12.9 ms,
-// 2048 x N=96 4.04 -> 3.66, 1024 x N=128 2.05 -> 2.00).  Five CTAs of four warps per SM (102 registers): with 80
-// registers the direct rule's loads and MUFU results are not overlapped, with
-// 128 the series wait.  One sum, before (one column per CTA, every thread
-// working out every pair, all 25 orders staged) and now: 8192 x N=32 32.6 ->
-// 13.3 ms, 4096 x N=128 20.7 -> 15.0, 1024 x N=128 2.44 -> 2.05, 333 x N=64
-// 0.49 -> 0.23.  Two points per lane, which halves the operand loads, was
-// slower (20.4 and 19.6 ms on the first two): 96 registers are too few for it.
+// last, so that none waits for another's between stages either (S == 1).  Five
+// CTAs of four warps per SM (102 registers): with 80 registers the direct
+// rule's loads and MUFU results are not overlapped, with 128 the series wait.
+// One sum: 8192 x N=32 32.6 -> 12.9 ms, 4096 x N=128 20.7 -> 14.9, 1024 x N=128
+// 2.44 -> 2.00, 333 x N=64 0.49 -> 0.23.
 //
 // S warps share one unit when there are too few units to fill the chip: they
 // take the sources of a stage in turn and leave the contributions in shared

@@ -44,10 +44,8 @@
 // its 64 cycles, the whole shared-memory rate) next to the epilogues' own
 // reads and writes there.  With every epilogue access left out of the copy
 // the kernels still took 75-95% of their time.  One network pass, 1024
-// vesicles, before (one warp per lane quarter, one vesicle per up2 item, its
-// block input staged in shared memory, MMAs issued from per-thread values) and
-// now, ms: advection 56.1 -> 49.3, near field 48.7 -> 34.9, advection-tension
-// 42.5 -> 31.8.  The near field's kernels: down 1.20 -> 0.92, up1 0.45 -> 0.33,
+// vesicles, ms: advection 56.1 -> 49.3, near field 48.7 -> 34.9,
+// advection-tension 42.5 -> 31.8.  The near field's kernels: down 1.20 -> 0.92, up1 0.45 -> 0.33,
 // up2 1.83 -> 1.23; the advection's 1.67 -> 1.41, 0.62 -> 0.51, 2.05 -> 1.86.
 #include <math.h>
 #include <stdio.h>
@@ -622,7 +620,6 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) down_kernel(KArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // The transposed convolutions, split in two kernels so that their weight
 // images and per-group arrays are small enough for several warp groups per SM:
 //   up1: transposed conv 1 (intermediate [kcd][L/4] -> [kcd][L/2], BF16 rows
@@ -801,9 +798,7 @@ __global__ void __launch_bounds__(NG * kGroupThreads, 1) up1_kernel(KArgs a) {
 // accumulators each.  The residual and the bias go into the mix accumulators
 // while the transposed conv runs, straight from global memory (prefetched into
 // L2 one item ahead), so the block input needs no shared memory.  The two
-// halves of the mix are issued by two threads.  Loading the residual one item
-// ahead into registers was slower (671 against 645 us at 512 vesicles of the
-// near field), as was one thread issuing both halves.
+// halves of the mix are issued by two threads (one was slower).
 template <int KCD, int NG, int VU>
 __global__ void __launch_bounds__(NG * kGroupThreads, 1) up2_kernel(KArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
